@@ -218,11 +218,43 @@ void mix_run(gb_ctx* ctx, const MixDev& m, int dtype, const void* x, void* y, do
 void add_diag(gb_ctx* ctx, int dtype, void* y, const std::vector<int64_t>& offs,
               const std::vector<double>& vals, int64_t count, int64_t ds);
 
-// FP64 / complex GEMM on CUDA cores, column-major, batched with strides.
+struct Packed;
+// FP64 / complex GEMM, column-major, batched with strides.
 // op: 'N', 'T' or 'C'.  C = alpha*op(A)*op(B) + beta*C (beta = 0 does not read C).
+// pA / pB: the same operands already cut into digits (slice_operand).
 void gemm_fp64(gb_ctx* ctx, int dtype, char opA, char opB, int64_t M, int64_t N, int64_t K,
                cplx alpha, const void* A, int64_t lda, int64_t sA, const void* B, int64_t ldb,
-               int64_t sB, cplx beta, void* C, int64_t ldc, int64_t sC, int64_t batch);
+               int64_t sB, cplx beta, void* C, int64_t ldc, int64_t sC, int64_t batch,
+               const Packed* pA = nullptr, const Packed* pB = nullptr);
+
+// FP64 products on the tensor cores in exact integer arithmetic (gemm_f64.cu)
+constexpr int F64_SLICES = 7;
+// Real multiply-adds from which the digits win: the small-tile kernel takes 6.5 us + 1.75 us
+// per million (128 x 128 x 128 complex, 8.4 M: 23 us; 256 x 128 x 128: 35 us), the digit path
+// 25-28 us for anything up to 70 M and 8 us less with one operand already cut.
+constexpr double F64_SLICED_MIN_MAC = 1.2e7;
+constexpr double F64_SLICED_MIN_MAC_CUT = 8e6;  // one operand constant
+bool gemm_sliced_wanted(gb_ctx* ctx, int dtype, int64_t M, int64_t N, int64_t K, int64_t batch,
+                        double min_mac = F64_SLICED_MIN_MAC);
+size_t sliced_bytes(int64_t R, int64_t K, bool cx, int role, int64_t batch);
+void slice_operand(gb_ctx* ctx, int dtype, int role, char op, int64_t R, int64_t K,
+                   const void* src, int64_t ld, int64_t stride, int64_t batch, Packed& out,
+                   void* dst);
+// false (nothing done) when the digits do not fit in memory
+bool gemm_fp64_sliced(gb_ctx* ctx, int dtype, char opA, char opB, int64_t M, int64_t N, int64_t K,
+                      double alpha, const void* A, int64_t lda, int64_t sA, const void* B,
+                      int64_t ldb, int64_t sB, double beta, void* C, int64_t ldc, int64_t sC,
+                      int64_t batch, const Packed* pA, const Packed* pB);
+// plain FP64 FMAs in small tiles
+struct SmallPlan {
+  int tile = 0, tm = 4, tn = 8, splits = 1;
+  bool ok = false;
+};
+SmallPlan gemm_small_plan(int sms, int64_t M, int64_t N, int64_t K, int64_t batch);
+void gemm_small(cudaStream_t st, const SmallPlan& p, int dtype, char opA, char opB, int64_t M,
+                int64_t N, int64_t K, cplx alpha, const void* A, int64_t lda, int64_t sA,
+                const void* B, int64_t ldb, int64_t sB, cplx beta, bool use_beta, void* C,
+                int64_t ldc, int64_t sC, int64_t batch, int64_t kchunk);
 
 // BLAS-1 style helpers over n elements of dtype
 void fill_zero(gb_ctx* ctx, void* p, size_t bytes);
@@ -264,6 +296,12 @@ struct Packed {
   bool cnt_valid = false;
   int esz = 2;               // plane element bytes: 2 (BF16 planes) or 4 (TF32 planes)
   int bk = 64;               // k-block (elements per 128-byte swizzle row): 64 or 32
+  // FP64 operands cut into digits (slices > 0): planes [batch][slices][rows][Kp] of BF16
+  // integers, one biased exponent per logical row, one byte per 32-row x 64-k block (mrows
+  // row groups) that holds a nonzero
+  int slices = 0;
+  int* exps = nullptr;
+  uint8_t* nz = nullptr;
 };
 // which operand of C = op(A) op(B) is being packed
 enum PackRole { PACK_AS_A = 0, PACK_AS_B = 1 };

@@ -981,6 +981,22 @@ CUtensorMap make_plane_map(void* data, int esz, int64_t kdim, int64_t rows, int6
   return m;
 }
 
+// map over digit planes: a box of one 128-byte K row, box_rows rows and box_planes planes
+CUtensorMap make_slice_map(void* data, int64_t kdim, int64_t rows, int64_t planes, int box_rows,
+                           int box_planes) {
+  load_encode();
+  CUtensorMap m;
+  cuuint64_t dims[3] = {(cuuint64_t)kdim, (cuuint64_t)rows, (cuuint64_t)planes};
+  cuuint64_t strides[2] = {(cuuint64_t)kdim * 2, (cuuint64_t)kdim * rows * 2};
+  cuuint32_t box[3] = {64, (cuuint32_t)box_rows, (cuuint32_t)box_planes};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = g_encode(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, data, dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) throw Error(GB_ERR_CUDA, "cuTensorMapEncodeTiled failed (digit planes)");
+  return m;
+}
+
 bool tc_available(gb_ctx* ctx) {
   int major = 0, minor = 0;
   cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, ctx->device);
@@ -1142,7 +1158,7 @@ void gemm(gb_ctx* ctx, int prec, int dtype, char opA, char opB, int64_t M, int64
   GB_REQUIRE(!c_f32 || (prec != GB_PREC_FP64 && K > 0), "gemm: FP32 output only in split mode");
   if (prec == GB_PREC_FP64 || K == 0) {
     gemm_fp64(ctx, dtype, opA, opB, M, N, K, cplx{alpha, 0}, A, lda, sA, B, ldb, sB,
-              cplx{beta, 0}, C, ldc, sC, batch);
+              cplx{beta, 0}, C, ldc, sC, batch, pA, pB);
     // every region written: a full output map
     if (outmap) GB_CHECK_CUDA(cudaMemsetAsync(outmap, 0xff, outmap_bytes(M, N), ctx->stream));
     return;

@@ -208,6 +208,17 @@ static void* dalloc(gb_heff* h, size_t bytes) {
   return p;
 }
 
+// the same for buffers an operator can do without
+static void* try_dalloc(gb_heff* h, size_t bytes) {
+  try {
+    return dalloc(h, bytes);
+  } catch (const Error& e) {
+    if (e.code != GB_ERR_OOM) throw;
+    cudaGetLastError();
+    return nullptr;
+  }
+}
+
 // T1 is an M x N column-major matrix; the mix input i starts at offset io[i] and advances
 // by M * xnM per output column n
 static void record_t1_geometry(gb_heff* h, int64_t M, int64_t N, const std::vector<int64_t>& io,
@@ -265,12 +276,32 @@ static void prepare_t2p(gb_heff* h) {
 }
 
 static void prepack(gb_heff* h, Step& s) {
+  gb_ctx* ctx = h->ctx;
   if (h->prec == GB_PREC_FP64) {
-    s.hasPA = s.hasPB = false;
+    // digits of the operator's own constants, cut once for all applications (an environment
+    // that a term reads in place may be written to between applications)
+    auto own = [h](const void* p) {
+      return std::find(h->owned.begin(), h->owned.end(), (void*)p) != h->owned.end();
+    };
+    if (s.hasPA || s.hasPB ||
+        !gemm_sliced_wanted(ctx, h->dtype, s.M, s.N, s.K, 1, F64_SLICED_MIN_MAC_CUT))
+      return;
+    const bool cx = is_cplx(h->dtype);
+    if (s.srcA == S_CONST && own(s.cA)) {
+      if (void* d = try_dalloc(h, sliced_bytes(s.M, s.K, cx, PACK_AS_A, 1))) {
+        slice_operand(ctx, h->dtype, PACK_AS_A, s.opA, s.M, s.K, s.cA, s.lda, 0, 1, s.pA, d);
+        s.hasPA = true;
+      }
+    }
+    if (s.srcB == S_CONST && own(s.cB)) {
+      if (void* d = try_dalloc(h, sliced_bytes(s.N, s.K, cx, PACK_AS_B, 1))) {
+        slice_operand(ctx, h->dtype, PACK_AS_B, s.opB, s.N, s.K, s.cB, s.ldb, 0, 1, s.pB, d);
+        s.hasPB = true;
+      }
+    }
     return;
   }
   prepare_t2p(h);
-  gb_ctx* ctx = h->ctx;
   if (s.srcA == S_CONST && !s.hasPA) {
     void* dst = dalloc(h, packed_bytes(s.M, s.K, is_cplx(h->dtype), PACK_AS_A, 1, h->prec));
     pack_operand(ctx, h->dtype, PACK_AS_A, s.opA, s.M, s.K, s.cA, s.lda, 0, 1, s.pA, dst,

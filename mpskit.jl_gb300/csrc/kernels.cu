@@ -399,7 +399,8 @@ __global__ void splitk_reduce_kernel(int64_t M, int64_t N, int nsplit, const T* 
 
 void gemm_fp64(gb_ctx* ctx, int dtype, char opA, char opB, int64_t M, int64_t N, int64_t K,
                cplx alpha, const void* A, int64_t lda, int64_t sA, const void* B, int64_t ldb,
-               int64_t sB, cplx beta, void* C, int64_t ldc, int64_t sC, int64_t batch) {
+               int64_t sB, cplx beta, void* C, int64_t ldc, int64_t sC, int64_t batch,
+               const Packed* pA, const Packed* pB) {
   if (M == 0 || N == 0 || batch == 0) return;
   GB_REQUIRE(batch <= 65535, "gemm: batch too large");
   GB_REQUIRE((N + GBN - 1) / GBN <= 65535, "gemm: N too large");
@@ -414,6 +415,38 @@ void gemm_fp64(gb_ctx* ctx, int dtype, char opA, char opB, int64_t M, int64_t N,
       scale(ctx, dtype, M * N, beta, C);
     }
     return;
+  }
+  if (alpha.im == 0.0 && beta.im == 0.0 &&
+      (pA || pB || gemm_sliced_wanted(ctx, dtype, M, N, K, batch)) &&
+      gemm_fp64_sliced(ctx, dtype, opA, opB, M, N, K, alpha.re, A, lda, sA, B, ldb, sB, beta.re, C,
+                       ldc, sC, batch, pA, pB))
+    return;
+  const double mac = (double)M * (double)N * (double)K * (double)batch * (is_cplx(dtype) ? 4 : 1);
+  if (mac < F64_SLICED_MIN_MAC) {
+    const SmallPlan p = gemm_small_plan(std::max(1, ctx->num_sms), M, N, K, batch);
+    if (p.ok) {
+      if (p.splits > 1) {
+        const int64_t kchunk = (K + p.splits - 1) / p.splits;
+        const int ns = (int)((K + kchunk - 1) / kchunk);
+        void* W = scratch(ctx, SLOT_SPLITK, (size_t)ns * M * N * elem_size(dtype));
+        gemm_small(ctx->stream, p, dtype, opA, opB, M, N, K, alpha, A, lda, 0, B, ldb, 0,
+                   cplx{0, 0}, false, W, M, M * N, ns, kchunk);
+        const unsigned rb = (unsigned)std::min<int64_t>((M * N + 255) / 256, 4096);
+        if (is_cplx(dtype))
+          splitk_reduce_kernel<dcx><<<rb, 256, 0, ctx->stream>>>(
+              M, N, ns, (const dcx*)W, mk(beta.re, beta.im), use_beta, (dcx*)C, ldc);
+        else
+          splitk_reduce_kernel<double><<<rb, 256, 0, ctx->stream>>>(
+              M, N, ns, (const double*)W, beta.re, use_beta, (double*)C, ldc);
+        count_launch(ctx);
+      } else {
+        gemm_small(ctx->stream, p, dtype, opA, opB, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta,
+                   use_beta, C, ldc, sC, batch, 0);
+      }
+      LAUNCH_CHECK();
+      count_launch(ctx);
+      return;
+    }
   }
   // large products skip zero 64 x 64 x 64 blocks (block-sparse operands stored densely)
   uint32_t* masks = nullptr;

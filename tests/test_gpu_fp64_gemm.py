@@ -1,0 +1,158 @@
+"""Plain-precision products of the device against extended precision.
+
+Entry bound: the digits keep every entry of a row (column) to half a unit of 2^-54 of its
+largest part, and the product digits left out are smaller still, so over K terms
+|C - C*| <= 2 K 2^-54 a b + 2^-53 |C*| with a, b the largest parts of the row and the column
+(four real products per complex one).  The plain-FMA kernel used for small products is within
+K 2^-53 sum |a_k| |b_k| <= K^2 2^-53 a b."""
+import numpy as np
+import pytest
+
+import mpsgb
+from mpsgb import _lib as L
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    return mpsgb.Context(0)
+
+
+def _rand(rng, shape, cx, spread):
+    x = rng.standard_normal(shape)
+    if cx:
+        x = x + 1j * rng.standard_normal(shape)
+    if spread:  # magnitudes over many decades inside every row and column
+        x = x * 10.0 ** rng.uniform(-spread, 0, shape)
+    return x
+
+
+def _wide(a):
+    return a.astype(np.clongdouble if np.iscomplexobj(a) else np.longdouble)
+
+
+def _part(a, axis):
+    return np.maximum(np.abs(a.real), np.abs(a.imag) if np.iscomplexobj(a) else 0).max(axis=axis)
+
+
+def _check(C, A, B, small):
+    """C = A B for 2-d arrays."""
+    K = A.shape[1]
+    ref = _wide(A) @ _wide(B)
+    err = np.abs(_wide(C) - ref).astype(np.float64)
+    n = 4.0 if np.iscomplexobj(C) else 1.0
+    scale = np.outer(_part(A, 1), _part(B, 0))
+    bound = n * (K * K * 2.0 ** -53 if small else 2 * K * 2.0 ** -54) * scale
+    bound = bound + 2.0 ** -52 * np.abs(ref).astype(np.float64)
+    assert np.all(err <= bound), float((err / np.maximum(bound, 1e-300)).max())
+    return float(np.linalg.norm(err) / np.linalg.norm(ref.astype(C.dtype)))
+
+
+# (rows / 2, K, columns): tile edges of 128 x 64 and 128 x 32, k-blocks of 64, one and many
+# splits, single rows and columns
+SHAPES = [(64, 384, 256, 0), (64, 385, 255, 3), (65, 191, 513, 0), (150, 290, 149, 8),
+          (301, 550, 37, 0), (1, 4097, 1500, 0), (1500, 4097, 1, 0), (33, 3000, 65, 0),
+          (510, 70, 600, 2), (160, 128, 129, 0), (11, 23, 69, 0), (8, 700, 9, 0), (2, 1, 3, 0)]
+
+
+@pytest.mark.parametrize("cx", [False, True])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_mul_tail(ctx, shape, cx):
+    h, K, N, spread = shape
+    rng = np.random.default_rng(hash(shape) % 1000)
+    A = _rand(rng, (h, 2, K), cx, spread)
+    C = _rand(rng, (K, N), cx, spread)
+    out = mpsgb.states.mul_tail(mpsgb.DeviceTensor.from_numpy(ctx, "mps", A),
+                                mpsgb.DeviceTensor.from_numpy(ctx, "bond", C)).numpy()
+    mac = 2 * h * K * N * (4 if cx else 1)
+    _check(out.reshape(2 * h, N, order="F"), A.reshape(2 * h, K, order="F"), C, mac < 1.2e7)
+    assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("cx", [False, True])
+def test_conjugated_and_accumulating_products(ctx, cx):
+    """Y - X (X' Y): a product with a conjugate transpose on the left, one that accumulates
+    with alpha = -1."""
+    rng = np.random.default_rng(5)
+    X = _rand(rng, (150, 2, 141), cx, 0) / 17.0
+    Y = _rand(rng, (150, 2, 333), cx, 0)  # 1.4e7 products
+    yd = mpsgb.DeviceTensor.from_numpy(ctx, "mps", Y)
+    mpsgb.states.project_complement_(yd, mpsgb.DeviceTensor.from_numpy(ctx, "mps", X))
+    x, y = _wide(X.reshape(300, 141, order="F")), _wide(Y.reshape(300, 333, order="F"))
+    ref = y - x @ (x.conj().T @ y)
+    got = yd.numpy().reshape(300, 333, order="F")
+    assert np.linalg.norm((got - ref).astype(got.dtype)) <= 4e-15 * np.linalg.norm(
+        ref.astype(got.dtype))
+
+
+@pytest.mark.parametrize("cx", [False, True])
+def test_batched_products(ctx, cx):
+    """Both environment steps: a batch over MPO channels, right operand conjugated."""
+    rng = np.random.default_rng(6)
+    dt = np.complex128 if cx else np.float64
+    W = np.asarray(mpsgb.heisenberg_XXX(6, dtype=dt).W[2])
+    Dl, Dr = 93, 110
+    GL = _rand(rng, (Dl, W.shape[0], Dl), cx, 0)
+    GR = _rand(rng, (Dr, W.shape[3], Dr), cx, 0)
+    A = _rand(rng, (Dl, 2, Dr), cx, 0)
+    dev = lambda k, a: mpsgb.DeviceTensor.from_numpy(ctx, k, a)
+    left = mpsgb.transfer_left(dev("gl", GL), W, dev("mps", A)).numpy()
+    right = mpsgb.transfer_right(dev("gr", GR), W, dev("mps", A)).numpy()
+    rl = np.einsum("bwk,kta->bwta", GL, A, optimize=True)
+    rl = np.einsum("bwta,wstv->bsva", rl, W, optimize=True)
+    rl = np.einsum("bsva,bsc->cva", rl, A.conj(), optimize=True)
+    rr = np.einsum("atq,qvr->atvr", A, GR, optimize=True)
+    rr = np.einsum("atvr,wstv->awsr", rr, W, optimize=True)
+    rr = np.einsum("awsr,bsr->awb", rr, A.conj(), optimize=True)
+    assert np.linalg.norm(left - rl) <= 3e-15 * np.linalg.norm(rl)
+    assert np.linalg.norm(right - rr) <= 3e-15 * np.linalg.norm(rr)
+
+
+@pytest.mark.parametrize("cx", [False, True])
+def test_zero_blocks_and_extremes(ctx, cx):
+    """Exact zeros stay exact zeros; huge, tiny and subnormal rows keep their scale."""
+    rng = np.random.default_rng(7)
+    h, K, N = 160, 320, 200  # 2e7 products
+    A = _rand(rng, (2 * h, K), cx, 0)
+    B = _rand(rng, (K, N), cx, 0)
+    A[:130, 64:] = 0
+    A[200:] = 0
+    B[:64, 70:] = 0
+    B[192:256] = 0
+    A[5] *= 1e300
+    A[6] *= 1e-300
+    B[:, 3] *= 1e-20
+    A[7, :] = 0
+    A[8] *= 0
+    A[8, 3] = 5e-324
+    out = mpsgb.states.mul_tail(
+        mpsgb.DeviceTensor.from_numpy(ctx, "mps", A.reshape(h, 2, K, order="F")),
+        mpsgb.DeviceTensor.from_numpy(ctx, "bond", B)).numpy().reshape(2 * h, N, order="F")
+    ref = A @ B
+    assert np.array_equal(out == 0, (np.abs(A) != 0).astype(float) @ (np.abs(B) != 0) == 0) or \
+        np.all(out[(np.abs(A) != 0).astype(float) @ (np.abs(B) != 0) == 0] == 0)
+    for r in (5, 6, 0, 131):
+        assert np.linalg.norm(out[r] - ref[r]) <= 1e-14 * np.linalg.norm(ref[r]), r
+    assert np.all(np.abs(out[8] - ref[8]) <= 1e-323)
+
+
+@pytest.mark.parametrize("cx", [False, True])
+def test_non_finite_entries(ctx, cx):
+    """A row or column with Inf or NaN gives what FMAs give; the others are unaffected."""
+    rng = np.random.default_rng(8)
+    h, K, N = 160, 320, 160
+    A, B = _rand(rng, (2 * h, K), cx, 0), _rand(rng, (K, N), cx, 0)
+    clean = A @ B
+    A[17, 20] = np.inf
+    A[140, 30] = np.nan
+    B[50, 77] = np.nan
+    out = mpsgb.states.mul_tail(
+        mpsgb.DeviceTensor.from_numpy(ctx, "mps", A.reshape(h, 2, K, order="F")),
+        mpsgb.DeviceTensor.from_numpy(ctx, "bond", B)).numpy().reshape(2 * h, N, order="F")
+    bad = np.zeros(out.shape, bool)
+    bad[[17, 140]] = True
+    bad[:, 77] = True
+    assert not np.isfinite(out[bad]).any()
+    assert np.isnan(out[140]).all() and np.isnan(out[:, 77]).all()
+    assert np.linalg.norm((out - clean)[~bad]) <= 1e-14 * np.linalg.norm(clean[~bad])
