@@ -905,6 +905,8 @@ int gb_ctx_destroy(gb_ctx* ctx) {
     cusolverDnDestroy((cusolverDnHandle_t)ctx->solver);
   }
   if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
+  for (auto e : ctx->orth_done)
+    if (e) cudaEventDestroy(e);
   for (auto e : ctx->prof_events) cudaEventDestroy(e);
   for (auto e : ctx->trace_ev) cudaEventDestroy(e);
   if (ctx->trace_start) cudaEventDestroy(ctx->trace_start);
@@ -1302,6 +1304,16 @@ int gb_basis_orthogonalize(gb_ctx* ctx, const gb_tensor* basis, int64_t k, gb_te
   DevGuard g(ctx->device);
   const int dt = w->dtype;
   const int64_t n = basis->dims[0];
+  if (k >= 1 && n > 0 && krylov_orth_fits((int)std::min<int64_t>(k, 1 << 20))) {
+    std::vector<cplx> c(k);
+    double norm = 0.0;
+    krylov_orth(ctx, dt, n, (int)k, basis->data, w->data, nullptr, c.data(), &norm);
+    for (int64_t j = 0; j < k; ++j) {
+      h[2 * j] = c[j].re;
+      h[2 * j + 1] = c[j].im;
+    }
+    return GB_OK;
+  }
   // classical Gram-Schmidt, two passes; h = the sum of both passes' projections
   std::vector<cplx> c1(k), c2(k), neg(k);
   for (int pass = 0; pass < 2; ++pass) {

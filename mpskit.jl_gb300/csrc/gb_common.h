@@ -64,6 +64,7 @@ enum ScratchSlot {
 };
 
 struct LanePool;
+constexpr int ORTH_SLOTS = 4;  // Krylov steps in flight (krylov_orth_start)
 
 }  // namespace gb
 
@@ -80,6 +81,7 @@ struct gb_ctx {
   gb::Scratch scratch[gb::SLOT_COUNT];
   double* h_pinned = nullptr;    // small pinned host buffer for scalar readback
   size_t h_pinned_elems = 0;
+  cudaEvent_t orth_done[gb::ORTH_SLOTS] = {};  // end of the Krylov steps in flight
   int num_sms = 0;
   bool lane = false;             // an auxiliary lane context (its GPU is shared with the others)
   int aux_prec = GB_PREC_FP64;   // precision of auxiliary state contractions
@@ -268,6 +270,22 @@ void multi_dot(gb_ctx* ctx, int dtype, int64_t n, int k, const void* V, int64_t 
 // w[i] += sum_j V[i + ld*j] * coef[j] for j < k (coef from host)
 void multi_axpy(gb_ctx* ctx, int dtype, int64_t n, int k, const void* V, int64_t ld,
                 const cplx* coef, void* w);
+// One Krylov step (orth.cu): w against the k vectors V_j (leading dimension n); vnext = w / |w|
+// (null: w in place).  h: the k projections, summed over the passes; *norm = |w|.  Waits for the
+// result.
+void krylov_orth(gb_ctx* ctx, int dtype, int64_t n, int k, const void* V, void* w, void* vnext,
+                 cplx* h, double* norm);
+bool krylov_orth_fits(int k);
+// the same in two halves, so that the next step can be queued before this one's numbers are
+// looked at; `slot` < ORTH_SLOTS tells steps in flight apart.  predict: a Lanczos step that
+// follows the one before on this context
+void krylov_orth_start(gb_ctx* ctx, int dtype, int64_t n, int k, bool predict, const void* V,
+                       void* w, void* vnext, int slot);
+void krylov_orth_wait(gb_ctx* ctx, int k, int slot, cplx* h, double* norm);
+void krylov_combine(gb_ctx* ctx, int dtype, int64_t n, int k, const void* V, const cplx* coef,
+                    const void* src, void* dst, bool normalize, double* norm);
+// pinned host memory of at least `elems` doubles, for kernels that report scalars
+double* host_results(gb_ctx* ctx, size_t elems);
 // finite check: returns true when all entries are finite
 bool all_finite(gb_ctx* ctx, int dtype, int64_t n, const void* x);
 

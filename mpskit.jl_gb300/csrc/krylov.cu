@@ -2,7 +2,7 @@
 //
 // eigsolve: KrylovKit's Lanczos as MPSKit uses it through `fixedpoint`
 // (src/algorithms/fixedpoint.jl:15-18): start from x0/|x0|, one matvec per expansion,
-// full re-orthogonalisation (two classical Gram-Schmidt passes), diagonalise the
+// full re-orthogonalisation (orth.cu, one launch per step), diagonalise the
 // projected matrix when the space is full, when beta <= tol, or after every step when
 // `eager`; a Ritz pair is converged when |beta * U[K, i]| <= tol; thick restart keeps
 // (3*krylovdim + 2)/5 Ritz vectors at most `maxiter` times.
@@ -28,12 +28,13 @@ void heff_apply_raw(gb_heff* h, const void* x, void* y);
 int heff_precision(const gb_heff* h);
 
 // Cyclic Jacobi eigen-decomposition of a small real symmetric matrix (row-major n x n).
-// D ascending; U[:, j] (row-major U[i*n + j]) the eigenvector of D[j].
+// D ascending; U[:, j] (row-major U[i*n + j]) the eigenvector of D[j].  Off-diagonal entries
+// far below the stopping level are left alone (the last sweeps consist of little else).
 void sym_eig(int n, const std::vector<double>& Ain, std::vector<double>& D,
              std::vector<double>& U) {
   std::vector<double> A(Ain);
-  U.assign((size_t)n * n, 0.0);
-  for (int i = 0; i < n; ++i) U[i * n + i] = 1.0;
+  std::vector<double> Ut((size_t)n * n, 0.0);  // row p: eigenvector p
+  for (int i = 0; i < n; ++i) Ut[i * n + i] = 1.0;
   for (int sweep = 0; sweep < 100; ++sweep) {
     double off = 0.0, tot = 0.0;
     for (int i = 0; i < n; ++i)
@@ -43,28 +44,36 @@ void sym_eig(int n, const std::vector<double>& Ain, std::vector<double>& D,
         if (i != j) off += a;
       }
     if (off <= 1e-30 * std::max(tot, 1e-300)) break;
+    const double skip = 1e-19 * std::sqrt(tot);
     for (int p = 0; p < n; ++p)
       for (int q = p + 1; q < n; ++q) {
-        double apq = A[p * n + q];
-        if (std::fabs(apq) < 1e-300) continue;
-        double app = A[p * n + p], aqq = A[q * n + q];
-        double theta = (aqq - app) / (2.0 * apq);
-        double t = (theta >= 0 ? 1.0 : -1.0) / (std::fabs(theta) + std::sqrt(theta * theta + 1.0));
-        double c = 1.0 / std::sqrt(t * t + 1.0), s = t * c;
-        for (int k = 0; k < n; ++k) {  // A <- J^T A J
-          double akp = A[k * n + p], akq = A[k * n + q];
-          A[k * n + p] = c * akp - s * akq;
-          A[k * n + q] = s * akp + c * akq;
+        const double apq = A[p * n + q];
+        if (std::fabs(apq) < 1e-300 || std::fabs(apq) <= skip) continue;
+        const double app = A[p * n + p], aqq = A[q * n + q];
+        const double theta = (aqq - app) / (2.0 * apq);
+        const double t =
+            (theta >= 0 ? 1.0 : -1.0) / (std::fabs(theta) + std::sqrt(theta * theta + 1.0));
+        const double c = 1.0 / std::sqrt(t * t + 1.0), s = t * c;
+        double* __restrict__ rp = &A[p * n];
+        double* __restrict__ rq = &A[q * n];
+        for (int k = 0; k < n; ++k) {  // rows p and q of J^T A: those of J^T A J off p and q
+          const double x = rp[k], y = rq[k];
+          rp[k] = c * x - s * y;
+          rq[k] = s * x + c * y;
         }
-        for (int k = 0; k < n; ++k) {
-          double apk = A[p * n + k], aqk = A[q * n + k];
-          A[p * n + k] = c * apk - s * aqk;
-          A[q * n + k] = s * apk + c * aqk;
+        rp[p] = app - t * apq;
+        rq[q] = aqq + t * apq;
+        rp[q] = rq[p] = 0.0;
+        for (int k = 0; k < n; ++k) {  // the columns follow by symmetry
+          A[k * n + p] = rp[k];
+          A[k * n + q] = rq[k];
         }
+        double* __restrict__ up = &Ut[p * n];
+        double* __restrict__ uq = &Ut[q * n];
         for (int k = 0; k < n; ++k) {
-          double ukp = U[k * n + p], ukq = U[k * n + q];
-          U[k * n + p] = c * ukp - s * ukq;
-          U[k * n + q] = s * ukp + c * ukq;
+          const double x = up[k], y = uq[k];
+          up[k] = c * x - s * y;
+          uq[k] = s * x + c * y;
         }
       }
   }
@@ -72,39 +81,107 @@ void sym_eig(int n, const std::vector<double>& Ain, std::vector<double>& D,
   for (int i = 0; i < n; ++i) idx[i] = i;
   std::sort(idx.begin(), idx.end(), [&](int a, int b) { return A[a * n + a] < A[b * n + b]; });
   D.resize(n);
-  std::vector<double> U2((size_t)n * n);
+  U.assign((size_t)n * n, 0.0);
   for (int j = 0; j < n; ++j) {
     D[j] = A[idx[j] * n + idx[j]];
-    for (int i = 0; i < n; ++i) U2[i * n + j] = U[i * n + idx[j]];
+    for (int i = 0; i < n; ++i) U[i * n + j] = Ut[idx[j] * n + i];
   }
-  U.swap(U2);
 }
 
-struct KrylovWork {
-  void* V = nullptr;  // (kd+1) vectors of n elements
-  void* w = nullptr;
-  void* tmp = nullptr;
-};
-
-static void orthogonalize(gb_ctx* ctx, int dtype, int64_t n, int k, void* V, void* w,
-                          std::vector<cplx>& h) {
-  std::vector<cplx> c(k), c2(k);
-  multi_dot(ctx, dtype, n, k, V, n, w, c.data());
-  std::vector<cplx> neg(k);
-  for (int j = 0; j < k; ++j) neg[j] = cplx{-c[j].re, -c[j].im};
-  multi_axpy(ctx, dtype, n, k, V, n, neg.data(), w);
-  multi_dot(ctx, dtype, n, k, V, n, w, c2.data());
-  for (int j = 0; j < k; ++j) neg[j] = cplx{-c2[j].re, -c2[j].im};
-  multi_axpy(ctx, dtype, n, k, V, n, neg.data(), w);
-  h.resize(k);
-  for (int j = 0; j < k; ++j) h[j] = cplx{c[j].re + c2[j].re, c[j].im + c2[j].im};
-}
-
-// x <- sum_j coef[j] V[j]
-static void combine(gb_ctx* ctx, int dtype, int64_t n, int k, const void* V,
-                    const std::vector<cplx>& coef, void* x) {
-  fill_zero(ctx, x, (size_t)n * elem_size(dtype));
-  multi_axpy(ctx, dtype, n, k, V, n, coef.data(), x);
+// The same by Householder tridiagonalisation and the implicit QL iteration (Golub & Van Loan,
+// Matrix Computations, sections 8.3-8.4), for callers that need no particular sign of the
+// eigenvectors: D ascending and, for the rows i0..n-1 of the eigenvector matrix only,
+// Z[(i - i0) * n + j].  With the last row alone a convergence test costs 4/3 n^3 instead of the
+// ~50 n^3 of the Jacobi sweeps.  False if an eigenvalue does not converge.
+static bool sym_eig_rows(int n, const std::vector<double>& Ain, int i0, std::vector<double>& D,
+                         std::vector<double>& Z) {
+  std::vector<double> A(Ain), d(n), e(n, 0.0), v(n), p(n);
+  const int nr = n - i0;
+  Z.assign((size_t)nr * n, 0.0);
+  for (int i = 0; i < nr; ++i) Z[i * n + i0 + i] = 1.0;
+  for (int k = 0; k + 2 < n; ++k) {  // reflect column k below the subdiagonal away
+    double sigma = 0.0;
+    for (int i = k + 2; i < n; ++i) sigma += A[i * n + k] * A[i * n + k];
+    if (sigma == 0.0) continue;
+    const double x0 = A[(k + 1) * n + k], mu = std::sqrt(x0 * x0 + sigma);
+    const double v0 = x0 <= 0 ? x0 - mu : -sigma / (x0 + mu);
+    const double beta = 2.0 * v0 * v0 / (sigma + v0 * v0);
+    v[k + 1] = 1.0;
+    for (int i = k + 2; i < n; ++i) v[i] = A[i * n + k] / v0;
+    double pv = 0.0;
+    for (int i = k + 1; i < n; ++i) {
+      double acc = 0.0;
+      for (int j = k + 1; j < n; ++j) acc += A[i * n + j] * v[j];
+      p[i] = beta * acc;
+      pv += p[i] * v[i];
+    }
+    const double h = 0.5 * beta * pv;
+    for (int i = k + 1; i < n; ++i) p[i] -= h * v[i];
+    for (int i = k + 1; i < n; ++i)
+      for (int j = k + 1; j < n; ++j) A[i * n + j] -= v[i] * p[j] + p[i] * v[j];
+    A[(k + 1) * n + k] = mu;
+    for (int r = 0; r < nr; ++r) {  // Z <- Z (1 - beta v v')
+      double acc = 0.0;
+      for (int i = k + 1; i < n; ++i) acc += Z[r * n + i] * v[i];
+      acc *= beta;
+      for (int i = k + 1; i < n; ++i) Z[r * n + i] -= acc * v[i];
+    }
+  }
+  for (int i = 0; i < n; ++i) d[i] = A[i * n + i];
+  for (int i = 0; i + 1 < n; ++i) e[i] = A[(i + 1) * n + i];
+  for (int l = 0; l < n; ++l) {
+    for (int it = 0;; ++it) {
+      int m = l;  // the block l..m does not decouple before m
+      for (; m + 1 < n; ++m)
+        if (std::fabs(e[m]) <= 1.1e-16 * (std::fabs(d[m]) + std::fabs(d[m + 1])) + 1e-300) break;
+      if (m == l) break;
+      if (it == 60) return false;
+      // shift: the eigenvalue of the leading 2 x 2 block closer to d[l]
+      double g = (d[l + 1] - d[l]) / (2.0 * e[l]);
+      double r = std::hypot(g, 1.0);
+      g = d[m] - d[l] + e[l] / (g + (g >= 0 ? r : -r));
+      double s = 1.0, c = 1.0, q = 0.0;
+      int i = m - 1;
+      for (; i >= l; --i) {  // chase the bulge up with rotations of columns i, i + 1
+        double f = s * e[i];
+        const double b = c * e[i];
+        r = std::hypot(f, g);
+        e[i + 1] = r;
+        if (r == 0.0) {
+          d[i + 1] -= q;
+          e[m] = 0.0;
+          break;
+        }
+        s = f / r;
+        c = g / r;
+        g = d[i + 1] - q;
+        r = (d[i] - g) * s + 2.0 * c * b;
+        q = s * r;
+        d[i + 1] = g + q;
+        g = c * r - b;
+        for (int k = 0; k < nr; ++k) {
+          f = Z[k * n + i + 1];
+          Z[k * n + i + 1] = s * Z[k * n + i] + c * f;
+          Z[k * n + i] = c * Z[k * n + i] - s * f;
+        }
+      }
+      if (i >= l) continue;
+      d[l] -= q;
+      e[l] = g;
+      e[m] = 0.0;
+    }
+  }
+  std::vector<int> idx(n);
+  for (int i = 0; i < n; ++i) idx[i] = i;
+  std::sort(idx.begin(), idx.end(), [&](int a, int b) { return d[a] < d[b]; });
+  D.resize(n);
+  std::vector<double> Zs((size_t)nr * n);
+  for (int j = 0; j < n; ++j) {
+    D[j] = d[idx[j]];
+    for (int r = 0; r < nr; ++r) Zs[r * n + j] = Z[r * n + idx[j]];
+  }
+  Z.swap(Zs);
+  return true;
 }
 
 // The vector space of a solve: the dense vectors of the operator, or -- for a U(1)
@@ -149,42 +226,59 @@ int heff_eigsolve_raw(gb_ctx* ctx, gb_heff* h, int64_t n_dense, int dtype, void*
   void* w = scratch(ctx, SLOT_KRYLOV_W, (size_t)n * es);
   auto vec = [&](int j) { return (void*)(V + (size_t)j * n * es); };
   sp.load(ctx, dtype, x, vec(0));
-  double nx = nrm2(ctx, dtype, n, vec(0));
+  double nx = 0.0;
+  krylov_combine(ctx, dtype, n, 0, nullptr, nullptr, vec(0), vec(0), true, &nx);
   if (!std::isfinite(nx)) throw Error(GB_ERR_NAN, "eigsolve: initial vector is not finite");
   GB_REQUIRE(nx > 0, "eigsolve: initial vector has zero norm");
-  scale(ctx, dtype, n, cplx{1.0 / nx, 0}, vec(0));
   const int howmany = 1;
   std::vector<double> H((size_t)(kd + 1) * (kd + 1), 0.0);  // row-major, stride kd+1
   const int LD = kd + 1;
   int K = 0, numops = 0, numiter = 1, converged = 0;
   double beta = 0.0;
-  std::vector<double> D, U;
+  std::vector<double> D, U, Z;
   std::vector<double> f;
+  std::vector<cplx> hc(kd + 1);
+  bool fresh = true;  // the next step couples to every vector (the first, or after a restart)
   // With split-precision contractions the residual cannot fall below the operator's own
   // accuracy (~1e-6 relative); two restarts in a row that do not bring it 10% below the
   // best value so far end the solve (reported as not converged, as when maxiter runs out)
   // instead of spending the remaining restarts on rounding noise.  A single slow restart of
   // a hard problem does not.  FP64 operators keep KrylovKit's plain maxiter rule.
   const bool split = heff_precision(h) != GB_PREC_FP64;
+  // Short vectors queue the next step before this one is checked: a step of up to 4 MB is
+  // 40-110 us and the host's share of it 15-50 us, so a solve that ends early loses one step
+  // (of typically ten) and every other one gains.  Longer steps hide the host by themselves.
+  const bool ahead = (size_t)n * es <= ((size_t)4 << 20);
+  int queued = 0;  // steps queued so far
+  auto issue = [&](int k, bool predict) {
+    sp.apply(vec(k), w);
+    krylov_orth_start(ctx, dtype, n, k + 1, predict, V, w, vec(k + 1), k % ORTH_SLOTS);
+    queued = k + 1;
+  };
   double best_res = INFINITY;
   int stalls = 0;
   while (true) {
-    sp.apply(vec(K), w);
+    if (queued <= K) issue(K, !fresh);
+    fresh = false;
+    // one step ahead: its matvec runs while the host looks at this step's numbers
+    if (ahead && K + 1 < kd) issue(K + 1, true);
+    krylov_orth_wait(ctx, K + 1, K % ORTH_SLOTS, hc.data(), &beta);
     ++numops;
-    std::vector<cplx> hc;
-    orthogonalize(ctx, dtype, n, K + 1, V, w, hc);
     for (int i = 0; i <= K; ++i) {
       H[i * LD + K] = hc[i].re;
       H[K * LD + i] = hc[i].re;
     }
     ++K;
-    beta = nrm2(ctx, dtype, n, w);
     if (!std::isfinite(beta))
       throw Error(GB_ERR_NAN, "eigsolve: non-finite residual (NaN or Inf in the operator)");
     if (K == kd || beta <= tol || (eager && K >= howmany)) {
       std::vector<double> Hk((size_t)K * K);
       for (int i = 0; i < K; ++i)
         for (int j = 0; j < K; ++j) Hk[i * K + j] = H[i * LD + j];
+      // the residual of the lowest Ritz pair first; the vectors only once they are used
+      if (K < kd && beta > tol && sym_eig_rows(K, Hk, K - 1, D, Z) &&
+          std::fabs(beta * Z[0]) > tol)
+        continue;
       sym_eig(K, Hk, D, U);
       f.assign(K, 0.0);
       for (int i = 0; i < K; ++i) f[i] = beta * U[(K - 1) * K + i];
@@ -192,11 +286,7 @@ int heff_eigsolve_raw(gb_ctx* ctx, gb_heff* h, int64_t n_dense, int dtype, void*
       while (converged < K && std::fabs(f[converged]) <= tol) ++converged;
       if (converged >= howmany || beta <= tol) break;
     }
-    if (K < kd) {
-      GB_CHECK_CUDA(cudaMemcpyAsync(vec(K), w, n * es, cudaMemcpyDeviceToDevice, ctx->stream));
-      scale(ctx, dtype, n, cplx{1.0 / beta, 0}, vec(K));
-      continue;
-    }
+    if (K < kd) continue;
     if (numiter == maxiter) break;
     if (split) {
       const double res = std::fabs(f[0]);
@@ -214,7 +304,8 @@ int heff_eigsolve_raw(gb_ctx* ctx, gb_heff* h, int64_t n_dense, int dtype, void*
     for (int j = 0; j < keep; ++j) {
       std::vector<cplx> coef(K);
       for (int i = 0; i < K; ++i) coef[i] = cplx{U[i * K + j], 0.0};
-      combine(ctx, dtype, n, K, V, coef, (char*)tmp + (size_t)j * n * es);
+      krylov_combine(ctx, dtype, n, K, V, coef.data(), nullptr, (char*)tmp + (size_t)j * n * es,
+                     false, nullptr);
     }
     GB_CHECK_CUDA(cudaMemcpyAsync(V, tmp, (size_t)keep * n * es, cudaMemcpyDeviceToDevice,
                                   ctx->stream));
@@ -224,17 +315,17 @@ int heff_eigsolve_raw(gb_ctx* ctx, gb_heff* h, int64_t n_dense, int dtype, void*
       H[keep * LD + j] = f[j];
       H[j * LD + keep] = f[j];
     }
-    GB_CHECK_CUDA(cudaMemcpyAsync(vec(keep), w, n * es, cudaMemcpyDeviceToDevice, ctx->stream));
-    scale(ctx, dtype, n, cplx{1.0 / beta, 0}, vec(keep));
+    GB_CHECK_CUDA(cudaMemcpyAsync(vec(keep), vec(kd), n * es, cudaMemcpyDeviceToDevice,
+                                  ctx->stream));
     K = keep;
+    queued = keep;
+    fresh = true;
     ++numiter;
   }
   std::vector<cplx> coef(K);
   for (int i = 0; i < K; ++i) coef[i] = cplx{U[i * K + 0], 0.0};
-  combine(ctx, dtype, n, K, V, coef, w);
-  double nn = nrm2(ctx, dtype, n, w);
-  scale(ctx, dtype, n, cplx{1.0 / nn, 0}, w);
-  sp.store(ctx, dtype, w, x);
+  krylov_combine(ctx, dtype, n, K, V, coef.data(), nullptr, sp.compact ? w : x, true, nullptr);
+  if (sp.compact) sp.store(ctx, dtype, w, x);
   *lambda = D[0];
   if (info) {
     info->converged = converged;
@@ -266,37 +357,37 @@ int heff_exponentiate_raw(gb_ctx* ctx, gb_heff* h, int64_t n_dense, int dtype, v
   char* V = (char*)scratch(ctx, SLOT_KRYLOV, (size_t)(kd + 1) * n * es);
   void* w = scratch(ctx, SLOT_KRYLOV_W, (size_t)n * es);
   auto vec = [&](int j) { return (void*)(V + (size_t)j * n * es); };
+  const int ahead = (size_t)n * es <= ((size_t)4 << 20) ? ORTH_SLOTS - 1 : 0;
   const std::complex<double> total(t_re, t_im);
+  std::vector<cplx> hc(kd + 1);
   double tau_left = 1.0, tau = 1.0;
   int numops = 0, numiter = 0;
   const int maxsteps = std::max(1, maxiter) * 50;
   while (tau_left > 0 && numiter < maxsteps) {
     ++numiter;
-    double nrm = nrm2(ctx, dtype, n, x);
+    double nrm = 0.0;
+    krylov_combine(ctx, dtype, n, 0, nullptr, nullptr, x, vec(0), true, &nrm);
     if (nrm == 0.0) break;
-    GB_CHECK_CUDA(cudaMemcpyAsync(vec(0), x, n * es, cudaMemcpyDeviceToDevice, ctx->stream));
-    scale(ctx, dtype, n, cplx{1.0 / nrm, 0}, vec(0));
     std::vector<double> alphas, betas;
     int K = 0;
     bool happy = false;
+    int queued = 0;
     for (int j = 0; j < kd; ++j) {
-      sp.apply(vec(j), w);
+      // nothing but a breakdown ends the expansion early: short vectors run ahead of the host
+      for (; queued <= std::min(j + ahead, kd - 1); ++queued) {
+        sp.apply(vec(queued), w);
+        krylov_orth_start(ctx, dtype, n, queued + 1, queued > 0, V, w, vec(queued + 1),
+                          queued % ORTH_SLOTS);
+      }
+      double b = 0.0;
+      krylov_orth_wait(ctx, j + 1, j % ORTH_SLOTS, hc.data(), &b);
       ++numops;
-      std::vector<cplx> hc;
-      orthogonalize(ctx, dtype, n, j + 1, V, w, hc);
-      double a = hc[j].re;
-      double b = nrm2(ctx, dtype, n, w);
-      alphas.push_back(a);
+      alphas.push_back(hc[j].re);
       betas.push_back(b);
       K = j + 1;
       if (b <= tol * 1e-3) {
         happy = true;
         break;
-      }
-      if (j + 1 < kd + 1) {
-        GB_CHECK_CUDA(cudaMemcpyAsync(vec(j + 1), w, n * es, cudaMemcpyDeviceToDevice,
-                                      ctx->stream));
-        scale(ctx, dtype, n, cplx{1.0 / b, 0}, vec(j + 1));
       }
     }
     std::vector<double> T((size_t)K * K, 0.0), D, U;
@@ -304,7 +395,7 @@ int heff_exponentiate_raw(gb_ctx* ctx, gb_heff* h, int64_t n_dense, int dtype, v
       T[i * K + i] = alphas[i];
       if (i + 1 < K) T[i * K + i + 1] = T[(i + 1) * K + i] = betas[i];
     }
-    sym_eig(K, T, D, U);
+    if (!sym_eig_rows(K, T, 0, D, U)) sym_eig(K, T, D, U);
     tau = std::min(tau, tau_left);
     std::vector<std::complex<double>> c(K);
     while (true) {
@@ -321,7 +412,7 @@ int heff_exponentiate_raw(gb_ctx* ctx, gb_heff* h, int64_t n_dense, int dtype, v
     for (int i = 0; i < K; ++i) coef[i] = cplx{nrm * c[i].real(), nrm * c[i].imag()};
     if (!is_cplx(dtype))
       for (auto& q : coef) q.im = 0.0;
-    combine(ctx, dtype, n, K, V, coef, x);
+    krylov_combine(ctx, dtype, n, K, V, coef.data(), nullptr, x, false, nullptr);
     tau_left -= tau;
     if (tau_left < 1e-15) tau_left = 0.0;
     tau = std::min(2 * tau, 1.0);
@@ -390,13 +481,15 @@ int env_linsolve_raw(gb_ctx* ctx, int side, const gb_tensor* W, const gb_tensor*
   };
   const bool split = prec != GB_PREC_FP64;
   const bool cx = is_cplx(dt);
+  std::vector<cplx> hc(kd + 1);
   double res = INFINITY, last = INFINITY;
   int it = 0, converged = 0;
   for (it = 0; it < std::max(1, maxiter); ++it) {
     // r = b - (x - T x)
     apply(x->data, w);
     axpy(ctx, dt, n, cplx{-1.0, 0.0}, b->data, w);  // w = (x - T x) - b
-    const double beta = nrm2(ctx, dt, n, w);
+    double beta = 0.0;
+    krylov_combine(ctx, dt, n, 0, nullptr, nullptr, w, vec(0), true, &beta);
     res = beta;
     if (beta <= tol) {
       converged = 1;
@@ -404,18 +497,15 @@ int env_linsolve_raw(gb_ctx* ctx, int side, const gb_tensor* W, const gb_tensor*
     }
     if (split && beta > 0.9 * last) break;
     last = beta;
-    GB_CHECK_CUDA(cudaMemcpyAsync(vec(0), w, (size_t)n * es, cudaMemcpyDeviceToDevice,
-                                  ctx->stream));
-    scale(ctx, dt, n, cplx{-1.0 / beta, 0.0}, vec(0));  // V0 = r / beta
+    scale(ctx, dt, n, cplx{-1.0, 0.0}, vec(0));  // V0 = r / beta
     std::vector<std::vector<zc>> R;                       // rotated Hessenberg columns
     std::vector<double> cs;
     std::vector<zc> sn, g(1, zc(beta, 0.0));
     int k = 0;
     for (int j = 0; j < kd; ++j) {
       apply(vec(j), w);
-      std::vector<cplx> hc;
-      orthogonalize(ctx, dt, n, j + 1, V, w, hc);
-      const double hn = nrm2(ctx, dt, n, w);
+      double hn = 0.0;
+      krylov_orth(ctx, dt, n, j + 1, V, w, vec(j + 1), hc.data(), &hn);
       std::vector<zc> h(j + 2);
       for (int i = 0; i <= j; ++i) h[i] = zc(hc[i].re, cx ? hc[i].im : 0.0);
       h[j + 1] = zc(hn, 0.0);
@@ -446,11 +536,6 @@ int env_linsolve_raw(gb_ctx* ctx, int side, const gb_tensor* W, const gb_tensor*
       k = j + 1;
       res = std::abs(g[j + 1]);
       if (res <= tol || hn < 1e-300) break;
-      if (j + 1 < kd) {
-        GB_CHECK_CUDA(cudaMemcpyAsync(vec(j + 1), w, (size_t)n * es, cudaMemcpyDeviceToDevice,
-                                      ctx->stream));
-        scale(ctx, dt, n, cplx{1.0 / hn, 0.0}, vec(j + 1));
-      }
     }
     // R y = g (upper triangular, columns R[j][0..j]); x += sum_i y_i V_i
     std::vector<zc> y(k);
