@@ -68,7 +68,7 @@ __device__ inline void load_elem(const PackArgs& p, const double* src, int64_t r
   if (p.cplx) {
     re = src[2 * addr];
     im = src[2 * addr + 1];
-    if (p.op == 'C') im = -im;
+    if (p.op == 'C') im = __longlong_as_double(__double_as_longlong(im) ^ (1ll << 63));
   } else {
     re = src[addr];
     im = 0.0;
@@ -110,10 +110,11 @@ __global__ void pack_kernel(PackArgs p, const double* __restrict__ src, E* __res
   for (int j = ty; j < 32; j += 8) {
     int64_t r = r0 + j, k = k0 + tx;
     if (r >= p.R || k >= p.Kh) continue;  // entries k >= K were loaded as zeros
-    double re = tre[j][tx], im = tim[j][tx];
-    nz |= (re != 0.0 || im != 0.0);
-    auto put = [&](int64_t row, int64_t col, double v) {
-      split_put_f(hi, lo, row * p.Kp + col, (float)v);
+    const double dre = tre[j][tx], dim = tim[j][tx];
+    nz |= ((__double_as_longlong(dre) | __double_as_longlong(dim)) << 1) != 0;
+    const float re = to_float(dre), im = p.cplx ? to_float(dim) : 0.f;
+    auto put = [&](int64_t row, int64_t col, float v) {
+      split_put_f(hi, lo, row * p.Kp + col, v);
     };
     if (!p.cplx) {
       put(r, k, re);
@@ -268,63 +269,99 @@ void pack_operand(gb_ctx* ctx, int dtype, int role, char op, int64_t R, int64_t 
 // y[a + out_off[J] + n*yn] = sum_e val[e] x[a + in_off[col[e]] + n*xn] written directly as
 // the packed B operand of the following GEMM: logical B element (k, m) with
 // k = a + kJ[J] (contraction index) and m = mJ[J] + n*mn (output column index).
+//
+// A block takes one output row J and a run of columns n; a thread takes four entries of each.
+// Bound, once the map is marked with one atomic per run and warp instead of one per 32 entries
+// (all of them on a few hundred words), by the FP64 sum (16 clocks per warp instruction and
+// SM) and by the traffic, 4 B read per entry and input and 4 B (BF16) written: 12.4 M entries,
+// one input each, 356 us before, NN us.
+constexpr int MIXE = 64;  // entries of a row kept in shared memory
+constexpr int MIXU = 4;   // entries of a column per thread
 template <bool CPLX, typename E, typename TX>
-__global__ void mixpack_kernel(int64_t A, int64_t N, int64_t xn, const int64_t* __restrict__ in_off,
-                               const int64_t* __restrict__ kJ, const int64_t* __restrict__ mJ,
-                               int64_t mn, const int* __restrict__ row_ptr,
-                               const int* __restrict__ col, const double* __restrict__ val,
-                               const TX* __restrict__ x, E* __restrict__ hi, int64_t Nlog,
-                               int64_t Kp, int64_t Kh, int64_t plane, uint32_t* __restrict__ mask,
-                               int kw, MixSkipDev sk) {
+__global__ void __launch_bounds__(128)
+    mixpack_kernel(int64_t A, int64_t N, int64_t xn, const int64_t* __restrict__ in_off,
+                   const int64_t* __restrict__ kJ, const int64_t* __restrict__ mJ, int64_t mn,
+                   const int* __restrict__ row_ptr, const int* __restrict__ col,
+                   const double* __restrict__ val, const TX* __restrict__ x, E* __restrict__ hi,
+                   int64_t Nlog, int64_t Kp, int64_t Kh, int64_t plane,
+                   uint32_t* __restrict__ mask, int kw, MixSkipDev sk, int64_t nper) {
   constexpr int BK = bk_of<E>();
+  __shared__ int64_t s_in[MIXE], s_roff[MIXE], s_coff[MIXE];
+  __shared__ double s_val[(CPLX ? 2 : 1) * MIXE];
   const int J = blockIdx.y;
-  const int e0 = row_ptr[J], e1 = row_ptr[J + 1];
+  const int e0 = row_ptr[J], ne = row_ptr[J + 1] - e0;
   const int lane = threadIdx.x % 32;
   E* lo = hi + plane;
-  auto put = [&](int64_t row, int64_t c, double v) { split_put_f(hi, lo, row * Kp + c, (float)v); };
-  auto mark = [&](int64_t row, int64_t kb) {
-    atomicOr(&mask[(row / MASK_ROWS) * kw + kb / 32], 1u << (kb % 32));
+  for (int e = threadIdx.x; e < min(ne, MIXE); e += 128) {
+    const int i = col[e0 + e];
+    s_in[e] = in_off[i];
+    if (sk.xmap) {
+      s_roff[e] = sk.roff[i];
+      s_coff[e] = sk.coff[i];
+    }
+    s_val[CPLX ? 2 * e : e] = val[CPLX ? 2 * (e0 + e) : e0 + e];
+    if (CPLX) s_val[2 * e + 1] = val[2 * (e0 + e) + 1];
+  }
+  __syncthreads();
+  auto in_of = [&](int e) { return e < MIXE ? s_in[e] : in_off[col[e0 + e]]; };
+  auto val_of = [&](int e, int p) {
+    return e < MIXE ? s_val[CPLX ? 2 * e + p : e] : val[CPLX ? 2 * (e0 + e) + p : e0 + e];
   };
-  for (int64_t n = blockIdx.z; n < N; n += gridDim.z) {
-    const int64_t m = mJ[J] + n * mn;
+  auto put = [&](int64_t row, int64_t c, double v) {
+    split_put_f(hi, lo, row * Kp + c, to_float(v));
+  };
+  const int64_t k0J = kJ[J], m0J = mJ[J];
+  const int64_t n0 = (int64_t)blockIdx.z * nper, n1 = min(N, n0 + nper);
+  // k-blocks already marked in the row tile that the last column fell into, per run of 32
+  // entries (they span two k-blocks at most): bit 2 u + (second block)
+  int64_t tile = -1, tile_im = -1;
+  int64_t base_marked = -1;
+  uint32_t marked = 0;
+  for (int64_t n = n0; n < n1; ++n) {
+    const int64_t m = m0J + n * mn;
+    if (m / MASK_ROWS != tile || (CPLX && (Nlog + m) / MASK_ROWS != tile_im)) {
+      tile = m / MASK_ROWS;
+      tile_im = CPLX ? (Nlog + m) / MASK_ROWS : -1;
+      marked = 0;
+    }
     // U(1): only the l' sector of (J, n) can be nonzero; every entry of it is written on
     // every call, and the rest of the operand stays zero from its allocation
-    int64_t lo = 0, hi = A;
+    int64_t alo = 0, ahi = A;
     if (sk.arange) {
       const int2 r = sk.arange[n * gridDim.y + J];
-      lo = r.x;
-      hi = r.y;
+      alo = r.x;
+      ahi = r.y;
     }
-    // every thread of the block runs the same number of iterations (warp-wide votes below)
-    for (int64_t base = lo + blockIdx.x * (int64_t)blockDim.x; base < hi;
-         base += (int64_t)gridDim.x * blockDim.x) {
-      const int64_t a = base + threadIdx.x;
-      bool valid = a < hi;
-      const int64_t k = a + kJ[J];
-      bool nz = false;
-      // input e of element (a, n) lies in box (row, column) of x's written-region map; the
-      // producer keeps every region outside the map at zero
-      auto box_set = [&](int i, int64_t row) {
-        const int64_t bit = ((row + sk.roff[i]) >> 7) * sk.onc + ((sk.coff[i] + n * sk.xnM) >> 7);
-        return ((sk.xmap[bit >> 5] >> (bit & 31)) & 1u) != 0u;
-      };
-      if (sk.xmap && !sk.arange) {
-        // warp-wide test first: the warp's 32 rows span at most two row boxes per input, so
-        // one pass of the lanes over the inputs decides whether anything is there to read
-        const int64_t wa0 = base + (threadIdx.x & ~31);
-        const int64_t wa1 = (wa0 + 31 < A ? wa0 + 31 : A - 1);
-        bool hit = false;
-        if (wa0 < A)
-          for (int e = e0 + lane; e < e1 && !hit; e += 32) {
-            const int i = col[e];
-            hit = box_set(i, wa0) || box_set(i, wa1);
+    for (int64_t base = alo + (int64_t)blockIdx.x * (128 * MIXU); base < ahi;
+         base += (int64_t)gridDim.x * (128 * MIXU)) {
+      if (base != base_marked) {  // another piece of the column: its k-blocks are others
+        base_marked = base;
+        marked = 0;
+      }
+      // a warp's run u: 32 entries from a0
+      bool hit[MIXU];
+#pragma unroll
+      for (int u = 0; u < MIXU; ++u) {
+        const int64_t a0 = base + u * 128 + (threadIdx.x & ~31);
+        hit[u] = a0 < ahi;
+        if (sk.xmap && !sk.arange && hit[u]) {
+          // input e of element (a, n) lies in box (row, column) of x's written-region map; the
+          // producer keeps every region outside the map at zero.  The run spans at most two
+          // row boxes per input, so one pass of the lanes over the inputs decides.
+          const int64_t a1 = min(a0 + 31, A - 1);
+          bool h = false;
+          for (int e = lane; e < ne && !h; e += 32) {
+            const int64_t ro = e < MIXE ? s_roff[e] : sk.roff[col[e0 + e]];
+            const int64_t co = e < MIXE ? s_coff[e] : sk.coff[col[e0 + e]];
+            const int64_t cb = (co + n * sk.xnM) >> 7;
+            const int64_t q0 = ((a0 + ro) >> 7) * sk.onc + cb, q1 = ((a1 + ro) >> 7) * sk.onc + cb;
+            h = ((sk.xmap[q0 >> 5] >> (q0 & 31)) & 1u) || ((sk.xmap[q1 >> 5] >> (q1 & 31)) & 1u);
           }
-        hit = __any_sync(0xffffffffu, hit);
-        if (!hit) {
-          // nothing to read: the output is zero; it is written only where the previous
-          // apply marked its box (the planes hold zeros everywhere else)
-          if (valid) {
-            const int64_t kb0 = k / BK;
+          hit[u] = __any_sync(0xffffffffu, h);
+          if (!hit[u] && a0 + lane < A) {
+            // nothing to read: the output is zero; it is written only where the previous
+            // apply marked its box (the planes hold zeros everywhere else)
+            const int64_t k = a0 + lane + k0J, kb0 = k / BK;
             auto prev = [&](int64_t row, int64_t kb) {
               return (sk.prev[(row / MASK_ROWS) * kw + kb / 32] >> (kb % 32)) & 1u;
             };
@@ -335,42 +372,62 @@ __global__ void mixpack_kernel(int64_t A, int64_t N, int64_t xn, const int64_t* 
               if (prev(Nlog + m, kb0 + Kh / BK)) put(Nlog + m, Kh + k, 0.0);
             }
           }
-          valid = false;  // nothing to compute or mark
         }
       }
-      if (valid) {
-        if (CPLX) {
-          double re = 0.0, im = 0.0;
-          for (int e = e0; e < e1; ++e) {
-            const TX* xv = x + 2 * (a + in_off[col[e]] + n * xn);
-            const double xr = xv[0], xi = xv[1];
-            double vr = val[2 * e], vi = val[2 * e + 1];
-            re = fma(vr, xr, fma(-vi, xi, re));
-            im = fma(vr, xi, fma(vi, xr, im));
+      double re[MIXU], im[MIXU];
+#pragma unroll
+      for (int u = 0; u < MIXU; ++u) re[u] = im[u] = 0.0;
+      const int64_t a = base + threadIdx.x;
+      for (int e = 0; e < ne; ++e) {
+        const TX* xe = x + (CPLX ? 2 : 1) * (in_of(e) + n * xn);
+        const double vr = val_of(e, 0), vi = CPLX ? val_of(e, 1) : 0.0;
+#pragma unroll
+        for (int u = 0; u < MIXU; ++u) {
+          if (!hit[u] || a + u * 128 >= ahi) continue;
+          if (CPLX) {
+            const double xr = to_double(xe[2 * (a + u * 128)]), xi = to_double(xe[2 * (a + u * 128) + 1]);
+            re[u] = fma(vr, xr, fma(-vi, xi, re[u]));
+            im[u] = fma(vr, xi, fma(vi, xr, im[u]));
+          } else {
+            re[u] = fma(vr, to_double(xe[a + u * 128]), re[u]);
           }
-          put(m, k, re);
-          put(m, Kh + k, -im);
-          put(Nlog + m, k, im);
-          put(Nlog + m, Kh + k, re);
-          nz = (re != 0.0 || im != 0.0);
-        } else {
-          double acc = 0.0;
-          for (int e = e0; e < e1; ++e)
-            acc = fma(val[e], (double)x[a + in_off[col[e]] + n * xn], acc);
-          put(m, k, acc);
-          nz = acc != 0.0;
         }
       }
-      // one atomic per (k-block, warp): the first lane with a nonzero value in its group
-      const int64_t kb = valid ? k / BK : -1;
-      const unsigned grp = __match_any_sync(0xffffffffu, kb);
-      const unsigned nzb = __ballot_sync(0xffffffffu, nz);
-      if (nz && lane == __ffs(grp & nzb) - 1) {
-        mark(m, kb);
-        if (CPLX) {
-          mark(m, kb + Kh / BK);
-          mark(Nlog + m, kb);
-          mark(Nlog + m, kb + Kh / BK);
+#pragma unroll
+      for (int u = 0; u < MIXU; ++u) {
+        const bool valid = hit[u] && a + u * 128 < ahi;
+        const int64_t k = a + u * 128 + k0J;
+        bool nz = false;
+        if (valid) {
+          put(m, k, re[u]);
+          nz = (__double_as_longlong(re[u]) << 1) != 0;
+          if (CPLX) {
+            const double mim = __longlong_as_double(__double_as_longlong(im[u]) ^ (1ll << 63));
+            put(m, Kh + k, mim);
+            put(Nlog + m, k, im[u]);
+            put(Nlog + m, Kh + k, re[u]);
+            nz |= (__double_as_longlong(im[u]) << 1) != 0;
+          }
+        }
+        const int64_t kfirst = __shfl_sync(0xffffffffu, k, 0) / BK;
+        const unsigned all = __ballot_sync(0xffffffffu, nz);
+        const unsigned second = __ballot_sync(0xffffffffu, k / BK != kfirst);
+        const uint32_t want = ((all & ~second) ? 1u : 0u) | ((all & second) ? 2u : 0u);
+        const uint32_t fresh = want & ~(marked >> (2 * u));
+        if (fresh) {
+          marked |= fresh << (2 * u);
+          if (lane < 2 && ((fresh >> lane) & 1u)) {
+            const int64_t kb = kfirst + lane;
+            auto mark = [&](int64_t row, int64_t b) {
+              atomicOr(&mask[(row / MASK_ROWS) * kw + b / 32], 1u << (b % 32));
+            };
+            mark(m, kb);
+            if (CPLX) {
+              mark(m, kb + Kh / BK);
+              mark(Nlog + m, kb);
+              mark(Nlog + m, kb + Kh / BK);
+            }
+          }
         }
       }
     }
@@ -407,16 +464,18 @@ void mixpack_run(gb_ctx* ctx, const MixDev& m, const int64_t* kJ, const int64_t*
                                   cudaMemcpyDeviceToDevice, ctx->stream));
   }
   clear_mask(ctx, out);
-  // a block walks N / gridDim.z output columns: long-lived blocks, since with structural
-  // skipping most of a block's work is a map test
   const int64_t span = sk.arange ? std::max<int64_t>(sk.arange_max, 1) : m.A;
-  dim3 grid((unsigned)std::min<int64_t>((span + 127) / 128, 64), (unsigned)m.nJ,
-            (unsigned)std::min<int64_t>(m.N, 32));
+  const int64_t bx = std::min<int64_t>((span + 128 * MIXU - 1) / (128 * MIXU), 64);
+  // runs of columns: long enough to mark the map rarely, short enough to fill the chip
+  const int64_t want = std::max<int64_t>(1, 8 * (int64_t)std::max(1, ctx->num_sms) / (bx * m.nJ));
+  const int64_t nper = std::max<int64_t>(
+      {std::min<int64_t>(16, (m.N + want - 1) / want), (m.N + 65534) / 65535, 1});
+  dim3 grid((unsigned)bx, (unsigned)m.nJ, (unsigned)((m.N + nper - 1) / nper));
   const int64_t plane = out.rows * out.Kp;
 #define GB_MIXPACK(C, E, TX)                                                                  \
   mixpack_kernel<C, E, TX><<<grid, 128, 0, ctx->stream>>>(                                    \
       m.A, m.N, m.xn, m.in_off, kJ, mJ, mn, m.row_ptr, m.col, m.val, (const TX*)x,            \
-      (E*)out.data, Nlog, out.Kp, out.Kh, plane, out.mask, out.kw, sk)
+      (E*)out.data, Nlog, out.Kp, out.Kh, plane, out.mask, out.kw, sk, nper)
 #define GB_MIXPACK_X(C, E)          \
   do {                              \
     if (x_f32) GB_MIXPACK(C, E, float); \
@@ -633,11 +692,12 @@ struct TileMasks {
 
 template <int BN>
 __device__ __forceinline__ TileMasks<BN> tile_masks(const PArgs& p, int mi, int ni, int z) {
+  // a mask row covers 128 rows: a wider tile of B ORs its two, narrower ones share theirs
   TileMasks<BN> t;
   t.a = p.maskA + (p.batchA > 1 ? z : 0) * p.mskA_b + (int64_t)mi * p.kw;
-  int64_t r0 = (int64_t)ni * (BN / MASK_ROWS);
+  int64_t r0 = (int64_t)ni * BN / MASK_ROWS;
   t.b = p.maskB + (p.batchB > 1 ? z : 0) * p.mskB_b + r0 * p.kw;
-  t.nb = (int)std::min<int64_t>(BN / MASK_ROWS, p.mrowsB - r0);
+  t.nb = (int)std::min<int64_t>(BN > MASK_ROWS ? BN / MASK_ROWS : 1, p.mrowsB - r0);
   return t;
 }
 
@@ -870,6 +930,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         return cz + m + args.ldc * n;
       };
       const bool alpha_one = args.alpha == 1.0;
+      const bool plain = alpha_one && args.beta == 0.0;
       auto store = [&](int64_t e, double val) {
         if (args.c_f32) {
           float* p = (float*)args.C + e;
@@ -899,12 +960,42 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         TMEM_LD32(taddr, v);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         if (m >= args.M) continue;
+        // the three forms a GEMM of an operator has, without FP64 arithmetic but the one
+        // addition of an accumulating term: the FP64 pipe issues a warp instruction in 16
+        // clocks, and a conversion and an unused multiply or add per element were most of a
+        // tile's time
+        if (plain && args.c_f32) {
 #pragma unroll
-        for (int jj = 0; jj < 32; ++jj) {
-          const int64_t n = n0 + c0 + jj;
-          if (n >= args.N) break;
-          const double x = (double)__uint_as_float(v[jj]);
-          store(off(n), alpha_one ? x : args.alpha * x);
+          for (int jj = 0; jj < 32; ++jj) {
+            const int64_t n = n0 + c0 + jj;
+            if (n < args.N) ((float*)args.C)[off(n)] = __uint_as_float(v[jj]);
+          }
+        } else if (plain) {
+#pragma unroll
+          for (int jj = 0; jj < 32; ++jj) {
+            const int64_t n = n0 + c0 + jj;
+            if (n < args.N) args.C[off(n)] = to_double(__uint_as_float(v[jj]));
+          }
+        } else if (alpha_one && args.beta == 1.0 && !args.c_f32) {
+          double old[32];  // all loads before the first store: their latencies overlap
+#pragma unroll
+          for (int jj = 0; jj < 32; ++jj) {
+            const int64_t n = n0 + c0 + jj;
+            old[jj] = n < args.N ? args.C[off(n)] : 0.0;
+          }
+#pragma unroll
+          for (int jj = 0; jj < 32; ++jj) {
+            const int64_t n = n0 + c0 + jj;
+            if (n < args.N) args.C[off(n)] = old[jj] + to_double(__uint_as_float(v[jj]));
+          }
+        } else {
+#pragma unroll
+          for (int jj = 0; jj < 32; ++jj) {
+            const int64_t n = n0 + c0 + jj;
+            if (n >= args.N) break;
+            const double x = (double)__uint_as_float(v[jj]);
+            store(off(n), alpha_one ? x : args.alpha * x);
+          }
         }
       }
       tc_fence_before();
@@ -1065,8 +1156,17 @@ void gemm_split(gb_ctx* ctx, int dtype, const Packed& A, const Packed& B, int64_
     GB_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "gemm_split: grid too large");
     gemm_bf16x3_kernel<<<grid, TC_THREADS, TC_SMEM_BYTES, ctx->stream>>>(ma, mb, a);
   } else {
-    const int bn = ctx->gemm_bn ? ctx->gemm_bn : (Npk <= 128 ? 128 : 256);
-    if (bn == 128) mb = make_map(B, 128);
+    // Tile width: 256 columns where that gives every SM a tile; narrower ones read A more
+    // often but put more SMs to work (256 x 1024 x 1024 tf32x3: 8 tiles of 256 columns 88 us,
+    // 32 of 64 columns NN us).  The products of an element are summed in the same order.
+    int bn = ctx->gemm_bn;
+    if (!bn) {
+      const int64_t mt = (M + TC_BM - 1) / TC_BM;
+      auto tiles = [&](int w) { return mt * ((Npk + w - 1) / w) * batch; };
+      bn = Npk <= 64 ? 64 : Npk <= 128 ? 128 : 256;
+      while (bn > 64 && tiles(bn) < std::max(1, ctx->num_sms)) bn /= 2;
+    }
+    if (bn != TC_BN) mb = make_map(B, bn);
     PArgs p;
     p.M = M;
     p.N = Npk;
@@ -1124,7 +1224,10 @@ void gemm_split(gb_ctx* ctx, int dtype, const Packed& A, const Packed& B, int64_
     });                                                                                       \
     gemm_bf16x3_persistent<BN_, ST_, TF_><<<grid, TC_THREADS, SM, ctx->stream>>>(ma, mb, p); \
   } while (0)
-    if (bn == 128) {
+    if (bn == 64) {
+      if (tf32) GB_PERSISTENT(64, 8, true);
+      else GB_PERSISTENT(64, 8, false);
+    } else if (bn == 128) {
       if (tf32) GB_PERSISTENT(128, 6, true);
       else GB_PERSISTENT(128, 6, false);
     } else {

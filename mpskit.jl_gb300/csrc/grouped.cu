@@ -326,7 +326,7 @@ __global__ void gpack_kernel(const GPackTile* __restrict__ tiles, const int32_t*
     const int kp = T.kp0 + kk;
     float v = 0.0f;
     if (i < T.nr && kp < kl && in[kk])
-      v = (float)src[(int64_t)rdense[T.rp0 + i] * rs + ((int64_t)kdense[k0 + kp] - klo) * ks];
+      v = to_float(src[(int64_t)rdense[T.rp0 + i] * rs + ((int64_t)kdense[k0 + kp] - klo) * ks]);
     t[i][kk] = v;
   }
   __syncthreads();
@@ -484,8 +484,8 @@ __global__ void gmix_kernel(int64_t nJ, int64_t N, int64_t xn, const int64_t* __
           const int64_t a = a0 + 32 * u;
           xv[u] = a < en.hi ? xp[a] : 0.0f;
         }
-        const float vh = (float)val[e];
-        const float vl = (float)(val[e] - (double)vh);
+        const float vh = to_float(val[e]);
+        const float vl = std::is_same<E, float>::value ? (float)(val[e] - (double)vh) : 0.0f;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           if (std::is_same<E, float>::value) {
@@ -870,7 +870,21 @@ __global__ void __launch_bounds__(G_THREADS, 1)
 #pragma unroll
             for (int jj = 0; jj < 16; ++jj) {
               co[jj] = __shfl_sync(0xffffffffu, myco, h + jj);
-              val[jj] = (double)__uint_as_float(v[h + jj]);
+              val[jj] = to_double(__uint_as_float(v[h + jj]));
+            }
+            if (alpha_one && beta_one && !f32) {
+              // the accumulating form: one FP64 addition per element and no other
+              if (!rvalid) continue;
+              const double* Cd = (const double*)args.C;
+              double cv[16];
+#pragma unroll
+              for (int jj = 0; jj < 16; ++jj)
+                cv[jj] = ((int64_t)T.n0 + c0 + h + jj < nend) ? Cd[roff + co[jj]] : 0.0;
+#pragma unroll
+              for (int jj = 0; jj < 16; ++jj)
+                if ((int64_t)T.n0 + c0 + h + jj < nend)
+                  ((double*)args.C)[roff + co[jj]] = cv[jj] + val[jj];
+              continue;
             }
             if (!alpha_one) {
 #pragma unroll
@@ -920,7 +934,18 @@ __global__ void __launch_bounds__(G_THREADS, 1)
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
               ro[i] = __shfl_sync(0xffffffffu, roff, h + i);
-              val[i] = (double)xb[(h + i) * 33 + lane];
+              val[i] = to_double(xb[(h + i) * 33 + lane]);
+            }
+            if (alpha_one && beta_one && !f32) {
+              if (!cvalid) continue;
+              const double* Cd = (const double*)args.C;
+              double cv[16];
+#pragma unroll
+              for (int i = 0; i < 16; ++i) cv[i] = (mrow0 + h + i < T.mlim) ? Cd[ro[i] + co] : 0.0;
+#pragma unroll
+              for (int i = 0; i < 16; ++i)
+                if (mrow0 + h + i < T.mlim) ((double*)args.C)[ro[i] + co] = cv[i] + val[i];
+              continue;
             }
             if (!alpha_one) {
 #pragma unroll

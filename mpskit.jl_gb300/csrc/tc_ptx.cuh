@@ -45,6 +45,33 @@ __device__ __forceinline__ bool plane_nz(__nv_bfloat16 a) { return __bfloat162fl
 __device__ __forceinline__ bool plane_nz(float a) { return a != 0.f; }
 inline bool is_tf32(int prec) { return prec == GB_PREC_TF32X3; }
 
+// ------------------------------------------------------------------ FP32 <-> FP64 by the bits
+// Conversions run on the FP64 pipe (one warp instruction per 16 clocks and SM); these give the
+// same results with a handful of integer instructions.
+// (double)x; subnormal and non-finite values take the conversion
+__device__ __forceinline__ double to_double(float x) {
+  const uint32_t u = __float_as_uint(x), mag = u & 0x7fffffffu;
+  if (__builtin_expect(mag - 0x00800000u < 0x7f000000u, 1))
+    return __hiloint2double((int)((u & 0x80000000u) | ((mag >> 3) + 0x38000000u)),
+                            (int)(u << 29));
+  return mag ? (double)x : __hiloint2double((int)u, 0);
+}
+__device__ __forceinline__ double to_double(double x) { return x; }
+// (float)x, to nearest even, without the FP64 pipe; values outside FP32's normal range (and
+// their rounding) take the conversion
+__device__ __forceinline__ float to_float(double x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  const uint32_t mag = hi & 0x7fffffffu;
+  if (__builtin_expect(mag - 0x38100000u < 0x0fd00000u, 1)) {
+    // 20 + 3 bits kept; the rest decides
+    uint32_t r = ((mag - 0x38000000u) << 3) | (lo >> 29);
+    const uint32_t rest = lo & 0x1fffffffu;
+    r += (rest > 0x10000000u || (rest == 0x10000000u && (r & 1u))) ? 1u : 0u;
+    return __uint_as_float((hi & 0x80000000u) | r);
+  }
+  return (mag | lo) ? (float)x : __uint_as_float(hi & 0x80000000u);
+}
+
 // ------------------------------------------------------------------ PTX helpers
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
