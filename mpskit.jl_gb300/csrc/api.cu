@@ -440,6 +440,16 @@ void qr_pos(gb_ctx* ctx, int dtype, int64_t m, int64_t n, const void* M, void* Q
   cudaDataType t = cx ? CUDA_C_64F : CUDA_R_64F;
   const size_t es = elem_size(dtype);
   int64_t k = std::min(m, n);
+  if (m >= n) {
+    if (qr_gram(ctx, dtype, m, n, M, Q, R)) return;
+  } else if (m > 0 && qr_gram(ctx, dtype, m, m, M, Q, R)) {
+    // wide: the factors of the first m columns, and Q' times the others
+    gemm_fp64(ctx, dtype, 'C', 'N', m, n - m, m, cplx{1, 0}, Q, m, 0,
+              (const char*)M + (size_t)m * m * es, m, 0, cplx{0, 0}, (char*)R + (size_t)m * m * es,
+              m, 0, 1);
+    GB_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
+    return;
+  }
   int64_t ncols = std::max(n, k);
   // work matrix: m x n copy of M (plus room for orgqr on the first k columns)
   char* A = (char*)scratch(ctx, SLOT_GAUGE, (size_t)m * ncols * es + 256);

@@ -7,8 +7,8 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(ROOT, "csrc")
 BUILD = os.path.join(ROOT, "_build")
-SOURCES = ["kernels.cu", "gemm_f64.cu", "gemm_tc.cu", "grouped.cu", "heff.cu", "krylov.cu", "orth.cu", "api.cu",
-           "u1.cu", "noalloc.cu", "packed.cu"]
+SOURCES = ["kernels.cu", "gemm_f64.cu", "gemm_tc.cu", "grouped.cu", "heff.cu", "krylov.cu",
+           "orth.cu", "qr.cu", "api.cu", "u1.cu", "noalloc.cu", "packed.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
 

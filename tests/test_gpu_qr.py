@@ -1,0 +1,108 @@
+"""Positive QR and LQ against Householder factors in extended conditions.
+
+Q' Q = 1 and Q R = A hold to a few n eps whatever the condition number (both the Gram route and
+the Householder routine it falls back to); the factors themselves differ from another algorithm's
+by n eps cond(A)."""
+import numpy as np
+import pytest
+
+import mpsgb
+
+pytestmark = pytest.mark.gpu
+EPS = np.finfo(np.float64).eps
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    return mpsgb.Context(0)
+
+
+def _ref(a):
+    q, r = np.linalg.qr(a)
+    ph = np.diagonal(r).copy()
+    ph[ph == 0] = 1
+    ph = ph / np.abs(ph)
+    return q * ph, np.conj(ph)[:, None] * r
+
+
+def _check(a, q, r, cond):
+    m, n = a.shape
+    k = min(m, n)
+    assert np.linalg.norm(q.conj().T @ q - np.eye(k)) <= 8 * n * EPS
+    assert np.linalg.norm(a - q @ r) <= 8 * n * EPS * np.linalg.norm(a)
+    assert np.all(np.tril(r, -1) == 0)
+    d = np.diagonal(r)[:k]
+    assert np.all(d.real >= 0) and np.all(d.imag == 0)
+    if cond is not None:
+        q0, r0 = _ref(a)
+        assert np.linalg.norm(q - q0) <= 8 * n * EPS * cond
+        assert np.linalg.norm(r - r0) <= 8 * n * EPS * cond * np.linalg.norm(r0)
+
+
+def _matrix(rng, m, n, cx, cond):
+    a = rng.standard_normal((m, n)) + (1j * rng.standard_normal((m, n)) if cx else 0)
+    if cond:
+        u, _, v = np.linalg.svd(a, full_matrices=False)
+        a = u * np.logspace(0, -np.log10(cond), min(m, n)) @ v
+        return a, cond
+    s = np.linalg.svd(a, compute_uv=False)
+    return a, s[0] / s[-1]
+
+
+# one column, block rows and their edges, one block row of the update more, wide matrices, block
+# rows longer than a pass of the chip
+SHAPES = [(2, 1), (6, 3), (32, 16), (40, 17), (64, 33), (96, 48), (130, 65), (512, 256),
+          (700, 300), (20, 34), (64, 100), (256, 256), (1100, 1024), (1100, 1025)]
+
+
+@pytest.mark.parametrize("cx", [False, True])
+@pytest.mark.parametrize("m,n", SHAPES)
+def test_left_and_right(ctx, m, n, cx):
+    rng = np.random.default_rng(m * n)
+    if m % 2:
+        m += 1
+    a, cond = _matrix(rng, m, n, cx, None)
+    al, c = mpsgb.left_orth(mpsgb.DeviceTensor.from_numpy(
+        ctx, "mps", a.reshape(m // 2, 2, n, order="F")))
+    _check(a, al.numpy().reshape(m, -1, order="F"), c.numpy(), cond if m >= n else None)
+    # LQ of the adjoint: the same factors
+    b = a.conj().T
+    c2, ar = mpsgb.right_orth(mpsgb.DeviceTensor.from_numpy(
+        ctx, "mps", b.reshape(n, 2, m // 2, order="F")))
+    _check(a, ar.numpy().reshape(-1, m, order="F").conj().T, c2.numpy().conj().T,
+           cond if m >= n else None)
+    assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("cond", [1e3, 1e5, 1e7, 1e10, 1e15])
+@pytest.mark.parametrize("cx", [False, True])
+def test_ill_conditioned(ctx, cx, cond):
+    """From one correction to several and to the Householder fallback."""
+    rng = np.random.default_rng(int(np.log10(cond)))
+    a, c = _matrix(rng, 200, 90, cx, cond)
+    al, r = mpsgb.left_orth(mpsgb.DeviceTensor.from_numpy(
+        ctx, "mps", a.reshape(100, 2, 90, order="F")))
+    _check(a, al.numpy().reshape(200, 90, order="F"), r.numpy(), c if cond <= 1e10 else None)
+
+
+def test_rank_deficient_scaled_and_non_finite(ctx):
+    rng = np.random.default_rng(9)
+    a = rng.standard_normal((80, 30))
+    a[:, 20:] = 0  # an enlarged bond: zero columns appended
+    q, r = (t.numpy() for t in mpsgb.left_orth(mpsgb.DeviceTensor.from_numpy(
+        ctx, "mps", a.reshape(40, 2, 30, order="F"))))
+    _check(a, q.reshape(80, 30, order="F"), r, None)
+    for scale in (1e-150, 1e150):  # squares leave the range of FP64 only beyond this
+        b = scale * rng.standard_normal((80, 30))
+        b[:, ::2] *= 1e-4
+        q, r = (t.numpy() for t in mpsgb.left_orth(mpsgb.DeviceTensor.from_numpy(
+            ctx, "mps", b.reshape(40, 2, 30, order="F"))))
+        _check(b, q.reshape(80, 30, order="F"), r, None)
+    for scale in (1e-200, 1e200):  # the Gram matrix under- or overflows: Householder
+        b = scale * rng.standard_normal((80, 30))
+        q, r = (t.numpy() for t in mpsgb.left_orth(mpsgb.DeviceTensor.from_numpy(
+            ctx, "mps", b.reshape(40, 2, 30, order="F"))))
+        assert np.linalg.norm(q.reshape(80, 30, order="F").T @ q.reshape(80, 30, order="F")
+                              - np.eye(30)) <= 8 * 30 * EPS
+        assert np.all(np.abs(b - q.reshape(80, 30, order="F") @ r) <= 240 * EPS * np.abs(b).max())
+    assert ctx.device_status() == 0
