@@ -322,11 +322,11 @@ struct Packed {
   int esz = 2;               // plane element bytes: 2 (BF16 planes) or 4 (TF32 planes)
   int bk = 64;               // k-block (elements per 128-byte swizzle row): 64 or 32
   // FP64 operands cut into digits (slices > 0): planes [batch][slices][rows][Kp] of BF16
-  // integers, one biased exponent per logical row, one byte per 32-row x 64-k block (mrows
-  // row groups) that holds a nonzero
+  // integers, one biased exponent per logical row, a word per 32-row x 64-k block (mrows
+  // row groups): nonzero if the block is
   int slices = 0;
   int* exps = nullptr;
-  uint8_t* nz = nullptr;
+  uint32_t* nz = nullptr;
 };
 // which operand of C = op(A) op(B) is being packed
 enum PackRole { PACK_AS_A = 0, PACK_AS_B = 1 };

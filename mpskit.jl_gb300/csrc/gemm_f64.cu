@@ -18,7 +18,7 @@
 //    the only rounding besides the slicing is the final one to FP64.
 //
 //    Measured (one product, operands cut included; SIMT tiles / here): complex 256 x 256 x 256
-//    531 / 27 us, complex 512 x 512 x 256 530 / 42 us, real 2048^3 8.6 / 0.58 ms = 30 TFLOP/s.
+//    531 / 21 us, complex 512 x 512 x 256 530 / 39 us, real 2048^3 8.6 / 0.58 ms = 30 TFLOP/s.
 //    Its error against extended precision at K = 128..256 is 5.7e-17 of the result (the FMAs':
 //    3.8e-16).
 //
@@ -60,7 +60,8 @@ struct SliceArgs {
   int* part;           // [batch][nchunk][R] maxima of the biased exponent
   int* exps;           // [batch][R]
   __nv_bfloat16* planes;  // [batch][SL][rows][Kp]
-  uint8_t* nz;         // [batch][groups][Kp / 64]: a 32-row x 64-k block holds a nonzero
+  uint32_t* nz;        // [batch][groups][Kp / 64]: a 32-row x 64-k block holds a nonzero (a
+                       // byte for each 8 rows)
   int64_t groups;
   int rblk;            // row blocks of 32
   int nblk;            // blocks of this operand in the launch
@@ -155,13 +156,189 @@ __device__ __forceinline__ uint32_t digit_pair(uint32_t b0, uint32_t b1) {
   return __byte_perm(__float_as_uint(f0), __float_as_uint(f1), 0x7632);
 }
 
-// digits of a 32-row x 64-k block: the source block goes through shared memory (its
-// contiguous index is R or K), each warp then writes whole 128-byte K lines of the planes.
-// Bound by the writes: 14 bytes per real entry (28 per complex entry of A, 56 of B); below a
-// few million entries by its latency.
+// digits of an RB-row x 64-k block: the source block goes through shared memory (its contiguous
+// index is R or K), each warp then writes whole 128-byte K lines of the planes.
+template <int RB>
+struct SliceSmem {
+  double re[RB][65], im[RB][65];
+  int e[RB];       // largest biased exponents of the rows: this CTA's k-blocks
+  int all[RB];     // of the whole rows
+};
+
+template <int RB>
+__device__ __forceinline__ void slice_load(const SliceArgs& p, SliceSmem<RB>& s, const double* src,
+                                           int64_t r0, int64_t k0, int& nz, bool maxima) {
+  const int tid = threadIdx.x;
+  const long long flip = p.conj ? (long long)(1ull << 63) : 0;
+  int m = 0;
+  double re[RB / 4], im[RB / 4];
+#pragma unroll
+  for (int i = 0; i < RB / 4; ++i) {
+    const int e = tid + 256 * i;
+    const int rr = p.rowfast ? e % RB : e / 64, kk = p.rowfast ? e / RB : e % 64;
+    const int64_t r = r0 + rr, k = k0 + kk;
+    re[i] = im[i] = 0.0;
+    if (r < p.R && k < p.K) {
+      const int64_t ad = p.rowfast ? r + p.ld * k : k + p.ld * r;
+      if (p.cplx) {
+        const double2 v = ((const double2*)src)[ad];
+        re[i] = v.x;
+        im[i] = __longlong_as_double(__double_as_longlong(v.y) ^ flip);
+      } else {
+        re[i] = src[ad];
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < RB / 4; ++i) {
+    const int e = tid + 256 * i;
+    const int rr = p.rowfast ? e % RB : e / 64, kk = p.rowfast ? e / RB : e % 64;
+    // zero tests and sign flips on the bits: comparisons run on the FP64 pipe
+    nz |= ((__double_as_longlong(re[i]) | __double_as_longlong(im[i])) << 1) != 0;
+    s.re[rr][kk] = re[i];
+    if (p.cplx) s.im[rr][kk] = im[i];
+    if (maxima) {
+      const int x = max(biased_exp(re[i]), biased_exp(im[i]));
+      if (p.rowfast) {
+        m = max(m, x);
+      } else {
+        const int w = __reduce_max_sync(0xffffffffu, x);
+        if (tid % 32 == 0) atomicMax(&s.e[rr], w);
+      }
+    }
+  }
+  if (maxima && p.rowfast) atomicMax(&s.e[tid % RB], m);
+}
+
+template <int RB>
+__device__ __forceinline__ void slice_store(const SliceArgs& p, const SliceSmem<RB>& s, int z,
+                                            int64_t r0, int64_t k0) {
+  const int lane = threadIdx.x % 32, w = threadIdx.x / 32;
+  const int64_t plane = p.rows * p.Kp;
+  __nv_bfloat16* base = p.planes + (int64_t)z * SL * plane;
+  auto put = [&](int64_t row, int64_t k, unsigned long long y0, unsigned long long y1) {
+    uint32_t* d = (uint32_t*)(base + row * p.Kp + k) + lane;
+#pragma unroll
+    for (int i = 0; i < SL; ++i) {
+      const int sh = 8 * (SL - 1 - i);
+      const uint32_t mask = i == 0 ? 0x1ffu : 0xffu;  // the top digit may be +128
+      *d = digit_pair((uint32_t)(y0 >> sh) & mask, (uint32_t)(y1 >> sh) & mask);
+      d += plane / 2;
+    }
+  };
+  const unsigned long long two_bias = 2ull * 0x80808080808080ull;
+#pragma unroll 1
+  for (int rr = w; rr < RB; rr += 8) {
+    const int64_t r = r0 + rr;
+    if (r >= (p.isB && p.cplx ? p.imrow : p.R)) break;  // complex B: pad rows are written too
+    const int E = max(s.all[rr], 1);
+    const unsigned long long y0 = slice_bits(s.re[rr][2 * lane], E),
+                             y1 = slice_bits(s.re[rr][2 * lane + 1], E);
+    put(r, k0, y0, y1);
+    if (p.cplx) {
+      const unsigned long long w0 = slice_bits(s.im[rr][2 * lane], E),
+                               w1 = slice_bits(s.im[rr][2 * lane + 1], E);
+      if (!p.isB) {
+        put(r, p.Kh + k0, w0, w1);
+      } else {
+        // bytes of bias - m are those of 2 bias - (bias + m)
+        put(r, p.Kh + k0, two_bias - w0, two_bias - w1);
+        put(p.imrow + r, k0, w0, w1);
+        put(p.imrow + r, p.Kh + k0, y0, y1);
+      }
+    }
+  }
+}
+
+// flag of the RB-row x 64-k block at rows r0 (an 8-row piece writes its byte)
+template <int RB>
+__device__ __forceinline__ void slice_flags(const SliceArgs& p, int z, int64_t r0, int kb, int nz) {
+  const int64_t kbs = p.Kh / 64, kbp = p.Kp / 64;
+  uint32_t* nzb = p.nz + (int64_t)z * p.groups * kbp;
+  auto put = [&](int64_t i) {
+    if (RB == 32) nzb[i] = nz ? 1u : 0u;
+    else ((uint8_t*)(nzb + i))[r0 % 32 / 8] = nz ? 1 : 0;
+  };
+  const int64_t rb = r0 / 32;
+  put(rb * kbp + kb);
+  if (p.cplx) {
+    put(rb * kbp + kbs + kb);
+    if (p.isB) {
+      const int64_t ri = p.imrow / 32 + rb;
+      put(ri * kbp + kb);
+      put(ri * kbp + kbs + kb);
+    }
+  }
+}
+
+// Row maxima and digits in one launch: the CTAs of a cluster share a block of rows, each takes
+// every cs-th 64-k block, and the maxima meet in distributed shared memory.  A row's first pass
+// leaves the CTA's last k-block in shared memory; the others are read again (from L2).  Bound by
+// the writes: 14 bytes per real entry (28 per complex entry of A, 56 of B); below a few million
+// entries by its latency, which is why operands of few blocks are cut into 8-row pieces and why it
+// is one launch: complex 256 x 256, 16.5 us as
+// a launch for the maxima and one for the digits, 8.8 us here.
+template <int RB>
+__global__ void __launch_bounds__(256) slice_cluster_kernel(SliceArgs a, SliceArgs b, int cs) {
+  __shared__ SliceSmem<RB> s;
+  const int rank = (int)blockIdx.x % cs;  // clusters are runs of cs CTAs
+  int blk = (int)blockIdx.x / cs;
+  const bool second = blk >= a.nblk;
+  const SliceArgs& p = second ? b : a;
+  if (second) blk -= a.nblk;
+  const int kbs = (int)(p.Kh / 64);
+  const int per = p.rblk * (32 / RB), rb = blk % per, z = blk / per;
+  const int64_t r0 = (int64_t)rb * RB;
+  const double* src = p.src + (int64_t)z * p.stride * (p.cplx ? 2 : 1);
+  const int tid = threadIdx.x;
+  if (tid < RB) s.e[tid] = 0;
+  const int mine = rank < kbs ? (kbs - rank + cs - 1) / cs : 0;
+  int nz = 0;
+  for (int i = 0; i < mine; ++i) {
+    __syncthreads();
+    nz = 0;
+    slice_load<RB>(p, s, src, r0, (int64_t)(rank + i * cs) * 64, nz, true);
+  }
+  __syncwarp();
+  if (cs > 1) {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  } else {
+    __syncthreads();
+  }
+  if (tid < RB) {
+    int m = 0;
+    for (int c = 0; c < cs; ++c) {
+      uint32_t at;
+      int v;
+      asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_u32(&s.e[tid])), "r"(c));
+      asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+      m = max(m, v);
+    }
+    s.all[tid] = m;
+    if (rank == 0 && r0 + tid < p.R) p.exps[(int64_t)z * p.R + r0 + tid] = m;
+  }
+  // no CTA leaves while another reads its maxima
+  __syncwarp();
+  if (cs > 1) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+  for (int i = mine - 1; i >= 0; --i) {
+    const int kb = rank + i * cs;
+    if (i < mine - 1) {
+      __syncthreads();
+      nz = 0;
+      slice_load<RB>(p, s, src, r0, (int64_t)kb * 64, nz, false);
+    }
+    nz = __syncthreads_or(nz);
+    if (tid == 0) slice_flags<RB>(p, z, r0, kb, nz);
+    slice_store<RB>(p, s, z, r0, (int64_t)kb * 64);
+  }
+  if (cs > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+}
+
+// The digits alone, the row maxima being in p.part (few rows and a long contraction: a CTA per
+// 64-k block)
 __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a, SliceArgs b) {
-  __shared__ double sre[32][65], sim[32][65];
-  __shared__ int se[32];
+  __shared__ SliceSmem<32> s;
   const bool second = (int)blockIdx.x >= a.nblk;
   const SliceArgs& p = second ? b : a;
   int blk = second ? (int)blockIdx.x - a.nblk : (int)blockIdx.x;
@@ -179,80 +356,13 @@ __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a, SliceArgs b) {
         m = max(m, p.part[((int64_t)z * p.nchunk + c) * p.R + r0 + tid]);
       if (kb == 0) p.exps[(int64_t)z * p.R + r0 + tid] = m;
     }
-    se[tid] = m;
+    s.all[tid] = m;
   }
   int nz = 0;
-  const long long flip = p.conj ? (long long)(1ull << 63) : 0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int e = tid + 256 * i;
-    const int rr = p.rowfast ? e % 32 : e / 64, kk = p.rowfast ? e / 32 : e % 64;
-    const int64_t r = r0 + rr, k = k0 + kk;
-    double re = 0.0, im = 0.0;
-    if (r < p.R && k < p.K) {
-      const int64_t ad = p.rowfast ? r + p.ld * k : k + p.ld * r;
-      if (p.cplx) {
-        const double2 v = ((const double2*)src)[ad];
-        re = v.x;
-        im = __longlong_as_double(__double_as_longlong(v.y) ^ flip);
-      } else {
-        re = src[ad];
-      }
-    }
-    // zero tests and sign flips on the bits: comparisons run on the FP64 pipe
-    nz |= ((__double_as_longlong(re) | __double_as_longlong(im)) << 1) != 0;
-    sre[rr][kk] = re;
-    if (p.cplx) sim[rr][kk] = im;
-  }
+  slice_load<32>(p, s, src, r0, k0, nz, false);
   nz = __syncthreads_or(nz);
-  const int64_t kbp = p.Kp / 64;
-  if (tid == 0) {
-    uint8_t* nzb = p.nz + (int64_t)z * p.groups * kbp;
-    nzb[rb * kbp + kb] = nz ? 1 : 0;
-    if (p.cplx) {
-      nzb[rb * kbp + kbs + kb] = nz ? 1 : 0;
-      if (p.isB) {
-        const int64_t ri = p.imrow / 32 + rb;
-        nzb[ri * kbp + kb] = nz ? 1 : 0;
-        nzb[ri * kbp + kbs + kb] = nz ? 1 : 0;
-      }
-    }
-  }
-  const int lane = tid % 32, w = tid / 32;
-  const int64_t plane = p.rows * p.Kp;
-  __nv_bfloat16* base = p.planes + (int64_t)z * SL * plane;
-  auto put = [&](int64_t row, int64_t k, unsigned long long y0, unsigned long long y1) {
-    uint32_t* d = (uint32_t*)(base + row * p.Kp + k) + lane;
-#pragma unroll
-    for (int s = 0; s < SL; ++s) {
-      const int sh = 8 * (SL - 1 - s);
-      const uint32_t mask = s == 0 ? 0x1ffu : 0xffu;  // the top digit may be +128
-      *d = digit_pair((uint32_t)(y0 >> sh) & mask, (uint32_t)(y1 >> sh) & mask);
-      d += plane / 2;
-    }
-  };
-  const unsigned long long two_bias = 2ull * 0x80808080808080ull;
-#pragma unroll 1
-  for (int rr = w; rr < 32; rr += 8) {
-    const int64_t r = r0 + rr;
-    if (r >= (p.isB && p.cplx ? p.imrow : p.R)) break;  // complex B: pad rows are written too
-    const int E = max(se[rr], 1);
-    const unsigned long long y0 = slice_bits(sre[rr][2 * lane], E),
-                             y1 = slice_bits(sre[rr][2 * lane + 1], E);
-    put(r, k0, y0, y1);
-    if (p.cplx) {
-      const unsigned long long w0 = slice_bits(sim[rr][2 * lane], E),
-                               w1 = slice_bits(sim[rr][2 * lane + 1], E);
-      if (!p.isB) {
-        put(r, p.Kh + k0, w0, w1);
-      } else {
-        // bytes of bias - m are those of 2 bias - (bias + m)
-        put(r, p.Kh + k0, two_bias - w0, two_bias - w1);
-        put(p.imrow + r, k0, w0, w1);
-        put(p.imrow + r, p.Kh + k0, y0, y1);
-      }
-    }
-  }
+  if (tid == 0) slice_flags<32>(p, z, r0, kb, nz);
+  slice_store<32>(p, s, z, r0, k0);
 }
 
 // ------------------------------------------------------------------ the GEMM
@@ -268,7 +378,7 @@ struct SGArgs {
   int64_t rowsB;     // packed rows of B
   int nkb;           // Kp / 64
   int batchA, batchB;
-  const uint8_t *nzA, *nzB;
+  const uint32_t *nzA, *nzB;
   int64_t grpA, grpB;
   const int *eA, *eB;
   double alpha, beta;
@@ -445,8 +555,8 @@ __global__ void __launch_bounds__(SG_THREADS, 1)
   }
   if (warp == 2) {
     // the k-blocks in which both operands hold a nonzero, in order
-    const uint8_t* za = g.nzA + ((int64_t)zA * g.grpA + m0 / 32) * g.nkb;
-    const uint8_t* zb = g.nzB + ((int64_t)zB * g.grpB + n0 / 32) * g.nkb;
+    const uint32_t* za = g.nzA + ((int64_t)zA * g.grpA + m0 / 32) * g.nkb;
+    const uint32_t* zb = g.nzB + ((int64_t)zB * g.grpB + n0 / 32) * g.nkb;
     const int ga = (int)min((int64_t)4, g.grpA - m0 / 32);
     const int gb_ = (int)min((int64_t)(BN / 32), g.grpB - n0 / 32);
     int cnt = 0;
@@ -802,7 +912,7 @@ size_t sliced_bytes(int64_t R, int64_t K, bool cx, int role, int64_t batch) {
   const bool dbl = cx && role == PACK_AS_B;
   const int64_t rows = dbl ? 2 * rup(R, 32) : R;
   const int64_t groups = (rows + 31) / 32;
-  return (size_t)rup(batch * SL * rows * Kp * 2, 256) + (size_t)rup(batch * groups * (Kp / 64), 256) +
+  return (size_t)rup(batch * SL * rows * Kp * 2, 256) + (size_t)rup(batch * groups * (Kp / 64) * 4, 256) +
          (size_t)rup(batch * R * 4, 256) + (size_t)rup(batch * 16 * R * 4, 256);
 }
 
@@ -834,8 +944,8 @@ static SliceArgs slice_args(gb_ctx* ctx, int dtype, int role, char op, int64_t R
   char* d = (char*)dst;
   a.planes = (__nv_bfloat16*)d;
   d += rup(batch * SL * a.rows * a.Kp * 2, 256);
-  a.nz = (uint8_t*)d;
-  d += rup(batch * a.groups * (a.Kp / 64), 256);
+  a.nz = (uint32_t*)d;
+  d += rup(batch * a.groups * (a.Kp / 64) * 4, 256);
   a.exps = (int*)d;
   d += rup(batch * R * 4, 256);
   a.part = (int*)d;
@@ -859,13 +969,44 @@ static void slice_launch(gb_ctx* ctx, SliceArgs a, SliceArgs b) {
     const int64_t n = s.src ? (int64_t)s.rblk * s.batch * per : 0;
     GB_REQUIRE(n < (int64_t)1 << 30, "gemm: operand too large to slice");
     s.nblk = (int)n;
+    return n;
   };
+  // both operands have the same contraction
+  const int64_t kbs = a.Kh / 64, sms = std::max(1, ctx->num_sms);
+  const int64_t rows = blocks(a, 1) + blocks(b, 1);
+  // One launch unless a cluster's CTAs would each walk many k-blocks while SMs stand idle (real
+  // 128 x 2000: 12.7 us in one launch, 14.5 in two; 128 x 4000: 19 both; 128 x 8000: 30 and 23;
+  // 64 k-blocks a CTA and more: 1.4 times the two launches).  Blocks of 8 rows where those of 32
+  // would leave SMs idle (complex 256 x 512: 10.5 us against 12.6); beyond that they only cost
+  // reads (real 1024 x 512: 16.5 against 12.5).
+  const int cs = (int)std::min<int64_t>(8, kbs);
+  if (kbs <= 32 || rows * cs >= sms) {
+    const bool small = rows * cs <= sms;
+    if (small) {
+      blocks(a, 4);
+      blocks(b, 4);
+    }
+    GB_REQUIRE((int64_t)(a.nblk + b.nblk) * cs < (int64_t)1 << 31, "gemm: operand too large to slice");
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(a.nblk + b.nblk) * cs);
+    cfg.blockDim = dim3(256);
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {(unsigned)cs, 1, 1};
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (small) GB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, slice_cluster_kernel<8>, a, b, cs));
+    else GB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, slice_cluster_kernel<32>, a, b, cs));
+    count_launch(ctx);
+    return;
+  }
   blocks(a, a.nchunk);
   blocks(b, b.nchunk);
   slice_max_kernel<<<a.nblk + b.nblk, 256, 0, ctx->stream>>>(a, b);
   GB_CHECK_CUDA(cudaGetLastError());
-  blocks(a, a.Kh / 64);
-  blocks(b, b.Kh / 64);
+  blocks(a, kbs);
+  blocks(b, kbs);
   slice_kernel<<<a.nblk + b.nblk, 256, 0, ctx->stream>>>(a, b);
   GB_CHECK_CUDA(cudaGetLastError());
   count_launch_n(ctx, 2);
