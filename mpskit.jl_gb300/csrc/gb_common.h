@@ -30,6 +30,26 @@ void set_last_error(const std::string& msg);
       throw ::gb::Error(GB_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(_e)); \
   } while (0)
 
+// launch of a kernel that starts with chain_wait (tc_ptx.cuh): it may begin before the kernel
+// ahead of it in the stream has ended
+template <typename... P, typename... A>
+inline void launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem,
+                           cudaStream_t st, int cluster_x, int cluster_y, A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim = {(unsigned)cluster_x, (unsigned)cluster_y, 1};
+  cfg.attrs = at;
+  cfg.numAttrs = cluster_x * cluster_y > 1 ? 2 : 1;
+  GB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...));
+}
+
 #define GB_REQUIRE(cond, msg)                                  \
   do {                                                         \
     if (!(cond)) throw ::gb::Error(GB_ERR_ARG, std::string(msg)); \

@@ -75,6 +75,8 @@ __device__ __forceinline__ int biased_exp(double v) {
 // Bound by reading the operand once; a row of blocks per chunk keeps the chip busy when R is
 // small.  Latency-sized operands dominate, so both operands share one launch.
 __global__ void __launch_bounds__(256) slice_max_kernel(SliceArgs a, SliceArgs b) {
+  chain_release();
+  chain_wait();
   const bool second = (int)blockIdx.x >= a.nblk;
   const SliceArgs& p = second ? b : a;
   int blk = second ? (int)blockIdx.x - a.nblk : (int)blockIdx.x;
@@ -292,6 +294,8 @@ __global__ void __launch_bounds__(256) slice_cluster_kernel(SliceArgs a, SliceAr
   const double* src = p.src + (int64_t)z * p.stride * (p.cplx ? 2 : 1);
   const int tid = threadIdx.x;
   if (tid < RB) s.e[tid] = 0;
+  chain_release();
+  chain_wait();
   const int mine = rank < kbs ? (kbs - rank + cs - 1) / cs : 0;
   int nz = 0;
   for (int i = 0; i < mine; ++i) {
@@ -349,6 +353,8 @@ __global__ void __launch_bounds__(256) slice_kernel(SliceArgs a, SliceArgs b) {
   const int64_t r0 = (int64_t)rb * 32, k0 = (int64_t)kb * 64;
   const double* src = p.src + (int64_t)z * p.stride * (p.cplx ? 2 : 1);
   const int tid = threadIdx.x;
+  chain_release();
+  chain_wait();
   if (tid < 32) {
     int m = 0;
     if (r0 + tid < p.R) {
@@ -541,6 +547,8 @@ __global__ void __launch_bounds__(SG_THREADS, 1)
                  "r"(512));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
+  chain_release();
+  chain_wait();
   if (warp == 3) {
     for (int i = lane; i < 128; i += 32)
       sea[i] = m0 + i < g.M ? g.eA[(int64_t)zA * g.M + m0 + i] : 0;
@@ -842,9 +850,9 @@ struct SmallOps<double2> {
 
 template <typename T, int TM, int TN>
 __global__ void __launch_bounds__(128)
-    gemm_small_kernel(int opA, int opB, int64_t M, int64_t N, int64_t K, T alpha,
-                      const T* __restrict__ A, int64_t lda, int64_t sA, const T* __restrict__ B,
-                      int64_t ldb, int64_t sB, T beta, int use_beta, T* __restrict__ C,
+    gemm_small_kernel(int opA, int opB, int64_t M, int64_t N, int64_t K, T alpha, const T* A,
+                      int64_t lda, int64_t sA, const T* B, int64_t ldb, int64_t sB, T beta,
+                      int use_beta, T* C,
                       int64_t ldc, int64_t sC, int64_t kchunk) {
   using O = SmallOps<T>;
   constexpr int KG = 128 / (TM * TN);  // K groups
@@ -864,6 +872,8 @@ __global__ void __launch_bounds__(128)
   const int tm = o % TM, tn = o / TM;
   const bool live = m0 + tm < M && n0 + tn < N;
   T acc = O::zero();
+  chain_release();
+  chain_wait();
   for (int64_t kb = k0; kb < k1; kb += KB) {
     for (int e = tid; e < TM * KB; e += 128) {
       const int r = opA ? e / KB : e % TM, c = opA ? e % KB : e / TM;
@@ -987,28 +997,17 @@ static void slice_launch(gb_ctx* ctx, SliceArgs a, SliceArgs b) {
       blocks(b, 4);
     }
     GB_REQUIRE((int64_t)(a.nblk + b.nblk) * cs < (int64_t)1 << 31, "gemm: operand too large to slice");
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(a.nblk + b.nblk) * cs);
-    cfg.blockDim = dim3(256);
-    cfg.stream = ctx->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim = {(unsigned)cs, 1, 1};
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    if (small) GB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, slice_cluster_kernel<8>, a, b, cs));
-    else GB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, slice_cluster_kernel<32>, a, b, cs));
+    launch_chained(small ? slice_cluster_kernel<8> : slice_cluster_kernel<32>,
+                   dim3((unsigned)(a.nblk + b.nblk) * cs), 256, 0, ctx->stream, cs, 1, a, b, cs);
     count_launch(ctx);
     return;
   }
   blocks(a, a.nchunk);
   blocks(b, b.nchunk);
-  slice_max_kernel<<<a.nblk + b.nblk, 256, 0, ctx->stream>>>(a, b);
-  GB_CHECK_CUDA(cudaGetLastError());
+  launch_chained(slice_max_kernel, dim3(a.nblk + b.nblk), 256, 0, ctx->stream, 1, 1, a, b);
   blocks(a, kbs);
   blocks(b, kbs);
-  slice_kernel<<<a.nblk + b.nblk, 256, 0, ctx->stream>>>(a, b);
-  GB_CHECK_CUDA(cudaGetLastError());
+  launch_chained(slice_kernel, dim3(a.nblk + b.nblk), 256, 0, ctx->stream, 1, 1, a, b);
   count_launch_n(ctx, 2);
 }
 
@@ -1042,17 +1041,8 @@ static void launch_sliced(gb_ctx* ctx, const Packed& a, const Packed& b, SGArgs&
   const CUtensorMap mb = make_slice_map(b.data, b.Kp, b.rows, b.batch * SL, BN, SL);
   const int64_t tiles = (int64_t)g.mt * g.nt * batch;
   GB_REQUIRE(tiles < (int64_t)1 << 31, "gemm: too many tiles");
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)tiles, (unsigned)g.splits);
-  cfg.blockDim = dim3(SG_THREADS);
-  cfg.dynamicSmemBytes = S::SMEM;
-  cfg.stream = ctx->stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim = {1, (unsigned)g.splits, 1};
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  GB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemm_sliced_kernel<BN>, ma, mb, g));
+  launch_chained(gemm_sliced_kernel<BN>, dim3((unsigned)tiles, (unsigned)g.splits), SG_THREADS,
+                 S::SMEM, ctx->stream, 1, g.splits, ma, mb, g);
   count_launch(ctx);
 }
 
@@ -1170,14 +1160,9 @@ static void small_launch(cudaStream_t st, int tile, dim3 grid, int opA, int opB,
                          int64_t N, int64_t K, T alpha, const void* A, int64_t lda, int64_t sA,
                          const void* B, int64_t ldb, int64_t sB, T beta, int use_beta, void* C,
                          int64_t ldc, int64_t sC, int64_t kchunk) {
-  if (tile == 0)
-    gemm_small_kernel<T, 4, 8><<<grid, 128, 0, st>>>(opA, opB, M, N, K, alpha, (const T*)A, lda,
-                                                     sA, (const T*)B, ldb, sB, beta, use_beta,
-                                                     (T*)C, ldc, sC, kchunk);
-  else
-    gemm_small_kernel<T, 16, 8><<<grid, 128, 0, st>>>(opA, opB, M, N, K, alpha, (const T*)A, lda,
-                                                      sA, (const T*)B, ldb, sB, beta, use_beta,
-                                                      (T*)C, ldc, sC, kchunk);
+  launch_chained(tile == 0 ? gemm_small_kernel<T, 4, 8> : gemm_small_kernel<T, 16, 8>, grid, 128, 0,
+                 st, 1, 1, opA, opB, M, N, K, alpha, (const T*)A, lda, sA, (const T*)B, ldb, sB,
+                 beta, use_beta, (T*)C, ldc, sC, kchunk);
 }
 
 SmallPlan gemm_small_plan(int sms, int64_t M, int64_t N, int64_t K, int64_t batch) {

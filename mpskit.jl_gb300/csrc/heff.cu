@@ -24,6 +24,7 @@
 #include <sstream>
 
 #include "gb_common.h"
+#include "tc_ptx.cuh"
 #include "grouped.h"
 
 using gb::cplx;
@@ -1310,7 +1311,9 @@ void heff_apply_raw(gb_heff* h, const void* x, void* y);
 
 template <typename T>
 __global__ void runs_copy_kernel(const int64_t* __restrict__ runs, int64_t nruns,
-                                 const T* __restrict__ src, T* __restrict__ dst, int scatter) {
+                                 const T* src, T* dst, int scatter) {
+  chain_release();
+  chain_wait();
   for (int64_t c = blockIdx.x; c < nruns; c += gridDim.x) {
     const int64_t co = runs[3 * c], dof = runs[3 * c + 1], len = runs[3 * c + 2];
     for (int64_t i = threadIdx.x; i < len; i += blockDim.x) {
@@ -1326,14 +1329,13 @@ static void runs_copy(gb_heff* h, const void* src, void* dst, int scatter) {
   const unsigned grid = (unsigned)std::min<int64_t>(h->nruns, 152 * 8);
   if (grid == 0) return;
   if (is_cplx(h->dtype))
-    runs_copy_kernel<double2><<<grid, 256, 0, ctx->stream>>>(h->runs, h->nruns,
-                                                             (const double2*)src, (double2*)dst,
-                                                             scatter);
+    launch_chained(runs_copy_kernel<double2>, dim3(grid), 256, 0, ctx->stream, 1, 1,
+                   (const int64_t*)h->runs, (int64_t)h->nruns, (const double2*)src, (double2*)dst,
+                   scatter);
   else
-    runs_copy_kernel<double><<<grid, 256, 0, ctx->stream>>>(h->runs, h->nruns,
-                                                            (const double*)src, (double*)dst,
-                                                            scatter);
-  GB_CHECK_CUDA(cudaGetLastError());
+    launch_chained(runs_copy_kernel<double>, dim3(grid), 256, 0, ctx->stream, 1, 1,
+                   (const int64_t*)h->runs, (int64_t)h->nruns, (const double*)src, (double*)dst,
+                   scatter);
   count_launch(ctx);
 }
 

@@ -8,6 +8,7 @@
 #include <cmath>
 
 #include "gb_common.h"
+#include "tc_ptx.cuh"
 
 namespace gb {
 
@@ -110,8 +111,9 @@ template <typename T>
 __global__ void mix_kernel(int64_t A, int64_t N, int64_t xa, int64_t xn, int64_t ya, int64_t yn,
                            const int64_t* __restrict__ in_off, const int64_t* __restrict__ out_off,
                            const int* __restrict__ row_ptr, const int* __restrict__ col,
-                           const T* __restrict__ val, const T* __restrict__ x, T* __restrict__ y,
-                           double beta) {
+                           const T* __restrict__ val, const T* x, T* y, double beta) {
+  chain_release();
+  chain_wait();
   const int J = blockIdx.y;
   const int e0 = row_ptr[J], e1 = row_ptr[J + 1];
   const int64_t yo = out_off[J];
@@ -196,14 +198,14 @@ void mix_run(gb_ctx* ctx, const MixDev& m, int dtype, const void* x, void* y, do
   dim3 grid(nblocks(m.A, 128, 64), (unsigned)m.nJ, (unsigned)std::min<int64_t>(m.N, 65535));
   if (is_cplx(dtype)) {
     GB_REQUIRE(m.cplx, "mix: complex data needs complex coefficients");
-    mix_kernel<dcx><<<grid, 128, 0, ctx->stream>>>(m.A, m.N, m.xa, m.xn, m.ya, m.yn, m.in_off,
-                                                   m.out_off, m.row_ptr, m.col, (const dcx*)m.val,
-                                                   (const dcx*)x, (dcx*)y, beta);
+    launch_chained(mix_kernel<dcx>, grid, 128, 0, ctx->stream, 1, 1, m.A, m.N, m.xa, m.xn, m.ya,
+                   m.yn, m.in_off, m.out_off, m.row_ptr, m.col, (const dcx*)m.val, (const dcx*)x,
+                   (dcx*)y, beta);
   } else {
     GB_REQUIRE(!m.cplx, "mix: real data needs real coefficients");
-    mix_kernel<double><<<grid, 128, 0, ctx->stream>>>(m.A, m.N, m.xa, m.xn, m.ya, m.yn, m.in_off,
-                                                      m.out_off, m.row_ptr, m.col, m.val,
-                                                      (const double*)x, (double*)y, beta);
+    launch_chained(mix_kernel<double>, grid, 128, 0, ctx->stream, 1, 1, m.A, m.N, m.xa, m.xn, m.ya,
+                   m.yn, m.in_off, m.out_off, m.row_ptr, m.col, m.val, (const double*)x,
+                   (double*)y, beta);
   }
   LAUNCH_CHECK();
   count_launch(ctx);
@@ -384,9 +386,11 @@ __global__ void __launch_bounds__(256)
 
 // C = beta C + sum_z W[z] over the split-K slices, summed in slice order (deterministic)
 template <typename T>
-__global__ void splitk_reduce_kernel(int64_t M, int64_t N, int nsplit, const T* __restrict__ W,
-                                     T beta, bool use_beta, T* __restrict__ C, int64_t ldc) {
+__global__ void splitk_reduce_kernel(int64_t M, int64_t N, int nsplit, const T* W, T beta,
+                                     bool use_beta, T* C, int64_t ldc) {
   const int64_t MN = M * N;
+  chain_release();
+  chain_wait();
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < MN;
        e += (int64_t)gridDim.x * blockDim.x) {
     T v = W[e];
@@ -433,11 +437,12 @@ void gemm_fp64(gb_ctx* ctx, int dtype, char opA, char opB, int64_t M, int64_t N,
                    cplx{0, 0}, false, W, M, M * N, ns, kchunk);
         const unsigned rb = (unsigned)std::min<int64_t>((M * N + 255) / 256, 4096);
         if (is_cplx(dtype))
-          splitk_reduce_kernel<dcx><<<rb, 256, 0, ctx->stream>>>(
-              M, N, ns, (const dcx*)W, mk(beta.re, beta.im), use_beta, (dcx*)C, ldc);
+          launch_chained(splitk_reduce_kernel<dcx>, dim3(rb), 256, 0, ctx->stream, 1, 1, M, N, ns,
+                         (const dcx*)W, mk(beta.re, beta.im), use_beta, (dcx*)C, ldc);
         else
-          splitk_reduce_kernel<double><<<rb, 256, 0, ctx->stream>>>(
-              M, N, ns, (const double*)W, beta.re, use_beta, (double*)C, ldc);
+          launch_chained(splitk_reduce_kernel<double>, dim3(rb), 256, 0, ctx->stream, 1, 1, M, N,
+                         ns,
+                         (const double*)W, beta.re, use_beta, (double*)C, ldc);
         count_launch(ctx);
       } else {
         gemm_small(ctx->stream, p, dtype, opA, opB, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta,

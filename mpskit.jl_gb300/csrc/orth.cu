@@ -258,6 +258,7 @@ __global__ void __launch_bounds__(OT, 1) krylov_orth_kernel(OrthArgs g) {
   T* w = g.in_smem ? (T*)piece : wg;
   unsigned int target = 0;
   const int tid = threadIdx.x;
+  chain_release();
   for (int j = tid; j < g.k; j += OT) sh[j] = make_double2(0.0, 0.0);
   if (g.predict) {
     // what the recurrence predicts: the last projection and the last norm
@@ -379,6 +380,7 @@ __global__ void __launch_bounds__(OT) krylov_combine_kernel(CombineArgs a) {
   const int len = (int)(min(g.n, c0 + per) - c0);
   T* dst = (T*)g.vnext + c0;
   const T* src = g.k ? dst : (const T*)g.w + c0;
+  chain_release();
   for (int i = threadIdx.x; g.k && i < len; i += OT) {
     T s = Num<CPLX>::zero();
     const T* v = (const T*)g.V + c0 + i;

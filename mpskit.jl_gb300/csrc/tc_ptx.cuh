@@ -73,6 +73,18 @@ __device__ __forceinline__ float to_float(double x) {
 }
 
 // ------------------------------------------------------------------ PTX helpers
+// Programmatic dependent launch: kernels of a chain start while the one before them drains
+// (launch_chained), set themselves up and wait here for its memory before they touch any of it.
+// Every thread waits, so a kernel's end implies its predecessors' ends.  Data that the kernel
+// before may have written is read through plain pointers: a load through a const __restrict__
+// one may be moved above the wait.  Measured: an apply of two 128 x 256 x 256 complex products
+// (four launches) 41.5 us in plain launches, 34.0 us chained; a D = 32 time step of 3900 launches
+// 40.2 and 32.5 ms.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// the next kernel of the chain may start (once every CTA of this one has started)
+__device__ __forceinline__ void chain_release() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }

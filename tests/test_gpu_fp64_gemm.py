@@ -156,3 +156,22 @@ def test_non_finite_entries(ctx, cx):
     assert not np.isfinite(out[bad]).any()
     assert np.isnan(out[140]).all() and np.isnan(out[:, 77]).all()
     assert np.linalg.norm((out - clean)[~bad]) <= 1e-14 * np.linalg.norm(clean[~bad])
+
+
+@pytest.mark.parametrize("h,K", [(12, 24), (75, 150), (128, 256)])
+def test_chained_launches(ctx, h, K):
+    """Products that feed one another, queued without a wait: the same bits as one at a time."""
+    rng = np.random.default_rng(11)
+    C = [mpsgb.DeviceTensor.from_numpy(
+        ctx, "bond", np.linalg.qr(_rand(rng, (K, K), True, 0))[0]) for _ in range(3)]
+    a0 = mpsgb.DeviceTensor.from_numpy(ctx, "mps", _rand(rng, (h, 2, K), True, 0))
+
+    def run(wait):
+        a = a0
+        for i in range(40):
+            a = mpsgb.states.mul_tail(a, C[i % 3])
+            if wait:
+                ctx.synchronize()
+        return a.numpy()
+
+    assert np.array_equal(run(True), run(False))
