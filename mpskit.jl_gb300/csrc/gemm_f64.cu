@@ -996,7 +996,8 @@ static void slice_launch(gb_ctx* ctx, SliceArgs a, SliceArgs b) {
       blocks(a, 4);
       blocks(b, 4);
     }
-    GB_REQUIRE((int64_t)(a.nblk + b.nblk) * cs < (int64_t)1 << 31, "gemm: operand too large to slice");
+    GB_REQUIRE((int64_t)(a.nblk + b.nblk) * cs < (int64_t)1 << 31,
+               "gemm: operand too large to slice");
     launch_chained(small ? slice_cluster_kernel<8> : slice_cluster_kernel<32>,
                    dim3((unsigned)(a.nblk + b.nblk) * cs), 256, 0, ctx->stream, cs, 1, a, b, cs);
     count_launch(ctx);

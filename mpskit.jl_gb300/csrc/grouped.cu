@@ -361,10 +361,21 @@ __global__ void label_violation_kernel(const double* __restrict__ src, int64_t R
   for (int64_t sl = blockIdx.x; sl < S; sl += gridDim.x) {
     const int32_t b = labS[sl];
     const double* col = src + sl * sstr;
-    for (int64_t f = threadIdx.x; f < F; f += blockDim.x) {
-      if (col[f * fstr] == 0.0) continue;
-      const int32_t a = labF[f];
-      c += (a == NO_LABEL || b == NO_LABEL || a != b);
+    // zero tests on the bits (comparisons run on the FP64 pipe), four loads in flight
+    constexpr int U = 4;
+    for (int64_t f0 = threadIdx.x; f0 < F; f0 += U * 256) {
+      unsigned long long v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int64_t f = f0 + 256 * u;
+        v[u] = f < F ? (unsigned long long)__double_as_longlong(col[f * fstr]) << 1 : 0ull;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (v[u] == 0) continue;
+        const int32_t a = labF[f0 + 256 * u];
+        c += (a == NO_LABEL || b == NO_LABEL || a != b);
+      }
     }
   }
   for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
@@ -377,7 +388,7 @@ __global__ void dense_nnz_kernel(const double* __restrict__ src, int64_t rows, i
   const int64_t n = rows * cols;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
-    c += (src[(i % rows) + ld * (i / rows)] != 0.0);
+    c += ((unsigned long long)__double_as_longlong(src[(i % rows) + ld * (i / rows)]) << 1) != 0;
   for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(nnz, c);
 }

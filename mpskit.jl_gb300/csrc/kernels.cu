@@ -107,7 +107,33 @@ void permute(gb_ctx* ctx, int dtype, int nd, const int64_t* dims, const void* in
 }
 
 // ------------------------------------------------------------------ sparse mode mix
-template <typename T>
+// 1 * x + 0 as the sum below gives it, without the FP64 pipe: -0 becomes +0; a complex value
+// with an infinite or NaN part takes the products
+__device__ __forceinline__ double unit_term(double x) {
+  return ((unsigned long long)__double_as_longlong(x) << 1) == 0ull ? 0.0 : x;
+}
+__device__ __noinline__ dcx unit_term_slow(dcx x) {
+  return Ops<dcx>::fmaop(mk(1.0, 0.0), x, Ops<dcx>::zero());
+}
+__device__ __forceinline__ dcx unit_term(dcx x) {
+  const unsigned inf = 0x7ff00000u;
+  if (__builtin_expect((__double2hiint(x.re) & inf) == inf || (__double2hiint(x.im) & inf) == inf,
+                       0))
+    return unit_term_slow(x);
+  return mk(unit_term(x.re), unit_term(x.im));
+}
+__device__ __forceinline__ bool is_unit(double v) {
+  return __double_as_longlong(v) == 0x3ff0000000000000ll;
+}
+__device__ __forceinline__ bool is_unit(dcx v) {
+  return is_unit(v.re) && ((unsigned long long)__double_as_longlong(v.im) << 1) == 0ull;
+}
+
+// y[a, J, n] = sum_e val[e] x[a, col[e], n] (+ beta y).  A row of one entry with coefficient 1 --
+// the channels of an environment cut out of it -- is a copy, without FP64 arithmetic (16 clocks
+// per warp instruction and SM).
+// MIXC: entries in flight per thread
+template <typename T, int MIXC>
 __global__ void mix_kernel(int64_t A, int64_t N, int64_t xa, int64_t xn, int64_t ya, int64_t yn,
                            const int64_t* __restrict__ in_off, const int64_t* __restrict__ out_off,
                            const int* __restrict__ row_ptr, const int* __restrict__ col,
@@ -117,22 +143,60 @@ __global__ void mix_kernel(int64_t A, int64_t N, int64_t xa, int64_t xn, int64_t
   const int J = blockIdx.y;
   const int e0 = row_ptr[J], e1 = row_ptr[J + 1];
   const int64_t yo = out_off[J];
-  for (int64_t n = blockIdx.z; n < N; n += gridDim.z) {
-    for (int64_t a = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; a < A;
-         a += (int64_t)gridDim.x * blockDim.x) {
-      T acc = Ops<T>::zero();
-      const int64_t xb = a * xa + n * xn;
-      for (int e = e0; e < e1; ++e) acc = Ops<T>::fmaop(val[e], x[xb + in_off[col[e]]], acc);
-      T* yp = y + a * ya + yo + n * yn;
-      if (beta != 0.0) {
-        T old = *yp;
-        if constexpr (sizeof(T) == 8) {
-          acc = acc + beta * old;
-        } else {
-          acc = Ops<T>::add(acc, mk(beta * old.re, beta * old.im));
+  if (beta == 0.0 && e1 - e0 == 1 && is_unit(val[e0])) {
+    const int64_t io = in_off[col[e0]], piece = (int64_t)MIXC * blockDim.x;
+    for (int64_t n = blockIdx.z; n < N; n += gridDim.z) {
+      const T* xp = x + io + n * xn;
+      T* yp = y + yo + n * yn;
+      for (int64_t a0 = blockIdx.x * piece + threadIdx.x; a0 < A; a0 += gridDim.x * piece) {
+        T v[MIXC];
+#pragma unroll
+        for (int i = 0; i < MIXC; ++i) {
+          const int64_t a = a0 + i * blockDim.x;
+          if (a < A) v[i] = xp[a * xa];
+        }
+#pragma unroll
+        for (int i = 0; i < MIXC; ++i) {
+          const int64_t a = a0 + i * blockDim.x;
+          if (a < A) yp[a * ya] = unit_term(v[i]);
         }
       }
-      *yp = acc;
+    }
+    return;
+  }
+  const int64_t piece = (int64_t)MIXC * blockDim.x;
+  for (int64_t n = blockIdx.z; n < N; n += gridDim.z) {
+    for (int64_t a0 = blockIdx.x * piece + threadIdx.x; a0 < A; a0 += gridDim.x * piece) {
+      T acc[MIXC];
+#pragma unroll
+      for (int i = 0; i < MIXC; ++i) acc[i] = Ops<T>::zero();
+      const T* xp = x + a0 * xa + n * xn;
+      for (int e = e0; e < e1; ++e) {
+        const T* xe = xp + in_off[col[e]];
+        const T c = val[e];
+        T v[MIXC];
+#pragma unroll
+        for (int i = 0; i < MIXC; ++i)
+          if (a0 + i * blockDim.x < A) v[i] = xe[i * blockDim.x * xa];
+#pragma unroll
+        for (int i = 0; i < MIXC; ++i)
+          if (a0 + i * blockDim.x < A) acc[i] = Ops<T>::fmaop(c, v[i], acc[i]);
+      }
+      T* yp = y + a0 * ya + yo + n * yn;
+#pragma unroll
+      for (int i = 0; i < MIXC; ++i) {
+        if (a0 + i * blockDim.x >= A) continue;
+        T* p = yp + i * blockDim.x * ya;
+        if (beta != 0.0) {
+          const T old = *p;
+          if constexpr (sizeof(T) == 8) {
+            acc[i] = acc[i] + beta * old;
+          } else {
+            acc[i] = Ops<T>::add(acc[i], mk(beta * old.re, beta * old.im));
+          }
+        }
+        *p = acc[i];
+      }
     }
   }
 }
@@ -195,17 +259,26 @@ void mix_free(MixDev& m) {
 void mix_run(gb_ctx* ctx, const MixDev& m, int dtype, const void* x, void* y, double beta) {
   if (m.nJ == 0 || m.A == 0 || m.N == 0) return;
   GB_REQUIRE(m.nJ <= 65535, "mix: too many output rows");
-  dim3 grid(nblocks(m.A, 128, 64), (unsigned)m.nJ, (unsigned)std::min<int64_t>(m.N, 65535));
+  // Few entries: a block per 128, every SM as soon as possible (four entries per thread cost the
+  // 3 MB mix of a D = 64 solve 2 us).  Many: four entries in flight per thread and blocks that walk
+  // several columns (1.3 GB of channels in blocks of 128 entries: the launch of the blocks is the
+  // bound, 1.29 ms against 0.41).
+  const int64_t sms = std::max(1, ctx->num_sms);
+  const bool many = (m.A + 127) / 128 * m.nJ * m.N > 64 * sms;
+  const int64_t gx = nblocks(m.A, many ? 512 : 128, 64);
+  const int64_t fill = many ? (64 * sms + gx * m.nJ - 1) / (gx * m.nJ) : m.N;
+  dim3 grid((unsigned)gx, (unsigned)m.nJ, (unsigned)std::min<int64_t>({m.N, fill, 65535}));
+  auto run = [&](auto kernel, auto* v) {
+    using T = std::decay_t<decltype(*v)>;
+    launch_chained(kernel, grid, 128, 0, ctx->stream, 1, 1, m.A, m.N, m.xa, m.xn, m.ya, m.yn,
+                   m.in_off, m.out_off, m.row_ptr, m.col, (const T*)m.val, (const T*)x, (T*)y, beta);
+  };
   if (is_cplx(dtype)) {
     GB_REQUIRE(m.cplx, "mix: complex data needs complex coefficients");
-    launch_chained(mix_kernel<dcx>, grid, 128, 0, ctx->stream, 1, 1, m.A, m.N, m.xa, m.xn, m.ya,
-                   m.yn, m.in_off, m.out_off, m.row_ptr, m.col, (const dcx*)m.val, (const dcx*)x,
-                   (dcx*)y, beta);
+    run(many ? mix_kernel<dcx, 4> : mix_kernel<dcx, 1>, (dcx*)nullptr);
   } else {
     GB_REQUIRE(!m.cplx, "mix: real data needs real coefficients");
-    launch_chained(mix_kernel<double>, grid, 128, 0, ctx->stream, 1, 1, m.A, m.N, m.xa, m.xn, m.ya,
-                   m.yn, m.in_off, m.out_off, m.row_ptr, m.col, m.val, (const double*)x,
-                   (double*)y, beta);
+    run(many ? mix_kernel<double, 4> : mix_kernel<double, 1>, (double*)nullptr);
   }
   LAUNCH_CHECK();
   count_launch(ctx);
