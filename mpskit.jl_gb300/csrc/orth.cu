@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <mutex>
 
 #include "gb_common.h"
 #include "tc_ptx.cuh"
@@ -35,6 +36,8 @@ namespace {
 constexpr int OT = 512;              // threads per block
 constexpr int OW = OT / 32;          // warps
 constexpr int OKMAX = 128;           // basis vectors
+constexpr int LONG_PIECE = 1024;     // entries of a block's piece
+constexpr size_t OPIECE = 192 * 1024;  // bytes of a piece kept in shared memory
 
 struct OrthArgs {
   int64_t n, ld;
@@ -145,13 +148,27 @@ __device__ __forceinline__ void lane_sums(double (&v)[N], int lane) {
 // warp takes four vectors (and a share of the block's piece, so that every scheduler has work
 // for short lists of vectors).
 constexpr int JB = 4;
+// four sums per task: as many tasks as lists of four vectors, or two rounds of the warps
+constexpr int DOT_SUMS = JB * (OKMAX / JB + 1 > 2 * OW ? OKMAX / JB + 1 : 2 * OW);
+// Shares of the piece per four vectors.  Short pieces: eight tasks, two per scheduler (more only
+// add reductions).  Long ones: one or two full rounds of the warps, whichever leaves fewer idle --
+// with eight tasks half of them waited for the others' loads (3.5 M real entries, 12 vectors:
+// 472 us, 281 us with 16 to 32 tasks, the piece of w in shared memory and pairs of entries below;
+// pieces of up to 860 entries: the same either way).
+__device__ __forceinline__ int dot_shares(int groups, int len) {
+  if (len < LONG_PIECE) return groups >= 8 ? 1 : max(1, min(8 / groups, (len + 31) / 32));
+  const int a = max(1, OW / groups), b = max(1, 2 * OW / groups);
+  // tasks per round: a against b in rounds of OW
+  const int ra = (groups * a + OW - 1) / OW, rb = (groups * b + OW - 1) / OW;
+  return a * rb >= b * ra ? a : b;
+}
 template <bool CPLX, typename T>
 __device__ void block_dots(const OrthArgs& g, const T* V, const T* w, int64_t c0, int len, int cnt,
                            double2* sred) {
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int tot = cnt + 1;
   const int groups = (tot + JB - 1) / JB;
-  const int P = groups >= 8 ? 1 : max(1, min(8 / groups, (len + 31) / 32));
+  const int P = dot_shares(groups, len);
   for (int t = warp; t < groups * P; t += OW) {
     const int j1 = t / P * JB, p = t % P;
     const int nj = tot - j1;
@@ -162,7 +179,7 @@ __device__ void block_dots(const OrthArgs& g, const T* V, const T* w, int64_t c0
 #pragma unroll
     for (int j = 0; j < (CPLX ? 2 * JB : JB); ++j) acc[j] = 0.0;
     double none = 0.0;
-#pragma unroll 2
+#pragma unroll(CPLX ? 2 : 4)
     for (int i = p * 32 + lane; i < len; i += 32 * P) {
       const T b = w[i];
       T a[JB];
@@ -245,7 +262,7 @@ template <bool CPLX>
 __global__ void __launch_bounds__(OT, 1) krylov_orth_kernel(OrthArgs g) {
   using T = typename Num<CPLX>::T;
   extern __shared__ __align__(16) unsigned char piece[];
-  __shared__ double2 sred[OKMAX + 9 * JB];
+  __shared__ double2 sred[DOT_SUMS];
   __shared__ double2 sc[OKMAX + 1], sh[OKMAX + 1];
   __shared__ double2 spart[96];
   __shared__ double sinv, sleft;
@@ -320,7 +337,23 @@ __global__ void __launch_bounds__(OT, 1) krylov_orth_kernel(OrthArgs g) {
         for (int p = 0; p < Q - 1; ++p) add_to(keep, spart[p * L + tid]);
       }
     } else {
-      for (int r = 0; r < rounds; ++r) {
+      // pairs of entries, for twice the loads in flight
+      int r = 0;
+      for (; (r + 2) * OT <= len; r += 2) {
+        const int i = r * OT + tid;
+        T a = w[i], b = w[i + OT];
+        const T* v = V + c0 + i;
+#pragma unroll 8
+        for (int j = 0; j < g.k; ++j) {
+          const T* vj = v + (int64_t)j * g.ld;
+          const T x = vj[0], y = vj[OT];
+          sub_mul(a, x, sc[j]);
+          sub_mul(b, y, sc[j]);
+        }
+        w[i] = a;
+        w[i + OT] = b;
+      }
+      for (; r < rounds; ++r) {
         const int i = r * OT + tid;
         if (i < len) {
           T a = w[i];
@@ -392,7 +425,7 @@ __global__ void __launch_bounds__(OT) krylov_combine_kernel(CombineArgs a) {
   if (a.normalize) {
     __syncthreads();
     unsigned int target = 0;
-    __shared__ double2 sred[9 * JB];
+    __shared__ double2 sred[DOT_SUMS];
     block_dots<CPLX>(g, (const T*)nullptr, src, c0, len, 0, sred);
     __shared__ double sinv;
     if (all_sums(g, 1, sc, target)) {
@@ -465,10 +498,17 @@ void krylov_orth_start(gb_ctx* ctx, int dtype, int64_t n, int k, bool predict, c
   g.vnext = (double*)vnext;
   const int64_t per = ((n + blocks - 1) / blocks + 31) / 32 * 32;
   const size_t bytes = (size_t)per * elem_size(dtype);
-  g.in_smem = bytes <= 32 * 1024;
+  g.in_smem = bytes <= OPIECE;
   g.out = host_results(ctx, OSLOT * ORTH_SLOTS) + OSLOT * slot;
   if (!ctx->orth_done[slot])
     GB_CHECK_CUDA(cudaEventCreateWithFlags(&ctx->orth_done[slot], cudaEventDisableTiming));
+  static std::once_flag once;  // contexts may launch from several host threads
+  std::call_once(once, [] {
+    GB_CHECK_CUDA(cudaFuncSetAttribute(krylov_orth_kernel<true>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OPIECE));
+    GB_CHECK_CUDA(cudaFuncSetAttribute(krylov_orth_kernel<false>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OPIECE));
+  });
   void* args[] = {&g};
   GB_CHECK_CUDA(cudaLaunchCooperativeKernel(
       is_cplx(dtype) ? (const void*)krylov_orth_kernel<true> : (const void*)krylov_orth_kernel<false>,

@@ -94,3 +94,31 @@ def test_solve_that_exhausts_its_space(ctx, D):
     assert abs(val - np.linalg.eigvalsh(M)[0]) <= 1e-11 * np.abs(M).max()
     v = vec.numpy().reshape(-1, order="F")
     assert np.linalg.norm(M @ v - val * v) <= 1e-10 * np.abs(M).max()
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.complex128])
+@pytest.mark.parametrize("Dl,Dr", [(190, 190), (275, 280), (500, 340)])
+def test_solve_over_pieces_short_and_long(ctx, Dl, Dr, dtype):
+    """Pieces of 480, 1024 and 2240 entries per multiprocessor (short and long lists of sums in the
+    steps and in the final combination): the returned vector has norm one and the returned value
+    is its expectation value, each to the rounding of 2 Dl Dr squares added pairwise in parts."""
+    H = mpsgb.transverse_field_ising(8, dtype=dtype)
+    W = H.device(ctx, dtype)[3]
+    rng = np.random.default_rng(Dl)
+
+    def env(D, wide):
+        g = rng.standard_normal((D, wide, D)) / np.sqrt(D)
+        return (g + g.transpose(2, 1, 0)).astype(dtype)
+
+    op = mpsgb.DerivativeOperator(
+        ctx, L.GB_HEFF_AC, mpsgb.DeviceTensor.from_numpy(ctx, "gl", env(Dl, 3)),
+        W, None, mpsgb.DeviceTensor.from_numpy(ctx, "gr", env(Dr, 3)),
+        mpsgb.GB300Backend("fp64"))
+    x = rng.standard_normal((Dl, 2, Dr)).astype(dtype)
+    x0 = mpsgb.DeviceTensor.from_numpy(ctx, "mps", x / np.linalg.norm(x))
+    val, vec, _ = mpsgb.fixedpoint(op, x0, "SR", mpsgb.Lanczos(12, 1, 1e-12, True))
+    v = vec.numpy()
+    assert abs(np.linalg.norm(v) - 1) <= 64 * EPS
+    y = op(vec).numpy()
+    assert abs(np.vdot(v, y) - val) <= 1e-12 * np.linalg.norm(y)
+    assert ctx.device_status() == 0
