@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1)
   int* seb = (int*)(tmem_slot + 1);  // [BN] column exponents
   int* sea = seb + BN;               // [128] row exponents
 
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int warp = warp_index(), lane = threadIdx.x % 32;
   const int mi = blockIdx.x % g.mt, rest = blockIdx.x / g.mt;
   const int ni = rest % g.nt, z = rest / g.nt;
   const int split = blockIdx.y;
@@ -590,7 +590,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1)
   const int b1 = (int)((int64_t)cnt * (split + 1) / g.splits);
   const int nb = b1 - b0;
 
-  if (warp == 0 && lane == 0) {
+  if (warp == 0 && elect_one()) {
     // ---------------- TMA producer
     uint32_t ia = 0, ib = 0;
     bool ok = true;
@@ -621,7 +621,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1)
       for (uint32_t t = ib > (uint32_t)S::BST ? ib - S::BST : 0; t < ib; ++t)
         mbar_wait_bounded(smem_u32(&fullB[t % S::BST]), (t / S::BST) & 1, g.status, DRAIN_WAIT_NS);
     }
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1 && elect_one()) {
     // ---------------- MMA issuer
     uint32_t ia = 0, ib = 0;
     bool ok = true;

@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   uint64_t* accum = bars + 2 * TC_STAGES;   // [1]
   uint32_t* tmem_slot = (uint32_t*)(bars + 2 * TC_STAGES + 1);
 
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int warp = warp_index(), lane = threadIdx.x % 32;
   const int64_t m0 = (int64_t)blockIdx.x * TC_BM;
   const int64_t n0 = (int64_t)blockIdx.y * TC_BN;
   const int bz = blockIdx.z;
@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  if (warp == 0 && lane == 0) {
+  if (warp == 0 && elect_one()) {
     // ---------------- TMA producer
     int issued = 0;
     bool ok = true;
@@ -576,7 +576,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         mbar_wait_bounded(smem_u32(&full[s]), (it / TC_STAGES) & 1, args.status, DRAIN_WAIT_NS);
       }
     }
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1 && elect_one()) {
     // ---------------- MMA issuer
     const uint32_t idesc = idesc_bf16(TC_BM, TC_BN);
     bool ok = true;
@@ -676,6 +676,7 @@ struct PArgs {
 };
 
 constexpr int PS_RING = 4;
+constexpr int PS_THREADS = 224;  // A loads and schedule, MMA, four epilogue warps, B loads
 
 
 template <int BN>
@@ -702,7 +703,7 @@ __device__ __forceinline__ TileMasks<BN> tile_masks(const PArgs& p, int mi, int 
 }
 
 template <int BN, int STAGES, bool TF32>
-__global__ void __launch_bounds__(TC_THREADS, 1)
+__global__ void __launch_bounds__(PS_THREADS, 1)
     gemm_bf16x3_persistent(const __grid_constant__ CUtensorMap mapA,
                            const __grid_constant__ CUtensorMap mapB, PArgs args) {
   constexpr int BKE = TF32 ? 32 : 64;  // k elements per stage (one 128-byte swizzle row)
@@ -723,12 +724,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   int* snk = stile + PS_RING;                   // [RING]
   uint32_t* tmem_slot = (uint32_t*)(snk + PS_RING);
 
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int warp = warp_index(), lane = threadIdx.x % 32;
   const int mn = args.mt * args.nt;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
-      mbar_init(smem_u32(&full[s]), 1);
+      mbar_init(smem_u32(&full[s]), 2);  // both producers
       mbar_init(smem_u32(&empty[s]), 1);
     }
     for (int b = 0; b < 2; ++b) {
@@ -737,7 +738,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     }
     for (int r = 0; r < PS_RING; ++r) {
       mbar_init(smem_u32(&sfull[r]), 1);
-      mbar_init(smem_u32(&sempty[r]), 5);  // MMA thread + 4 epilogue warps
+      mbar_init(smem_u32(&sempty[r]), 6);  // B producer, MMA thread, 4 epilogue warps
     }
     mbar_init(smem_u32(done), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -755,9 +756,47 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  if (warp == 0 && lane == 0) {
-    // ---------------- scheduler + TMA producer
-    uint32_t g = 0, issued = 0;
+  // The k-blocks of a tile, the three plane pairs one after the other: load(stage, kb, plane of A,
+  // plane of B) once the stage is free.  A wait, an expect and a copy are some 200 clocks of the
+  // issuing thread, so A and B have a producer each (256 x 1024 x 1024 tf32x3: 39.0 and 37.8 us).
+  auto produce = [&](int mi, int ni, int z, uint32_t& g, auto&& load) -> bool {
+    TileMasks<BN> tm;
+    if (args.maskA) tm = tile_masks<BN>(args, mi, ni, z);
+    for (int pair = 0; pair < 3; ++pair) {
+      const int planeA = (pair == 2) ? 1 : 0, planeB = (pair == 1) ? 1 : 0;
+      for (int w = 0; w < (args.maskA ? args.kw : 1); ++w) {
+        uint32_t bits = args.maskA ? tm.word(w, args.kw) : 0u;
+        int kb = args.maskA ? -1 : 0;
+        for (;;) {
+          if (args.maskA) {
+            if (!bits) break;
+            kb = w * 32 + __ffs(bits) - 1;
+            bits &= bits - 1;
+          } else if (kb >= args.kblocks) {
+            break;
+          }
+          const int s = g % STAGES;
+          if (!mbar_wait_bounded(smem_u32(&empty[s]), ((g / STAGES) & 1) ^ 1, args.status,
+                                 args.wait_ns))
+            return false;
+          load(s, kb, planeA, planeB);
+          ++g;
+          if (!args.maskA) ++kb;
+        }
+      }
+    }
+    return true;
+  };
+  // drain copies still in flight before this CTA may exit
+  auto drain = [&](uint32_t issued) {
+    for (uint32_t it = issued > (uint32_t)STAGES ? issued - STAGES : 0; it < issued; ++it)
+      mbar_wait_bounded(smem_u32(&full[it % STAGES]), (it / STAGES) & 1, args.status,
+                        DRAIN_WAIT_NS);
+  };
+
+  if (warp == 0 && elect_one()) {
+    // ---------------- scheduler + producer of A
+    uint32_t g = 0;
     bool ok = true;
     for (int j = 0; ok; ++j) {
       int t = -1, nk = 0, mi = 0, ni = 0, z = 0;
@@ -818,46 +857,39 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           if (n1 > args.Nlog) set_range(std::max(n0, args.Nlog) - args.Nlog, n1 - args.Nlog);
         }
       }
-      const int64_t m0 = (int64_t)mi * TC_BM, n0 = (int64_t)ni * BN;
-      const int za0 = (args.batchA > 1 ? z : 0) * 2, zb0 = (args.batchB > 1 ? z : 0) * 2;
-      TileMasks<BN> tm;
-      if (args.maskA) tm = tile_masks<BN>(args, mi, ni, z);
-      for (int pair = 0; pair < 3 && ok; ++pair) {
-        const int planeA = (pair == 2) ? 1 : 0, planeB = (pair == 1) ? 1 : 0;
-        for (int w = 0; w < (args.maskA ? args.kw : 1) && ok; ++w) {
-          uint32_t bits = args.maskA ? tm.word(w, args.kw) : 0u;
-          int kb = args.maskA ? -1 : 0;
-          for (;;) {
-            if (args.maskA) {
-              if (!bits) break;
-              kb = w * 32 + __ffs(bits) - 1;
-              bits &= bits - 1;
-            } else if (kb >= args.kblocks) {
-              break;
-            }
-            const int s = g % STAGES;
-            ok = mbar_wait_bounded(smem_u32(&empty[s]), ((g / STAGES) & 1) ^ 1, args.status, args.wait_ns);
-            if (!ok) break;
-            const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);
-            const uint32_t fb = smem_u32(&full[s]);
-            mbar_expect_tx(fb, STAGE_BYTES);
-            tma_load_3d(sa, &mapA, fb, kb * BKE, (int)m0, za0 + planeA);
-            tma_load_3d(sa + A_BYTES, &mapB, fb, kb * BKE, (int)n0, zb0 + planeB);
-            ++g;
-            ++issued;
-            if (!args.maskA) ++kb;
-          }
-        }
-      }
+      const int64_t m0 = (int64_t)mi * TC_BM;
+      const int za0 = (args.batchA > 1 ? z : 0) * 2;
+      ok = produce(mi, ni, z, g, [&](int s, int kb, int planeA, int) {
+        const uint32_t fb = smem_u32(&full[s]);
+        mbar_expect_tx(fb, A_BYTES);
+        tma_load_3d(smem_u32(smem + s * STAGE_BYTES), &mapA, fb, kb * BKE, (int)m0, za0 + planeA);
+      });
     }
-    if (!ok) {
-      // drain copies still in flight before this CTA may exit
-      for (uint32_t it = issued > (uint32_t)STAGES ? issued - STAGES : 0; it < issued; ++it) {
-        const int s = it % STAGES;
-        mbar_wait_bounded(smem_u32(&full[s]), (it / STAGES) & 1, args.status, DRAIN_WAIT_NS);
-      }
+    if (!ok) drain(g);
+  } else if (warp == 6 && elect_one()) {
+    // ---------------- producer of B
+    uint32_t g = 0;
+    bool ok = true;
+    for (int j = 0; ok; ++j) {
+      const int slot = j % PS_RING;
+      ok = mbar_wait_bounded(smem_u32(&sfull[slot]), (j / PS_RING) & 1, args.status, args.wait_ns);
+      if (!ok) break;
+      const int t = stile[slot], nk = snk[slot];
+      mbar_arrive(smem_u32(&sempty[slot]));
+      if (t < 0) break;
+      if (nk == 0) continue;
+      const int z = t / mn, r = t - z * mn;
+      const int ni = r / args.mt, mi = r - ni * args.mt;
+      const int n0 = ni * BN, zb0 = (args.batchB > 1 ? z : 0) * 2;
+      ok = produce(mi, ni, z, g, [&](int s, int kb, int, int planeB) {
+        const uint32_t fb = smem_u32(&full[s]);
+        mbar_expect_tx(fb, B_BYTES);
+        tma_load_3d(smem_u32(smem + s * STAGE_BYTES) + A_BYTES, &mapB, fb, kb * BKE, n0,
+                    zb0 + planeB);
+      });
     }
-  } else if (warp == 1 && lane == 0) {
+    if (!ok) drain(g);
+  } else if (warp == 1 && elect_one()) {
     // ---------------- MMA issuer
     const uint32_t idesc = TF32 ? idesc_tf32(TC_BM, BN) : idesc_bf16(TC_BM, BN);
     uint32_t g = 0, acc = 0;
@@ -903,7 +935,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     // every MMA issued by this thread has retired once `done` completes
     mma_commit(smem_u32(done));
     mbar_wait_bounded(smem_u32(done), 0, args.status, DRAIN_WAIT_NS);
-  } else if (warp >= 2) {
+  } else if (warp >= 2 && warp < 6) {
     // ---------------- epilogue: TMEM -> registers -> FP64 global
     const int q = warp % 4;  // TMEM lane quarter accessible by this warp
     uint32_t acc = 0;
@@ -1222,7 +1254,7 @@ void gemm_split(gb_ctx* ctx, int dtype, const Packed& A, const Packed& B, int64_
       GB_CHECK_CUDA(cudaFuncSetAttribute(gemm_bf16x3_persistent<BN_, ST_, TF_>,               \
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, SM));   \
     });                                                                                       \
-    gemm_bf16x3_persistent<BN_, ST_, TF_><<<grid, TC_THREADS, SM, ctx->stream>>>(ma, mb, p); \
+    gemm_bf16x3_persistent<BN_, ST_, TF_><<<grid, PS_THREADS, SM, ctx->stream>>>(ma, mb, p); \
   } while (0)
     if (bn == 64) {
       if (tf32) GB_PERSISTENT(64, 8, true);

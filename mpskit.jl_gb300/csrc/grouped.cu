@@ -701,7 +701,7 @@ __global__ void __launch_bounds__(G_THREADS, 1)
   uint32_t* tmem_slot = (uint32_t*)(stile + G_RING);
   int* sflag = (int*)(tmem_slot + 1);    // split tile: units done before this one
 
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int warp = warp_index(), lane = threadIdx.x % 32;
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(smem_u32(&full[s]), 1);
@@ -733,7 +733,7 @@ __global__ void __launch_bounds__(G_THREADS, 1)
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  if (warp == 0 && lane == 0) {
+  if (warp == 0 && elect_one()) {
     // ---------------- scheduler + TMA producer
     uint32_t g = 0, issued = 0;
     bool ok = true;
@@ -778,7 +778,7 @@ __global__ void __launch_bounds__(G_THREADS, 1)
         mbar_wait_bounded(smem_u32(&full[it % STAGES]), (it / STAGES) & 1, args.status,
                           DRAIN_WAIT_NS);
     }
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1 && elect_one()) {
     // ---------------- MMA issuer
     uint32_t g = 0, acc = 0;
     bool ok = true;

@@ -100,6 +100,23 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                : "memory");
 }
+// The warp's index as a value the compiler knows to be the same in all lanes, and one lane of a
+// converged warp, known to be a single one.  Copies, MMAs and commits take their operands from
+// uniform registers: under a plain `lane == 0` each of them is issued in a loop over whatever
+// lanes may be active, and the issuing threads, not the memory or the tensor cores, set the pace
+// (a wait, an expect and a copy: 302 clocks under `lane == 0`, 191 here).
+__device__ __forceinline__ int warp_index() {
+  return __shfl_sync(0xffffffffu, (int)threadIdx.x / 32, 0);
+}
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b32 r;\n\t"
+      "elect.sync r|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(one));
+  return one != 0;
+}
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
