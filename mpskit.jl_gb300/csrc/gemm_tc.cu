@@ -270,11 +270,12 @@ void pack_operand(gb_ctx* ctx, int dtype, int role, char op, int64_t R, int64_t 
 // the packed B operand of the following GEMM: logical B element (k, m) with
 // k = a + kJ[J] (contraction index) and m = mJ[J] + n*mn (output column index).
 //
-// A block takes one output row J and a run of columns n; a thread takes four entries of each.
-// Bound, once the map is marked with one atomic per run and warp instead of one per 32 entries
-// (all of them on a few hundred words), by the FP64 sum (16 clocks per warp instruction and
-// SM) and by the traffic, 4 B read per entry and input and 4 B (BF16) written: 12.4 M entries,
-// one input each, 359 us before, 129 us.
+// A block takes one output row J and a run of columns n, a warp 128 consecutive entries of one
+// column at a time.  Bound by the instructions around an entry, not by the traffic (4 B read per
+// entry and input, 4 B written in BF16), so one test of the written-region map, one reduction of
+// the nonzero flags and at most one atomic serve the 128 entries, and a row of one input with a
+// coefficient that FP32 holds stays in FP32 (FP64 sums cost 16 clocks per warp instruction and
+// SM).  12.4 M entries, one input each: 129 us with 32 entries per test and FP64 products, 80 us.
 constexpr int MIXE = 64;  // entries of a row kept in shared memory
 constexpr int MIXU = 4;   // entries of a column per thread
 template <bool CPLX, typename E, typename TX>
@@ -312,8 +313,13 @@ __global__ void __launch_bounds__(128)
   };
   const int64_t k0J = kJ[J], m0J = mJ[J];
   const int64_t n0 = (int64_t)blockIdx.z * nper, n1 = min(N, n0 + nper);
-  // k-blocks already marked in the row tile that the last column fell into, per run of 32
-  // entries (they span two k-blocks at most): bit 2 u + (second block)
+  // One input with a coefficient that FP32 holds: its product with an FP32 value, exact in FP64,
+  // rounds to the FP32 product
+  const float c32 = ne == 1 ? to_float(val_of(0, 0)) : 0.f;
+  const bool single = std::is_same<TX, float>::value && ne == 1 &&
+                      to_double(c32) == val_of(0, 0) && (!CPLX || val_of(0, CPLX) == 0.0);
+  // k-blocks already marked in the row tile that the last column fell into, counted from the
+  // first one of the warp's run
   int64_t tile = -1, tile_im = -1;
   int64_t base_marked = -1;
   uint32_t marked = 0;
@@ -332,36 +338,33 @@ __global__ void __launch_bounds__(128)
       alo = r.x;
       ahi = r.y;
     }
-    for (int64_t base = alo + (int64_t)blockIdx.x * (128 * MIXU); base < ahi;
-         base += (int64_t)gridDim.x * (128 * MIXU)) {
-      if (base != base_marked) {  // another piece of the column: its k-blocks are others
-        base_marked = base;
+    // a warp's run: MIXU x 32 entries from a0
+    for (int64_t a0 = alo + ((int64_t)blockIdx.x * 4 + threadIdx.x / 32) * (32 * MIXU); a0 < ahi;
+         a0 += (int64_t)gridDim.x * (128 * MIXU)) {
+      if (a0 != base_marked) {  // another piece of the column: its k-blocks are others
+        base_marked = a0;
         marked = 0;
       }
-      // a warp's run u: 32 entries from a0
-      bool hit[MIXU];
-#pragma unroll
-      for (int u = 0; u < MIXU; ++u) {
-        const int64_t a0 = base + u * 128 + (threadIdx.x & ~31);
-        hit[u] = a0 < ahi;
-        if (sk.xmap && !sk.arange && hit[u]) {
-          // input e of element (a, n) lies in box (row, column) of x's written-region map; the
-          // producer keeps every region outside the map at zero.  The run spans at most two
-          // row boxes per input, so one pass of the lanes over the inputs decides.
-          const int64_t a1 = min(a0 + 31, A - 1);
-          bool h = false;
-          for (int e = lane; e < ne && !h; e += 32) {
-            const int64_t ro = e < MIXE ? s_roff[e] : sk.roff[col[e0 + e]];
-            const int64_t co = e < MIXE ? s_coff[e] : sk.coff[col[e0 + e]];
-            const int64_t cb = (co + n * sk.xnM) >> 7;
-            const int64_t q0 = ((a0 + ro) >> 7) * sk.onc + cb, q1 = ((a1 + ro) >> 7) * sk.onc + cb;
-            h = ((sk.xmap[q0 >> 5] >> (q0 & 31)) & 1u) || ((sk.xmap[q1 >> 5] >> (q1 & 31)) & 1u);
-          }
-          hit[u] = __any_sync(0xffffffffu, h);
-          if (!hit[u] && a0 + lane < A) {
-            // nothing to read: the output is zero; it is written only where the previous
-            // apply marked its box (the planes hold zeros everywhere else)
-            const int64_t k = a0 + lane + k0J, kb0 = k / BK;
+      const int64_t a = a0 + lane;
+      const int left = (int)min(ahi - a, (int64_t)(32 * MIXU));  // entries from this lane's first
+      if (sk.xmap && !sk.arange) {
+        // input e of element (a, n) lies in box (row, column) of x's written-region map; the
+        // producer keeps every region outside the map at zero.  The run spans at most two
+        // row boxes per input, so one pass of the lanes over the inputs decides.
+        const int64_t a1 = min(a0 + 32 * MIXU - 1, A - 1);
+        bool h = false;
+        for (int e = lane; e < ne && !h; e += 32) {
+          const int64_t ro = e < MIXE ? s_roff[e] : sk.roff[col[e0 + e]];
+          const int64_t co = e < MIXE ? s_coff[e] : sk.coff[col[e0 + e]];
+          const int64_t cb = (co + n * sk.xnM) >> 7;
+          const int64_t q0 = ((a0 + ro) >> 7) * sk.onc + cb, q1 = ((a1 + ro) >> 7) * sk.onc + cb;
+          h = ((sk.xmap[q0 >> 5] >> (q0 & 31)) & 1u) || ((sk.xmap[q1 >> 5] >> (q1 & 31)) & 1u);
+        }
+        if (!__any_sync(0xffffffffu, h)) {
+          // nothing to read: the output is zero; it is written only where the previous
+          // apply marked its box (the planes hold zeros everywhere else)
+          for (int u = 0; u < MIXU && 32 * u < left; ++u) {
+            const int64_t k = a + 32 * u + k0J, kb0 = k / BK;
             auto prev = [&](int64_t row, int64_t kb) {
               return (sk.prev[(row / MASK_ROWS) * kw + kb / 32] >> (kb % 32)) & 1u;
             };
@@ -372,61 +375,79 @@ __global__ void __launch_bounds__(128)
               if (prev(Nlog + m, kb0 + Kh / BK)) put(Nlog + m, Kh + k, 0.0);
             }
           }
+          continue;
         }
       }
-      double re[MIXU], im[MIXU];
-#pragma unroll
-      for (int u = 0; u < MIXU; ++u) re[u] = im[u] = 0.0;
-      const int64_t a = base + threadIdx.x;
-      for (int e = 0; e < ne; ++e) {
-        const TX* xe = x + (CPLX ? 2 : 1) * (in_of(e) + n * xn);
-        const double vr = val_of(e, 0), vi = CPLX ? val_of(e, 1) : 0.0;
+      float re[MIXU], im[CPLX ? MIXU : 1];
+      if (single) {
+        const TX* xe = x + (CPLX ? 2 : 1) * (in_of(0) + n * xn + a);
 #pragma unroll
         for (int u = 0; u < MIXU; ++u) {
-          if (!hit[u] || a + u * 128 >= ahi) continue;
-          if (CPLX) {
-            const double xr = to_double(xe[2 * (a + u * 128)]), xi = to_double(xe[2 * (a + u * 128) + 1]);
-            re[u] = fma(vr, xr, fma(-vi, xi, re[u]));
-            im[u] = fma(vr, xi, fma(vi, xr, im[u]));
-          } else {
-            re[u] = fma(vr, to_double(xe[a + u * 128]), re[u]);
+          const bool in = 32 * u < left;
+          re[u] = in ? (float)xe[(CPLX ? 2 : 1) * 32 * u] : 0.f;
+          if (CPLX) im[u] = in ? (float)xe[2 * 32 * u + 1] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < MIXU; ++u) {
+          re[u] *= c32;
+          if (CPLX) im[u] *= c32;
+        }
+      } else {
+        double dre[MIXU], dim[MIXU];
+#pragma unroll
+        for (int u = 0; u < MIXU; ++u) dre[u] = dim[u] = 0.0;
+        for (int e = 0; e < ne; ++e) {
+          const TX* xe = x + (CPLX ? 2 : 1) * (in_of(e) + n * xn + a);
+          const double vr = val_of(e, 0), vi = CPLX ? val_of(e, 1) : 0.0;
+#pragma unroll
+          for (int u = 0; u < MIXU; ++u) {
+            if (32 * u >= left) continue;
+            if (CPLX) {
+              const double xr = to_double(xe[2 * 32 * u]), xi = to_double(xe[2 * 32 * u + 1]);
+              dre[u] = fma(vr, xr, fma(-vi, xi, dre[u]));
+              dim[u] = fma(vr, xi, fma(vi, xr, dim[u]));
+            } else {
+              dre[u] = fma(vr, to_double(xe[32 * u]), dre[u]);
+            }
           }
+        }
+#pragma unroll
+        for (int u = 0; u < MIXU; ++u) {
+          re[u] = to_float(dre[u]);
+          if (CPLX) im[u] = to_float(dim[u]);
         }
       }
+      const int64_t kfirst = (a0 + k0J) / BK;
+      const int koff = (int)(a0 + k0J - kfirst * BK) + lane;  // of this lane's first entry
+      uint32_t want = 0;
+      E *h0 = hi + m * Kp + k0J + a, *l0 = h0 + plane;
 #pragma unroll
       for (int u = 0; u < MIXU; ++u) {
-        const bool valid = hit[u] && a + u * 128 < ahi;
-        const int64_t k = a + u * 128 + k0J;
-        bool nz = false;
-        if (valid) {
-          put(m, k, re[u]);
-          nz = (__double_as_longlong(re[u]) << 1) != 0;
-          if (CPLX) {
-            const double mim = __longlong_as_double(__double_as_longlong(im[u]) ^ (1ll << 63));
-            put(m, Kh + k, mim);
-            put(Nlog + m, k, im[u]);
-            put(Nlog + m, Kh + k, re[u]);
-            nz |= (__double_as_longlong(im[u]) << 1) != 0;
-          }
+        if (32 * u >= left) continue;
+        uint32_t bits = __float_as_uint(re[u]) << 1;
+        split_put_f(h0, l0, 32 * u, re[u]);
+        if (CPLX) {
+          bits |= __float_as_uint(im[u]) << 1;
+          split_put_f(h0 + Kh, l0 + Kh, 32 * u, -im[u]);
+          split_put_f(h0 + Nlog * Kp, l0 + Nlog * Kp, 32 * u, im[u]);
+          split_put_f(h0 + Nlog * Kp + Kh, l0 + Nlog * Kp + Kh, 32 * u, re[u]);
         }
-        const int64_t kfirst = __shfl_sync(0xffffffffu, k, 0) / BK;
-        const unsigned all = __ballot_sync(0xffffffffu, nz);
-        const unsigned second = __ballot_sync(0xffffffffu, k / BK != kfirst);
-        const uint32_t want = ((all & ~second) ? 1u : 0u) | ((all & second) ? 2u : 0u);
-        const uint32_t fresh = want & ~(marked >> (2 * u));
-        if (fresh) {
-          marked |= fresh << (2 * u);
-          if (lane < 2 && ((fresh >> lane) & 1u)) {
-            const int64_t kb = kfirst + lane;
-            auto mark = [&](int64_t row, int64_t b) {
-              atomicOr(&mask[(row / MASK_ROWS) * kw + b / 32], 1u << (b % 32));
-            };
-            mark(m, kb);
-            if (CPLX) {
-              mark(m, kb + Kh / BK);
-              mark(Nlog + m, kb);
-              mark(Nlog + m, kb + Kh / BK);
-            }
+        if (bits) want |= 1u << ((koff + 32 * u) / BK);
+      }
+      want = __reduce_or_sync(0xffffffffu, want);
+      const uint32_t fresh = want & ~marked;
+      if (fresh) {
+        marked |= fresh;
+        if ((fresh >> lane) & 1u) {
+          const int64_t kb = kfirst + lane;
+          auto mark = [&](int64_t row, int64_t b) {
+            atomicOr(&mask[(row / MASK_ROWS) * kw + b / 32], 1u << (b % 32));
+          };
+          mark(m, kb);
+          if (CPLX) {
+            mark(m, kb + Kh / BK);
+            mark(Nlog + m, kb);
+            mark(Nlog + m, kb + Kh / BK);
           }
         }
       }
