@@ -77,8 +77,8 @@ __device__ inline void load_elem(const PackArgs& p, const double* src, int64_t r
 
 // 32 x 32 tile transpose through shared memory; block = 32 x 8 threads.
 template <typename E>
-__global__ void pack_kernel(PackArgs p, const double* __restrict__ src, E* __restrict__ dst,
-                            uint32_t* __restrict__ mask, int kw, int64_t mrows) {
+__global__ void pack_kernel(PackArgs p, const double* src, E* dst, uint32_t* mask, int kw,
+                            int64_t mrows) {
   __shared__ double tre[32][33];
   __shared__ double tim[32][33];
   const int64_t b = blockIdx.z;
@@ -87,6 +87,8 @@ __global__ void pack_kernel(PackArgs p, const double* __restrict__ src, E* __res
   E* lo = hi + p.rows * p.Kp;
   const int64_t r0 = (int64_t)blockIdx.y * 32, k0 = (int64_t)blockIdx.x * 32;
   const int tx = threadIdx.x, ty = threadIdx.y;
+  chain_release();
+  chain_wait();
   bool rowfast = (p.role == 0) ? (p.op == 'N') : (p.op != 'N');
   // load: contiguous source index on threadIdx.x
   for (int j = ty; j < 32; j += 8) {
@@ -229,9 +231,26 @@ __global__ void nonzero_products_kernel(const uint32_t* __restrict__ ca, const u
   if ((threadIdx.x & 31) == 0 && acc != 0.0) atomicAdd(&work[1], 2.0 * acc);
 }
 
-static void clear_mask(gb_ctx* ctx, const Packed& p) {
-  GB_CHECK_CUDA(cudaMemsetAsync(p.mask, 0, (size_t)p.batch * p.mrows * p.kw * 4, ctx->stream));
+// prev = map (if asked for), map = 0
+__global__ void map_reset_kernel(uint32_t* map, uint32_t* prev, int64_t n) {
+  chain_release();
+  chain_wait();
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    if (prev) prev[i] = map[i];
+    map[i] = 0;
+  }
 }
+
+static void map_reset(gb_ctx* ctx, uint32_t* map, uint32_t* prev, size_t bytes) {
+  const int64_t n = (int64_t)(bytes / 4);
+  if (!n) return;
+  launch_chained(map_reset_kernel, dim3((unsigned)std::min<int64_t>((n + 255) / 256, 128)), 256, 0,
+                 ctx->stream, 1, 1, map, prev, n);
+  count_launch(ctx);
+}
+
+static size_t mask_bytes(const Packed& p) { return (size_t)p.batch * p.mrows * p.kw * 4; }
 
 void pack_operand(gb_ctx* ctx, int dtype, int role, char op, int64_t R, int64_t K,
                   const void* src, int64_t ld, int64_t stride, int64_t batch, Packed& out,
@@ -251,15 +270,24 @@ void pack_operand(gb_ctx* ctx, int dtype, int role, char op, int64_t R, int64_t 
   packed_layout(out, dst, R, K, cx, role, batch, prec);
   // the planes need no memset: the kernel writes every (row, k < Kh) entry, zeros
   // included for k >= K; only the nonzero map starts cleared
-  clear_mask(ctx, out);
+  map_reset(ctx, out.mask, nullptr, mask_bytes(out));
   GB_REQUIRE(batch <= 65535 && (R + 31) / 32 <= 65535, "pack: grid too large");
   dim3 grid((unsigned)((p.Kh + 31) / 32), (unsigned)((R + 31) / 32), (unsigned)batch);
-  if (out.esz == 4)
-    pack_kernel<float><<<grid, dim3(32, 8), 0, ctx->stream>>>(p, (const double*)src, (float*)dst,
-                                                              out.mask, out.kw, out.mrows);
-  else
-    pack_kernel<__nv_bfloat16><<<grid, dim3(32, 8), 0, ctx->stream>>>(
-        p, (const double*)src, (__nv_bfloat16*)dst, out.mask, out.kw, out.mrows);
+  auto run = [&](auto kernel, auto* planes) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(32, 8);
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    GB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, p, (const double*)src, planes, out.mask, out.kw,
+                                     out.mrows));
+  };
+  if (out.esz == 4) run(pack_kernel<float>, (float*)dst);
+  else run(pack_kernel<__nv_bfloat16>, (__nv_bfloat16*)dst);
   GB_CHECK_CUDA(cudaGetLastError());
   count_launch(ctx);
   if (ctx->counting) count_cols(ctx, out);
@@ -283,9 +311,9 @@ __global__ void __launch_bounds__(128)
     mixpack_kernel(int64_t A, int64_t N, int64_t xn, const int64_t* __restrict__ in_off,
                    const int64_t* __restrict__ kJ, const int64_t* __restrict__ mJ, int64_t mn,
                    const int* __restrict__ row_ptr, const int* __restrict__ col,
-                   const double* __restrict__ val, const TX* __restrict__ x, E* __restrict__ hi,
-                   int64_t Nlog, int64_t Kp, int64_t Kh, int64_t plane,
-                   uint32_t* __restrict__ mask, int kw, MixSkipDev sk, int64_t nper) {
+                   const double* __restrict__ val, const TX* x, E* hi, int64_t Nlog, int64_t Kp,
+                   int64_t Kh, int64_t plane, uint32_t* mask, int kw, MixSkipDev sk,
+                   int64_t nper) {
   constexpr int BK = bk_of<E>();
   __shared__ int64_t s_in[MIXE], s_roff[MIXE], s_coff[MIXE];
   __shared__ double s_val[(CPLX ? 2 : 1) * MIXE];
@@ -303,6 +331,8 @@ __global__ void __launch_bounds__(128)
     s_val[CPLX ? 2 * e : e] = val[CPLX ? 2 * (e0 + e) : e0 + e];
     if (CPLX) s_val[2 * e + 1] = val[2 * (e0 + e) + 1];
   }
+  chain_release();
+  chain_wait();
   __syncthreads();
   auto in_of = [&](int e) { return e < MIXE ? s_in[e] : in_off[col[e0 + e]]; };
   auto val_of = [&](int e, int p) {
@@ -481,10 +511,8 @@ void mixpack_run(gb_ctx* ctx, const MixDev& m, const int64_t* kJ, const int64_t*
     // the planes were zeroed at allocation and entries are skipped only where they are
     // known zero: keep the previous map to know which boxes may hold stale nonzeros
     sk = *skip;
-    GB_CHECK_CUDA(cudaMemcpyAsync(sk.prev, out.mask, (size_t)out.mrows * out.kw * 4,
-                                  cudaMemcpyDeviceToDevice, ctx->stream));
   }
-  clear_mask(ctx, out);
+  map_reset(ctx, out.mask, sk.xmap ? sk.prev : nullptr, mask_bytes(out));
   const int64_t span = sk.arange ? std::max<int64_t>(sk.arange_max, 1) : m.A;
   const int64_t bx = std::min<int64_t>((span + 128 * MIXU - 1) / (128 * MIXU), 64);
   // runs of columns: long enough to mark the map rarely, short enough to fill the chip
@@ -494,9 +522,9 @@ void mixpack_run(gb_ctx* ctx, const MixDev& m, const int64_t* kJ, const int64_t*
   dim3 grid((unsigned)bx, (unsigned)m.nJ, (unsigned)((m.N + nper - 1) / nper));
   const int64_t plane = out.rows * out.Kp;
 #define GB_MIXPACK(C, E, TX)                                                                  \
-  mixpack_kernel<C, E, TX><<<grid, 128, 0, ctx->stream>>>(                                    \
-      m.A, m.N, m.xn, m.in_off, kJ, mJ, mn, m.row_ptr, m.col, m.val, (const TX*)x,            \
-      (E*)out.data, Nlog, out.Kp, out.Kh, plane, out.mask, out.kw, sk, nper)
+  launch_chained(mixpack_kernel<C, E, TX>, grid, 128, 0, ctx->stream, 1, 1, m.A, m.N, m.xn,   \
+                 m.in_off, kJ, mJ, mn, m.row_ptr, m.col, m.val, (const TX*)x, (E*)out.data,   \
+                 Nlog, out.Kp, out.Kh, plane, out.mask, out.kw, sk, nper)
 #define GB_MIXPACK_X(C, E)          \
   do {                              \
     if (x_f32) GB_MIXPACK(C, E, float); \
@@ -772,6 +800,8 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
                  "r"(2 * BN));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
+  chain_release();
+  chain_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -1059,6 +1089,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
   }
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0) tiles_done(args.counter);
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
@@ -1209,15 +1240,25 @@ void gemm_split(gb_ctx* ctx, int dtype, const Packed& A, const Packed& B, int64_
     GB_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "gemm_split: grid too large");
     gemm_bf16x3_kernel<<<grid, TC_THREADS, TC_SMEM_BYTES, ctx->stream>>>(ma, mb, a);
   } else {
-    // Tile width: 256 columns where that gives every SM a tile; narrower ones read A more
-    // often but put more SMs to work (256 x 1024 x 1024 tf32x3: 8 tiles of 256 columns 88 us,
-    // 32 of 64 columns 47 us).  The products of an element are summed in the same order.
+    // Tile width: the one whose waves take least, a k-block of w columns costing what shared
+    // memory moves for it -- 128 + w rows of 128 bytes written by the copies and read by the
+    // MMAs, at 128 bytes a clock: 256 + 2 w clocks (measured, tf32 and bf16: 395 at 64 columns,
+    // 830 at 256).  256 x 1024 x 1024 tf32x3: 8 tiles of 256 columns 88 us, 32 of 64 columns 38,
+    // 64 of 32 columns 34; 509 x 2036 x 6108 bf16x3 (128 tiles of 64 columns, one wave) takes
+    // 1.5 times as long in 256 tiles of 32.  The products of an element are summed in the same
+    // order whatever the width.
     int bn = ctx->gemm_bn;
     if (!bn) {
-      const int64_t mt = (M + TC_BM - 1) / TC_BM;
-      auto tiles = [&](int w) { return mt * ((Npk + w - 1) / w) * batch; };
-      bn = Npk <= 64 ? 64 : Npk <= 128 ? 128 : 256;
-      while (bn > 64 && tiles(bn) < std::max(1, ctx->num_sms)) bn /= 2;
+      const int64_t mt = (M + TC_BM - 1) / TC_BM, sms = std::max(1, ctx->num_sms);
+      int64_t best = INT64_MAX;
+      for (int w = 256; w >= 32; w /= 2) {
+        const int64_t tiles = mt * ((Npk + w - 1) / w) * batch;
+        const int64_t t = ((tiles + sms - 1) / sms) * (256 + 2 * w);
+        if (t < best) {
+          best = t;
+          bn = w;
+        }
+      }
     }
     if (bn != TC_BN) mb = make_map(B, bn);
     PArgs p;
@@ -1259,13 +1300,10 @@ void gemm_split(gb_ctx* ctx, int dtype, const Packed& A, const Packed& B, int64_
       const size_t mb = outmap_bytes(M, N);
       if (p.skip_zero_out) {
         uint32_t* prev = outmap + mb / 4;
-        GB_CHECK_CUDA(
-            cudaMemcpyAsync(prev, outmap, mb, cudaMemcpyDeviceToDevice, ctx->stream));
         p.prevmap = prev;
       }
-      GB_CHECK_CUDA(cudaMemsetAsync(outmap, 0, mb, ctx->stream));
+      map_reset(ctx, outmap, p.skip_zero_out ? outmap + mb / 4 : nullptr, mb);
     }
-    GB_CHECK_CUDA(cudaMemsetAsync(ctx->d_tile_counter, 0, sizeof(unsigned int), ctx->stream));
     const unsigned grid = (unsigned)std::min<int64_t>(ntiles, std::max(1, ctx->num_sms));
 #define GB_PERSISTENT(BN_, ST_, TF_)                                                          \
   do {                                                                                        \
@@ -1275,9 +1313,13 @@ void gemm_split(gb_ctx* ctx, int dtype, const Packed& A, const Packed& B, int64_
       GB_CHECK_CUDA(cudaFuncSetAttribute(gemm_bf16x3_persistent<BN_, ST_, TF_>,               \
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, SM));   \
     });                                                                                       \
-    gemm_bf16x3_persistent<BN_, ST_, TF_><<<grid, PS_THREADS, SM, ctx->stream>>>(ma, mb, p); \
+    launch_chained(gemm_bf16x3_persistent<BN_, ST_, TF_>, dim3(grid), PS_THREADS, SM,         \
+                   ctx->stream, 1, 1, ma, mb, p);                                             \
   } while (0)
-    if (bn == 64) {
+    if (bn == 32) {
+      if (tf32) GB_PERSISTENT(32, 9, true);
+      else GB_PERSISTENT(32, 9, false);
+    } else if (bn == 64) {
       if (tf32) GB_PERSISTENT(64, 8, true);
       else GB_PERSISTENT(64, 8, false);
     } else if (bn == 128) {

@@ -298,9 +298,8 @@ void goperand_init(gb_ctx* ctx, GOperand& op, const GPlan& p, int side, void* da
 template <typename E>
 __global__ void gpack_kernel(const GPackTile* __restrict__ tiles, const int32_t* __restrict__ rdense,
                              const int32_t* __restrict__ kdense, const int32_t* __restrict__ kstart,
-                             const int32_t* __restrict__ klen, const double* __restrict__ src,
-                             int64_t rs, int64_t ks, int rowfast, E* __restrict__ hi,
-                             int64_t plane, int64_t kmax, unsigned long long* nnz, int64_t klo,
+                             const int32_t* __restrict__ klen, const double* src, int64_t rs,
+                             int64_t ks, int rowfast, E* hi, int64_t plane, int64_t kmax, unsigned long long* nnz, int64_t klo,
                              int64_t khi) {
   __shared__ float t[32][33];
   __shared__ unsigned char in[32];  // column in this pack's K range
@@ -317,6 +316,8 @@ __global__ void gpack_kernel(const GPackTile* __restrict__ tiles, const int32_t*
     }
     in[tx] = inr ? 1 : 0;
   }
+  chain_release();
+  chain_wait();
   __syncthreads();
   // load with the source's contiguous index on threadIdx.x; the planes keep at most 22 bits,
   // so the value is rounded to FP32 once and split there
@@ -415,14 +416,23 @@ int64_t gpack(gb_ctx* ctx, const GPlan& p, int side, const double* src, int64_t 
   const int rowfast = (rs == 1) ? 1 : 0;
   const int64_t plane = op.rows * op.kmax;
   const unsigned grid = (unsigned)sd.ptiles.size();
-  if (op.esz == 4)
-    gpack_kernel<float><<<grid, dim3(32, 8), 0, ctx->stream>>>(
-        p.d_ptiles[side], p.d_dense[side], p.d_kdense, p.d_kstart, p.d_klen, src, rs, ks,
-        rowfast, (float*)op.data, plane, op.kmax, cnt, klo, khi);
-  else
-    gpack_kernel<__nv_bfloat16><<<grid, dim3(32, 8), 0, ctx->stream>>>(
-        p.d_ptiles[side], p.d_dense[side], p.d_kdense, p.d_kstart, p.d_klen, src, rs, ks,
-        rowfast, (__nv_bfloat16*)op.data, plane, op.kmax, cnt, klo, khi);
+  auto run = [&](auto kernel, auto* planes) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(32, 8);
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    GB_CHECK_CUDA(cudaLaunchKernelEx(
+        &cfg, kernel, (const GPackTile*)p.d_ptiles[side], (const int32_t*)p.d_dense[side],
+        (const int32_t*)p.d_kdense, (const int32_t*)p.d_kstart, (const int32_t*)p.d_klen, src, rs,
+        ks, rowfast, planes, plane, op.kmax, cnt, klo, khi));
+  };
+  if (op.esz == 4) run(gpack_kernel<float>, (float*)op.data);
+  else run(gpack_kernel<__nv_bfloat16>, (__nv_bfloat16*)op.data);
   GB_CHECK_CUDA(cudaGetLastError());
   count_launch(ctx);
   return cnt ? nnz_read(ctx, cnt) : 0;
@@ -466,9 +476,11 @@ int64_t dense_nnz(gb_ctx* ctx, const double* src, int64_t rows, int64_t cols, in
 template <typename E>
 __global__ void gmix_kernel(int64_t nJ, int64_t N, int64_t xn, const int64_t* __restrict__ in_off,
                             const int* __restrict__ row_ptr, const int* __restrict__ col,
-                            const double* __restrict__ val, const float* __restrict__ x,
-                            const GMixEntry* __restrict__ ent, E* __restrict__ hi, int64_t plane,
+                            const double* __restrict__ val, const float* x,
+                            const GMixEntry* __restrict__ ent, E* hi, int64_t plane,
                             int64_t kmax) {
+  chain_release();
+  chain_wait();
   const int J = blockIdx.y;
   const int e0 = row_ptr[J], e1 = row_ptr[J + 1];
   const int lane = threadIdx.x & 31;
@@ -527,14 +539,12 @@ void gmix_run(gb_ctx* ctx, const MixDev& m, const GMixEntry* ent, int64_t span_m
   // 8 warps per block, one (J, n) pair per warp
   dim3 grid((unsigned)std::min<int64_t>((m.N + 7) / 8, 1024), (unsigned)m.nJ);
   const int64_t plane = out.rows * out.kmax;
-  if (out.esz == 4)
-    gmix_kernel<float><<<grid, 256, 0, ctx->stream>>>(m.nJ, m.N, m.xn, m.in_off, m.row_ptr,
-                                                      m.col, m.val, t1, ent, (float*)out.data,
-                                                      plane, out.kmax);
-  else
-    gmix_kernel<__nv_bfloat16><<<grid, 256, 0, ctx->stream>>>(
-        m.nJ, m.N, m.xn, m.in_off, m.row_ptr, m.col, m.val, t1, ent,
-        (__nv_bfloat16*)out.data, plane, out.kmax);
+  auto run = [&](auto kernel, auto* planes) {
+    launch_chained(kernel, grid, 256, 0, ctx->stream, 1, 1, m.nJ, m.N, m.xn, m.in_off, m.row_ptr,
+                   m.col, m.val, t1, ent, planes, plane, out.kmax);
+  };
+  if (out.esz == 4) run(gmix_kernel<float>, (float*)out.data);
+  else run(gmix_kernel<__nv_bfloat16>, (__nv_bfloat16*)out.data);
   GB_CHECK_CUDA(cudaGetLastError());
   count_launch(ctx);
 }
@@ -728,6 +738,8 @@ __global__ void __launch_bounds__(G_THREADS, 1)
                  "r"(2 * G_BN));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
+  chain_release();
+  chain_wait();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -1067,6 +1079,7 @@ __global__ void __launch_bounds__(G_THREADS, 1)
   }
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0) tiles_done(args.counter);
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
@@ -1119,7 +1132,6 @@ void gemm_grouped(gb_ctx* ctx, const GPlan& p, const GOperand& A, const GOperand
     ctx->prof_kind_flops[1] += p.block_flops;
     GB_CHECK_CUDA(cudaEventRecord(ev0, ctx->stream));
   }
-  GB_CHECK_CUDA(cudaMemsetAsync(ctx->d_tile_counter, 0, sizeof(unsigned int), ctx->stream));
   // split-K arrival counters start at zero whatever an earlier (possibly cut short) launch
   // left in them
   if (p.ncounters > 0)
@@ -1135,7 +1147,8 @@ void gemm_grouped(gb_ctx* ctx, const GPlan& p, const GOperand& A, const GOperand
       GB_CHECK_CUDA(cudaFuncSetAttribute(gemm_grouped_kernel<ST_, TF_>,                       \
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, SM));   \
     });                                                                                       \
-    gemm_grouped_kernel<ST_, TF_><<<grid, G_THREADS, SM, ctx->stream>>>(ma, mb, a);           \
+    launch_chained(gemm_grouped_kernel<ST_, TF_>, dim3(grid), G_THREADS, SM, ctx->stream, 1,  \
+                   1, ma, mb, a);                                                             \
   } while (0)
   if (tf32) GB_GROUPED(4, true);
   else GB_GROUPED(4, false);

@@ -211,4 +211,16 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
+// ------------------------------------------------------------------ tile counter
+// counter[0] hands out tiles, counter[1] counts the CTAs that are done with it: the last one
+// leaves both at zero for the next launch (a memset in between would cost a launch and break
+// the chain of launches).  Call from one thread, after the CTA's last tile.
+__device__ __forceinline__ void tiles_done(unsigned int* counter) {
+  if (atomicAdd(&counter[1], 1u) == gridDim.x - 1) {
+    counter[0] = 0;
+    counter[1] = 0;
+    __threadfence();
+  }
+}
+
 }  // namespace gb
