@@ -49,7 +49,12 @@ constexpr int G_BN = 256;     // widest tile (TMEM: two accumulators of 256 colu
 constexpr int G_BOXN = 64;    // rows per TMA box of the B operand
 constexpr int G_KPAD = 64;    // K padding of every group (one BF16 K-block, two TF32)
 constexpr int G_RING = 4;
-constexpr int G_THREADS = 192;
+// Producer, MMA and eight epilogue warps: an accumulating tile (FP64 loads and additions) and a
+// split one (partial sums from memory) wait for memory, four warps took longer over their output
+// than the MMAs over theirs (a 8192 x 2048 x 8192 block product of short blocks, 322 units: 120 us
+// with four, 98 us with eight; 8192 x 79872 x 2048 to FP32 262 and 220 us).
+constexpr int G_EPI = 8;
+constexpr int G_THREADS = 64 + 32 * G_EPI;
 inline int64_t rup(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
 }  // namespace
 
@@ -681,7 +686,7 @@ struct GArgs {
 
 template <int STAGES>
 constexpr int grouped_smem() {
-  return STAGES * (G_BM * 128 + G_BN * 128) + 4 * 32 * 33 * 4 + 1024 + 512;
+  return STAGES * (G_BM * 128 + G_BN * 128) + G_EPI * 32 * 33 * 4 + 1024 + 512;
 }
 
 template <int STAGES, bool TF32>
@@ -696,8 +701,8 @@ __global__ void __launch_bounds__(G_THREADS, 1)
   constexpr int BOX_BYTES = G_BOXN * 128;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  float* xbuf = (float*)(smem + STAGES * STAGE_BYTES);  // [4 warps][32][33] transposes
-  uint64_t* bars = (uint64_t*)(xbuf + 4 * 32 * 33);
+  float* xbuf = (float*)(smem + STAGES * STAGE_BYTES);  // [G_EPI warps][32][33] transposes
+  uint64_t* bars = (uint64_t*)(xbuf + G_EPI * 32 * 33);
   uint64_t* full = bars;                 // [STAGES]  TMA -> MMA
   uint64_t* empty = full + STAGES;       // [STAGES]  MMA -> TMA
   uint64_t* tfull = empty + STAGES;      // [2]       MMA -> epilogue
@@ -705,7 +710,7 @@ __global__ void __launch_bounds__(G_THREADS, 1)
   uint64_t* sfull = tempty + 2;          // [RING]    scheduler -> consumers
   uint64_t* sempty = sfull + G_RING;     // [RING]    consumers -> scheduler
   uint64_t* done = sempty + G_RING;      // [1]       all MMAs retired
-  uint64_t* ep1 = done + 1;              // [1]       split tile: 4 epilogue warps wrote
+  uint64_t* ep1 = done + 1;              // [1]       split tile: the epilogue warps wrote
   uint64_t* ep2 = ep1 + 1;               // [1]       split tile: arrival counted
   int* stile = (int*)(ep2 + 1);          // [RING]
   uint32_t* tmem_slot = (uint32_t*)(stile + G_RING);
@@ -719,14 +724,14 @@ __global__ void __launch_bounds__(G_THREADS, 1)
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&tfull[b]), 1);
-      mbar_init(smem_u32(&tempty[b]), 4);
+      mbar_init(smem_u32(&tempty[b]), G_EPI);
     }
     for (int r = 0; r < G_RING; ++r) {
       mbar_init(smem_u32(&sfull[r]), 1);
-      mbar_init(smem_u32(&sempty[r]), 5);  // MMA thread + 4 epilogue warps
+      mbar_init(smem_u32(&sempty[r]), 1 + G_EPI);  // MMA thread + epilogue warps
     }
     mbar_init(smem_u32(done), 1);
-    mbar_init(smem_u32(ep1), 4);
+    mbar_init(smem_u32(ep1), G_EPI);
     mbar_init(smem_u32(ep2), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"((unsigned long long)&mapA) : "memory");
@@ -841,6 +846,7 @@ __global__ void __launch_bounds__(G_THREADS, 1)
   } else if (warp >= 2) {
     // ---------------- epilogue: TMEM -> registers -> C
     const int q = warp % 4;  // TMEM lane quarter accessible by this warp
+    const int cfirst = 32 * ((warp - 2) / 4), cstep = 32 * (G_EPI / 4);  // this warp's columns
     float* xb = xbuf + (warp - 2) * 32 * 33;
     const bool f32 = args.c_f32 != 0;
     const double alpha = args.alpha, beta = args.beta;
@@ -994,10 +1000,11 @@ __global__ void __launch_bounds__(G_THREADS, 1)
       if (T.nkb == 0) {
         // no K member in this group: C = beta * C over the tile
         if (rvalid)
-          for (int64_t n = T.n0; n < nend; ++n) {
-            const int64_t e = roff + args.coloff[n];
-            putC(e, beta != 0.0 ? beta * loadC(e) : 0.0);
-          }
+          for (int c0 = cfirst; c0 < T.nw; c0 += cstep)
+            for (int64_t n = T.n0 + c0; n < std::min<int64_t>(nend, T.n0 + c0 + 32); ++n) {
+              const int64_t e = roff + args.coloff[n];
+              putC(e, beta != 0.0 ? beta * loadC(e) : 0.0);
+            }
         continue;
       }
       const uint32_t buf = acc & 1;
@@ -1010,7 +1017,7 @@ __global__ void __launch_bounds__(G_THREADS, 1)
         // the last unit of the tile to finish adds all slots in unit order and stores
         float* own = args.partial + (size_t)(T.pslot + T.sid) * (G_BM * G_BN);
 #pragma unroll 1
-        for (int c0 = 0; c0 < T.nw; c0 += 32) {
+        for (int c0 = cfirst; c0 < T.nw; c0 += cstep) {
           uint32_t v[32];
           const uint32_t taddr = tmem + ((uint32_t)(32 * q) << 16) + buf * G_BN + (uint32_t)c0;
           TMEM_LD32(taddr, v);
@@ -1046,7 +1053,7 @@ __global__ void __launch_bounds__(G_THREADS, 1)
         if (before != T.nsplit - 1) continue;
         __threadfence();
 #pragma unroll 1
-        for (int c0 = 0; c0 < T.nw; c0 += 32) {
+        for (int c0 = cfirst; c0 < T.nw; c0 += cstep) {
           float sum[32];
 #pragma unroll
           for (int jj = 0; jj < 32; ++jj) sum[jj] = 0.0f;
@@ -1064,7 +1071,7 @@ __global__ void __launch_bounds__(G_THREADS, 1)
         continue;
       }
 #pragma unroll 1
-      for (int c0 = 0; c0 < T.nw; c0 += 32) {
+      for (int c0 = cfirst; c0 < T.nw; c0 += cstep) {
         uint32_t v[32];
         const uint32_t taddr = tmem + ((uint32_t)(32 * q) << 16) + buf * G_BN + (uint32_t)c0;
         TMEM_LD32(taddr, v);
