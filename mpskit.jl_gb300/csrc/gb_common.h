@@ -269,10 +269,14 @@ bool gemm_fp64_sliced(gb_ctx* ctx, int dtype, char opA, char opB, int64_t M, int
                       int64_t batch, const Packed* pA, const Packed* pB);
 // plain FP64 FMAs in small tiles
 struct SmallPlan {
-  int tile = 0, tm = 4, tn = 8, splits = 1;
+  int tm = 4, tn = 8, splits = 1;
   bool ok = false;
 };
-SmallPlan gemm_small_plan(int sms, int64_t M, int64_t N, int64_t K, int64_t batch);
+SmallPlan gemm_small_plan(int sms, int64_t M, int64_t N, int64_t K, int64_t batch, bool cx);
+// y = x R + L x (+ y) of a small operator in one launch; false: run them one by one
+bool gemm_small_dual(gb_ctx* ctx, int dtype, int64_t Ml, int64_t d, int64_t Nr, int64_t K1,
+                     const void* R, int64_t ldr, int64_t K2, const void* L, int64_t ldl,
+                     const void* x, bool accumulate, void* y);
 void gemm_small(cudaStream_t st, const SmallPlan& p, int dtype, char opA, char opB, int64_t M,
                 int64_t N, int64_t K, cplx alpha, const void* A, int64_t lda, int64_t sA,
                 const void* B, int64_t ldb, int64_t sB, cplx beta, bool use_beta, void* C,

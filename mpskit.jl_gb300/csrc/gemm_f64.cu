@@ -23,7 +23,7 @@
 //    3.8e-16).
 //
 //  * gemm_small_kernel -- plain FP64 FMAs in tiles small enough that a product of a few
-//    million FMAs is spread over all SMs (complex 22 x 69 x 23: 240 / 6.5 us).
+//    million FMAs is spread over all SMs (complex 22 x 69 x 23: 240 / 3.6 us).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -826,9 +826,12 @@ __global__ void __launch_bounds__(SG_THREADS, 1)
 }
 
 // ------------------------------------------------------------------ small products
-// TM x TN outputs per CTA of 128 threads, one output per thread and K group: the FP64 pipe is
-// the bound (two FMAs per clock and SM), so the tile is chosen to put work on every SM rather
-// than for operand reuse.  The K groups' partial sums are added in order.
+// TM x TN outputs per CTA of 128 threads, KG adjacent lanes share an output's contraction: the FP64
+// pipe is the bound (two FMAs per clock and SM) together with the latency of one pass through the
+// operands, so the tile is chosen to put work on every SM rather than for operand reuse, and the
+// next piece of the operands is loaded while one is used.  Two products may add up in one output
+// (y = x R + L x), one launch
+// instead of two of 4.5 us for complex 32 x 64 x 64 and 64 x 32 x 64.
 template <typename T>
 struct SmallOps;
 template <>
@@ -837,6 +840,7 @@ struct SmallOps<double> {
   static __device__ double fma_(double a, double b, double c) { return fma(a, b, c); }
   static __device__ double add(double a, double b) { return a + b; }
   static __device__ double conj(double a) { return a; }
+  static __device__ double shfl_xor(double a, int d) { return __shfl_xor_sync(0xffffffffu, a, d); }
 };
 template <>
 struct SmallOps<double2> {
@@ -846,72 +850,125 @@ struct SmallOps<double2> {
   }
   static __device__ double2 add(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
   static __device__ double2 conj(double2 a) { return make_double2(a.x, -a.y); }
+  static __device__ double2 shfl_xor(double2 a, int d) {
+    return make_double2(__shfl_xor_sync(0xffffffffu, a.x, d), __shfl_xor_sync(0xffffffffu, a.y, d));
+  }
+};
+
+template <typename T>
+struct SmallProduct {
+  const T *A, *B;
+  int64_t lda, sA, ldb, sB, K;
+  int opA, opB;  // 0 'N', 1 'T', 2 'C'
+};
+template <typename T>
+struct SmallArgs {
+  int64_t M, N, ldc, sC, kchunk;
+  T alpha, beta;
+  int use_beta, products;
+  T* C;
+  SmallProduct<T> p[2];
 };
 
 template <typename T, int TM, int TN>
-__global__ void __launch_bounds__(128)
-    gemm_small_kernel(int opA, int opB, int64_t M, int64_t N, int64_t K, T alpha, const T* A,
-                      int64_t lda, int64_t sA, const T* B, int64_t ldb, int64_t sB, T beta,
-                      int use_beta, T* C,
-                      int64_t ldc, int64_t sC, int64_t kchunk) {
+__global__ void __launch_bounds__(128) gemm_small_kernel(const __grid_constant__ SmallArgs<T> g) {
   using O = SmallOps<T>;
-  constexpr int KG = 128 / (TM * TN);  // K groups
-  constexpr int KB = 32;
-  __shared__ T As[KB][TM + 1];
-  __shared__ T Bs[KB][TN + 1];
-  __shared__ T red[KG > 1 ? (KG - 1) * TM * TN : 1];
+  constexpr int KG = 128 / (TM * TN);  // lanes of an output
+  constexpr int KB = KG > 1 ? 64 : 32;
+  constexpr int LD = KB + (KG > 1 ? KG : 1);  // rows of neighbouring outputs in other banks
+  constexpr int NA = TM * KB / 128, NB = TN * KB / 128;
+  __shared__ T As[TM * LD], Bs[TN * LD];
   const int64_t bz = blockIdx.z;
-  const int64_t k0 = kchunk ? bz * kchunk : 0, k1 = kchunk ? min(K, k0 + kchunk) : K;
-  if (!kchunk) {
-    A += bz * sA;
-    B += bz * sB;
-  }
-  C += bz * sC;
   const int64_t m0 = (int64_t)blockIdx.x * TM, n0 = (int64_t)blockIdx.y * TN;
-  const int tid = threadIdx.x, o = tid % (TM * TN), kg = tid / (TM * TN);
+  const int tid = threadIdx.x, kg = tid % KG, o = tid / KG;
   const int tm = o % TM, tn = o / TM;
-  const bool live = m0 + tm < M && n0 + tn < N;
+  const bool live = m0 + tm < g.M && n0 + tn < g.N;
+  T a[NA], b[NB];
+  // the piece of product q that starts at kb
+  auto load = [&](int q, int64_t kb, int64_t k1) {
+    const SmallProduct<T>& p = g.p[q];
+    const T *A = p.A + (g.kchunk ? 0 : bz * p.sA), *Bq = p.B + (g.kchunk ? 0 : bz * p.sB);
+#pragma unroll
+    for (int i = 0; i < NA; ++i) {
+      const int e = tid + 128 * i;
+      const int r = p.opA ? e / KB : e % TM, c = p.opA ? e % KB : e / TM;
+      a[i] = O::zero();
+      if (m0 + r < g.M && kb + c < k1)
+        a[i] = p.opA ? A[kb + c + p.lda * (m0 + r)] : A[m0 + r + p.lda * (kb + c)];
+      if (p.opA == 2) a[i] = O::conj(a[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const int e = tid + 128 * i;
+      const int c = p.opB ? e % TN : e / KB, r = p.opB ? e / TN : e % KB;
+      b[i] = O::zero();
+      if (n0 + c < g.N && kb + r < k1)
+        b[i] = p.opB ? Bq[n0 + c + p.ldb * (kb + r)] : Bq[kb + r + p.ldb * (n0 + c)];
+      if (p.opB == 2) b[i] = O::conj(b[i]);
+    }
+  };
+  int64_t kb = g.kchunk ? bz * g.kchunk : 0, k1 = g.kchunk ? min(g.p[0].K, kb + g.kchunk) : g.p[0].K;
+  int q = 0;
   T acc = O::zero();
   chain_release();
   chain_wait();
-  for (int64_t kb = k0; kb < k1; kb += KB) {
-    for (int e = tid; e < TM * KB; e += 128) {
-      const int r = opA ? e / KB : e % TM, c = opA ? e % KB : e / TM;
-      T v = O::zero();
-      if (m0 + r < M && kb + c < k1) {
-        v = opA ? A[kb + c + lda * (m0 + r)] : A[m0 + r + lda * (kb + c)];
-        if (opA == 2) v = O::conj(v);
+  load(0, kb, k1);
+  for (;;) {
+    {
+      const SmallProduct<T>& p = g.p[q];
+#pragma unroll
+      for (int i = 0; i < NA; ++i) {
+        const int e = tid + 128 * i;
+        As[p.opA ? (e / KB) * LD + e % KB : (e % TM) * LD + e / TM] = a[i];
       }
-      As[c][r] = v;
-    }
-    for (int e = tid; e < TN * KB; e += 128) {
-      const int c = opB ? e % TN : e / KB, r = opB ? e / TN : e % KB;
-      T v = O::zero();
-      if (n0 + c < N && kb + r < k1) {
-        v = opB ? B[n0 + c + ldb * (kb + r)] : B[kb + r + ldb * (n0 + c)];
-        if (opB == 2) v = O::conj(v);
+#pragma unroll
+      for (int i = 0; i < NB; ++i) {
+        const int e = tid + 128 * i;
+        Bs[p.opB ? (e % TN) * LD + e / TN : (e / KB) * LD + e % KB] = b[i];
       }
-      Bs[r][c] = v;
     }
     __syncthreads();
+    const int kn = (int)min((int64_t)KB, k1 - kb);
+    kb += KB;
+    bool more = kb < k1;
+    if (!more && q + 1 < g.products) {
+      ++q;
+      kb = 0;
+      k1 = g.p[q].K;
+      more = k1 > 0;
+    }
+    if (more) load(q, kb, k1);
     if (live) {
-      const int kn = (int)min((int64_t)KB, k1 - kb);
 #pragma unroll 4
-      for (int k = kg; k < kn; k += KG) acc = O::fma_(As[k][tm], Bs[k][tn], acc);
+      for (int k = kg; k < kn; k += KG) acc = O::fma_(As[tm * LD + k], Bs[tn * LD + k], acc);
     }
+    if (!more) break;
     __syncthreads();
   }
+  // the lanes' sums, by one warp: four from shared memory each, then across the 32 / (TM TN) lanes
+  // of an output (exchanging them in every warp is up to five times the FP64 instructions)
+  int out = o;
   if (KG > 1) {
-    if (kg > 0) red[(kg - 1) * TM * TN + o] = acc;
+    constexpr int LP = KG > 1 ? KG / 4 : 1;
+    __shared__ T red[KG > 1 ? 128 : 1];
+    red[tid] = acc;
     __syncthreads();
-    if (kg > 0) return;
-    for (int i = 0; i < KG - 1; ++i) acc = O::add(acc, red[i * TM * TN + o]);
+    if (tid >= 32) return;
+    out = tid / LP;
+    const T* part = red + out * KG + tid % LP;
+    acc = part[0];
+#pragma unroll
+    for (int i = 1; i < 4; ++i) acc = O::add(acc, part[i * LP]);
+#pragma unroll
+    for (int d = 1; d < LP; d *= 2) acc = O::add(acc, O::shfl_xor(acc, d));
+    if (tid % LP) return;
   }
-  if (!live) return;
-  const int64_t m = m0 + tm, n = n0 + tn;
-  T v = O::fma_(alpha, acc, O::zero());
-  if (use_beta) v = O::fma_(beta, C[m + ldc * n], v);
-  C[m + ldc * n] = v;
+  const int64_t m = m0 + out % TM, n = n0 + out / TM;
+  if (m >= g.M || n >= g.N) return;
+  T* C = g.C + bz * g.sC + m + g.ldc * n;
+  T v = O::fma_(g.alpha, acc, O::zero());
+  if (g.use_beta) v = O::fma_(g.beta, *C, v);
+  *C = v;
 }
 
 // ------------------------------------------------------------------ host side
@@ -1154,49 +1211,96 @@ bool gemm_fp64_sliced(gb_ctx* ctx, int dtype, char opA, char opB, int64_t M, int
   return true;
 }
 
-// launches the small-tile kernel; kchunk > 0: slice z of the grid covers kchunk contraction
-// indices and writes its partial product to C + z sC
 template <typename T>
-static void small_launch(cudaStream_t st, int tile, dim3 grid, int opA, int opB, int64_t M,
-                         int64_t N, int64_t K, T alpha, const void* A, int64_t lda, int64_t sA,
-                         const void* B, int64_t ldb, int64_t sB, T beta, int use_beta, void* C,
-                         int64_t ldc, int64_t sC, int64_t kchunk) {
-  launch_chained(tile == 0 ? gemm_small_kernel<T, 4, 8> : gemm_small_kernel<T, 16, 8>, grid, 128, 0,
-                 st, 1, 1, opA, opB, M, N, K, alpha, (const T*)A, lda, sA, (const T*)B, ldb, sB,
-                 beta, use_beta, (T*)C, ldc, sC, kchunk);
+static void small_launch(cudaStream_t st, const SmallPlan& p, const SmallArgs<T>& g,
+                         int64_t batch) {
+  void (*kernel)(SmallArgs<T>) = p.tm == 16   ? gemm_small_kernel<T, 16, 8>
+                                 : p.tn == 8  ? gemm_small_kernel<T, 4, 8>
+                                 : p.tm == 4  ? gemm_small_kernel<T, 4, 4>
+                                              : gemm_small_kernel<T, 2, 4>;
+  const dim3 grid((unsigned)((g.M + p.tm - 1) / p.tm), (unsigned)((g.N + p.tn - 1) / p.tn),
+                  (unsigned)batch);
+  launch_chained(kernel, grid, 128, 0, st, 1, 1, g);
 }
 
-SmallPlan gemm_small_plan(int sms, int64_t M, int64_t N, int64_t K, int64_t batch) {
+// The tile (and split of the contraction) whose busiest SM is done first, by a model fitted to
+// measured times: the FP64 pipe's clocks (real: two FMAs a clock), 0.6 of what a tile costs
+// besides (some 320 clocks, 500 complex, and 250 for every further 64 contraction indices; the rest
+// hides behind other tiles), 900 clocks of latency per 64 contraction indices at least.  The 16 x 8
+// tile has one lane per output and needs many tiles per SM to hide its chain of additions.  In us
+// for tiles of 16 x 8, 4 x 8, 4 x 4, 2 x 4: real 600 x 8 x 600: 8.1, 14, 24, 47; real 200 x 200 x
+// 150: 28, 23, 17, 16; complex 32 x 32 x 160: 7.2, 5.4, 5.6, 7.7; complex 128^3: -, 30, 30, 22.
+SmallPlan gemm_small_plan(int sms, int64_t M, int64_t N, int64_t K, int64_t batch, bool cx) {
+  static const int tile[4][2] = {{16, 8}, {4, 8}, {4, 4}, {2, 4}};
   SmallPlan p;
-  p.tm = 16;
-  p.tn = 8;
-  auto tiles = [&](int tm) { return ((M + tm - 1) / tm) * ((N + 7) / 8) * batch; };
-  if (tiles(16) < 4 * (int64_t)sms) {
-    p.tile = 0;
-    p.tm = 4;
-  } else {
-    p.tile = 1;
+  double best = 1e300;
+  for (const auto& t : tile) {
+    const int64_t n = ((M + t[0] - 1) / t[0]) * ((N + t[1] - 1) / t[1]) * batch;
+    int64_t sp = 1;  // splits cost the launch that adds them up
+    if (batch == 1 && K >= 512)
+      sp = std::max<int64_t>(1, std::min<int64_t>({32, K / 256, 4 * (int64_t)sms / n}));
+    const int64_t pieces = ((K + sp - 1) / sp + 63) / 64;
+    const double waves = (double)((n * sp + sms - 1) / sms);
+    const double work = t[0] * t[1] * (double)K / sp * (cx ? 2.0 : 0.5) *
+                        (t[0] == 16 && n * sp < 8 * (int64_t)sms ? 2.0 : 1.0);
+    const double rest = (cx ? 500.0 : 320.0) + 250.0 * (double)(pieces - 1);
+    const double clk =
+        std::max(waves * (work + 0.6 * rest), 900.0 * (double)pieces) + (sp > 1 ? 4000.0 : 0.0);
+    if (clk < best) {
+      best = clk;
+      p.tm = t[0];
+      p.tn = t[1];
+      p.splits = (int)sp;
+    }
   }
-  const int64_t t = tiles(p.tm);
-  p.ok = (M + p.tm - 1) / p.tm < (int64_t)1 << 31 && (N + 7) / 8 <= 65535 && batch <= 65535;
-  p.splits = 1;
-  if (batch == 1 && t * 2 <= sms && K >= 128)
-    p.splits = (int)std::max<int64_t>(1, std::min<int64_t>({2 * sms / t, K / 64, 32}));
+  p.ok = (M + p.tm - 1) / p.tm < (int64_t)1 << 31 && (N + p.tn - 1) / p.tn <= 65535 &&
+         batch <= 65535;
   return p;
+}
+
+template <typename T>
+static SmallProduct<T> small_product(char opA, char opB, int64_t K, const void* A, int64_t lda,
+                                     int64_t sA, const void* B, int64_t ldb, int64_t sB) {
+  return SmallProduct<T>{(const T*)A, (const T*)B, lda, sA, ldb, sB, K, opcode(opA), opcode(opB)};
 }
 
 void gemm_small(cudaStream_t st, const SmallPlan& p, int dtype, char opA, char opB, int64_t M,
                 int64_t N, int64_t K, cplx alpha, const void* A, int64_t lda, int64_t sA,
                 const void* B, int64_t ldb, int64_t sB, cplx beta, bool use_beta, void* C,
                 int64_t ldc, int64_t sC, int64_t batch, int64_t kchunk) {
-  dim3 grid((unsigned)((M + p.tm - 1) / p.tm), (unsigned)((N + p.tn - 1) / p.tn), (unsigned)batch);
-  if (is_cplx(dtype))
-    small_launch<double2>(st, p.tile, grid, opcode(opA), opcode(opB), M, N, K,
-                          make_double2(alpha.re, alpha.im), A, lda, sA, B, ldb, sB,
-                          make_double2(beta.re, beta.im), use_beta, C, ldc, sC, kchunk);
-  else
-    small_launch<double>(st, p.tile, grid, opcode(opA), opcode(opB), M, N, K, alpha.re, A, lda, sA,
-                         B, ldb, sB, beta.re, use_beta, C, ldc, sC, kchunk);
+  auto run = [&](auto al, auto be) {
+    using T = decltype(al);
+    SmallArgs<T> g{M, N, ldc, sC, kchunk, al, be, use_beta ? 1 : 0, 1, (T*)C, {}};
+    g.p[0] = small_product<T>(opA, opB, K, A, lda, sA, B, ldb, sB);
+    small_launch(st, p, g, batch);
+  };
+  if (is_cplx(dtype)) run(make_double2(alpha.re, alpha.im), make_double2(beta.re, beta.im));
+  else run(alpha.re, beta.re);
+}
+
+// y[l, s, r] = sum_k x[l, k] R[k, (s, r)] + sum_k L[(l, s), k] x[k, r] (+ y): one launch where both
+// products are small.  x is contiguous: Ml x K1 for the first product, K2 x Nr for the second.
+bool gemm_small_dual(gb_ctx* ctx, int dtype, int64_t Ml, int64_t d, int64_t Nr, int64_t K1,
+                     const void* R, int64_t ldr, int64_t K2, const void* L, int64_t ldl,
+                     const void* x, bool accumulate, void* y) {
+  const bool cx = is_cplx(dtype);
+  const double mac = (double)Ml * (double)d * (double)Nr * (cx ? 4 : 1);
+  // each by itself would be a small product
+  if (mac * (double)std::max(K1, K2) >= F64_SLICED_MIN_MAC_CUT) return false;
+  const SmallPlan p = gemm_small_plan(std::max(1, ctx->num_sms), Ml, Nr, K1 + K2, d, cx);
+  if (!p.ok) return false;
+  auto run = [&](auto one) {
+    using T = decltype(one);
+    SmallArgs<T> g{Ml, Nr, Ml * d, Ml, 0, one, one, accumulate ? 1 : 0, 2, (T*)y, {}};
+    // column (s, r) of R is its column s + d r; row (l, s) of L its row l + Ml s
+    g.p[0] = small_product<T>('N', 'N', K1, x, Ml, 0, R, ldr * d, ldr);
+    g.p[1] = small_product<T>('N', 'N', K2, L, ldl, Ml, x, K2, 0);
+    small_launch(ctx->stream, p, g, d);
+  };
+  if (cx) run(make_double2(1.0, 0.0));
+  else run(1.0);
+  count_launch(ctx);
+  return true;
 }
 
 }  // namespace gb

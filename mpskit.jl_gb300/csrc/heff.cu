@@ -1973,7 +1973,26 @@ void heff_apply_raw(gb_heff* h, const void* x, void* y) {
   const bool fused_t2 = h->prec != GB_PREC_FP64 && h->t2p_ready;
   if (!fused_t2 && h->t2_elems && !h->t2)
     h->t2 = dalloc(h, (size_t)h->t2_elems * elem_size(h->dtype));
-  for (const Step& s : h->steps) {
+  // a product with x on the left and the next one with x on the right, both into y
+  auto pair_of = [&](size_t i) {
+    if (h->prec != GB_PREC_FP64 || i + 1 >= h->steps.size()) return false;
+    const Step &p = h->steps[i], &q = h->steps[i + 1];
+    return p.is_gemm && q.is_gemm && p.srcA == S_X && p.srcB == S_CONST && p.dst == S_Y &&
+           q.srcA == S_CONST && q.srcB == S_X && q.dst == S_Y && q.accumulate && p.opA == 'N' &&
+           p.opB == 'N' && q.opA == 'N' && q.opB == 'N' && p.lda == p.M && p.ldc == p.M &&
+           q.ldb == q.K && q.ldc == q.M && q.M % p.M == 0 && p.N == q.N * (q.M / p.M) &&
+           p.M * p.K == q.K * q.N;
+  };
+  for (size_t i = 0; i < h->steps.size(); ++i) {
+    const Step& s = h->steps[i];
+    if (pair_of(i)) {
+      const Step& q = h->steps[i + 1];
+      if (gemm_small_dual(ctx, h->dtype, s.M, q.M / s.M, q.N, s.K, s.cB, s.ldb, q.K, q.cA, q.lda, x,
+                          s.accumulate, y)) {
+        ++i;
+        continue;
+      }
+    }
     if (s.is_gemm) {
       void* C = (void*)ptr(s.dst, nullptr);
       double beta = s.accumulate ? 1.0 : 0.0;

@@ -500,7 +500,8 @@ void gemm_fp64(gb_ctx* ctx, int dtype, char opA, char opB, int64_t M, int64_t N,
     return;
   const double mac = (double)M * (double)N * (double)K * (double)batch * (is_cplx(dtype) ? 4 : 1);
   if (mac < F64_SLICED_MIN_MAC) {
-    const SmallPlan p = gemm_small_plan(std::max(1, ctx->num_sms), M, N, K, batch);
+    const SmallPlan p = gemm_small_plan(std::max(1, ctx->num_sms), M, N, K, batch,
+                                        is_cplx(dtype));
     if (p.ok) {
       if (p.splits > 1) {
         const int64_t kchunk = (K + p.splits - 1) / p.splits;

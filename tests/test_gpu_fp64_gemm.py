@@ -175,3 +175,28 @@ def test_chained_launches(ctx, h, K):
         return a.numpy()
 
     assert np.array_equal(run(True), run(False))
+
+
+@pytest.mark.parametrize("cx", [False, True])
+@pytest.mark.parametrize("Dl,Dr", [(1, 1), (3, 5), (7, 64), (65, 33), (90, 91), (160, 170)])
+def test_left_and_right_products_together(ctx, Dl, Dr, cx):
+    """A one-site operator whose products with the two environments share a launch (all but the
+    largest), every tile of the small products and its remainders among them.  Each product errs
+    by at most 4e-16 sqrt(K) of its terms' norm."""
+    rng = np.random.default_rng(Dl + Dr)
+    dt = np.complex128 if cx else np.float64
+    H = mpsgb.heisenberg_XXX(6, dtype=dt)
+    W = np.asarray(H.W[2])
+    GL, GR = _rand(rng, (Dl, W.shape[0], Dl), cx, 0), _rand(rng, (Dr, W.shape[3], Dr), cx, 0)
+    GL[:, 0, :] = np.eye(Dl)  # the channels "not started" and "finished"
+    GR[:, -1, :] = np.eye(Dr)
+    x = _rand(rng, (Dl, 2, Dr), cx, 0)
+    dev = lambda k, a: mpsgb.DeviceTensor.from_numpy(ctx, k, a)
+    op = mpsgb.DerivativeOperator(ctx, mpsgb._lib.GB_HEFF_AC, dev("gl", GL),
+                                  H.device(ctx, dt)[2], None, dev("gr", GR),
+                                  mpsgb.GB300Backend("fp64"))
+    ref = np.einsum("bwk,kta->bwta", GL, x, optimize=True)
+    ref = np.einsum("bwta,wstv->bsva", ref, W, optimize=True)
+    scale = np.linalg.norm(np.einsum("bsva,avc->bsc", np.abs(ref), np.abs(GR), optimize=True))
+    ref = np.einsum("bsva,avc->bsc", ref, GR, optimize=True)
+    assert np.linalg.norm(op(dev("mps", x)).numpy() - ref) <= 4e-15 * scale
