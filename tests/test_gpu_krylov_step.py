@@ -33,10 +33,11 @@ def _orthogonalize(ctx, V, w):
 
 # pieces of 64 entries on 152 multiprocessors: one, two and all blocks, one entry more; pieces
 # in shared memory and too long for it; one to five vectors (one barrier or two), the longest
-# list and one past it
+# list and one past it; the longest vectors of a single cluster and one entry more
 @pytest.mark.parametrize("cx", [False, True])
 @pytest.mark.parametrize("n,k", [(3, 2), (64, 5), (65, 9), (130, 4), (9728, 3), (9729, 30),
-                                 (40000, 8), (400001, 13), (900000, 7), (700, 128), (700, 129)])
+                                 (40000, 8), (400001, 13), (900000, 7), (700, 128), (700, 129),
+                                 (2048, 15), (2049, 15), (4096, 20), (4097, 3)])
 def test_decomposition(ctx, n, k, cx):
     rng = np.random.default_rng(n + k)
     V = rng.standard_normal((n, k)) + (1j * rng.standard_normal((n, k)) if cx else 0)
