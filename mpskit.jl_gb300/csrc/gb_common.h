@@ -273,6 +273,9 @@ struct SmallPlan {
   bool ok = false;
 };
 SmallPlan gemm_small_plan(int sms, int64_t M, int64_t N, int64_t K, int64_t batch, bool cx);
+// digits of x as the left operand (R1 x K1) of one product and the right one (K2 x R2) of another
+bool slice_both(gb_ctx* ctx, int dtype, const void* x, int64_t R1, int64_t K1, int64_t R2,
+                int64_t K2, Packed& a, Packed& b);
 // y = x R + L x (+ y) of a small operator in one launch; false: run them one by one
 bool gemm_small_dual(gb_ctx* ctx, int dtype, int64_t Ml, int64_t d, int64_t Nr, int64_t K1,
                      const void* R, int64_t ldr, int64_t K2, const void* L, int64_t ldl,

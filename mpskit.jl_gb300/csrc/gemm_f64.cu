@@ -1038,8 +1038,8 @@ static void slice_launch(gb_ctx* ctx, SliceArgs a, SliceArgs b) {
     s.nblk = (int)n;
     return n;
   };
-  // both operands have the same contraction
-  const int64_t kbs = a.Kh / 64, sms = std::max(1, ctx->num_sms);
+  const int64_t ka = a.Kh / 64, kb = b.src ? b.Kh / 64 : 0, kbs = std::max(ka, kb);
+  const int64_t sms = std::max(1, ctx->num_sms);
   const int64_t rows = blocks(a, 1) + blocks(b, 1);
   // One launch unless a cluster's CTAs would each walk many k-blocks while SMs stand idle (real
   // 128 x 2000: 12.7 us in one launch, 14.5 in two; 128 x 4000: 19 both; 128 x 8000: 30 and 23;
@@ -1063,8 +1063,8 @@ static void slice_launch(gb_ctx* ctx, SliceArgs a, SliceArgs b) {
   blocks(a, a.nchunk);
   blocks(b, b.nchunk);
   launch_chained(slice_max_kernel, dim3(a.nblk + b.nblk), 256, 0, ctx->stream, 1, 1, a, b);
-  blocks(a, kbs);
-  blocks(b, kbs);
+  blocks(a, ka);
+  blocks(b, kb);
   launch_chained(slice_kernel, dim3(a.nblk + b.nblk), 256, 0, ctx->stream, 1, 1, a, b);
   count_launch_n(ctx, 2);
 }
@@ -1075,6 +1075,26 @@ void slice_operand(gb_ctx* ctx, int dtype, int role, char op, int64_t R, int64_t
   SliceArgs a = slice_args(ctx, dtype, role, op, R, K, src, ld, stride, batch, dst, out);
   SliceArgs none{};
   slice_launch(ctx, a, none);
+}
+
+// x as the left operand of one product (R1 x K1) and the right operand of another (K2 x R2), cut in
+// one launch; both stay in the context's scratch.  False when that does not fit.
+bool slice_both(gb_ctx* ctx, int dtype, const void* x, int64_t R1, int64_t K1, int64_t R2,
+                int64_t K2, Packed& a, Packed& b) {
+  const bool cx = is_cplx(dtype);
+  void *da = nullptr, *db = nullptr;
+  try {
+    da = scratch(ctx, SLOT_PACK_A, sliced_bytes(R1, K1, cx, PACK_AS_A, 1));
+    db = scratch(ctx, SLOT_PACK_B, sliced_bytes(R2, K2, cx, PACK_AS_B, 1));
+  } catch (const Error& e) {
+    if (e.code != GB_ERR_OOM) throw;
+    cudaGetLastError();
+    return false;
+  }
+  const SliceArgs aa = slice_args(ctx, dtype, PACK_AS_A, 'N', R1, K1, x, R1, 0, 1, da, a);
+  const SliceArgs ab = slice_args(ctx, dtype, PACK_AS_B, 'N', R2, K2, x, K2, 0, 1, db, b);
+  slice_launch(ctx, aa, ab);
+  return true;
 }
 
 bool gemm_sliced_wanted(gb_ctx* ctx, int dtype, int64_t M, int64_t N, int64_t K, int64_t batch,
