@@ -299,13 +299,16 @@ void pack_operand(gb_ctx* ctx, int dtype, int role, char op, int64_t R, int64_t 
 // k = a + kJ[J] (contraction index) and m = mJ[J] + n*mn (output column index).
 //
 // A block takes one output row J and a run of columns n, a warp 128 consecutive entries of one
-// column at a time.  Bound by the instructions around an entry, not by the traffic (4 B read per
-// entry and input, 4 B written in BF16), so one test of the written-region map, one reduction of
-// the nonzero flags and at most one atomic serve the 128 entries, and a row of one input with a
-// coefficient that FP32 holds stays in FP32 (FP64 sums cost 16 clocks per warp instruction and
-// SM).  12.4 M entries, one input each: 129 us with 32 entries per test and FP64 products, 80 us.
+// column at a time.  Bound by the instructions around an entry and the latency of a column's map
+// word and values, not by the traffic (4 B read per entry and input, 4 B written in BF16).  So one
+// test of the written-region map, one reduction of the nonzero flags and at most one atomic serve
+// the 128 entries, and a row of one input -- most rows -- keeps its run from column to column, has
+// four columns in flight and multiplies in FP32 (FP64 sums cost 16 clocks per warp instruction and
+// SM).  12.4 M entries, one input each: 129 us with 32 entries per test and FP64 products, 80 us
+// with 128 entries, 36 us with columns in flight and FP32 products (38 with two columns).
 constexpr int MIXE = 64;  // entries of a row kept in shared memory
 constexpr int MIXU = 4;   // entries of a column per thread
+constexpr int MIXN = 4;   // columns in flight (single inputs)
 template <bool CPLX, typename E, typename TX>
 __global__ void __launch_bounds__(128)
     mixpack_kernel(int64_t A, int64_t N, int64_t xn, const int64_t* __restrict__ in_off,
@@ -343,11 +346,87 @@ __global__ void __launch_bounds__(128)
   };
   const int64_t k0J = kJ[J], m0J = mJ[J];
   const int64_t n0 = (int64_t)blockIdx.z * nper, n1 = min(N, n0 + nper);
-  // One input with a coefficient that FP32 holds: its product with an FP32 value, exact in FP64,
-  // rounds to the FP32 product
+  // One FP32 input: the product with the coefficient c = c32 + cl, rounded to FP32, from FP32
+  // operations (product, its exact error and cl's share), as close to c x as the FP64 product
+  // rounded to FP32 and the same value but for ties within 2^-48.  Coefficients near the ends of
+  // FP32's range, and complex ones, take the sum in FP64.
   const float c32 = ne == 1 ? to_float(val_of(0, 0)) : 0.f;
+  const float cl = ne == 1 ? to_float(val_of(0, 0) - to_double(c32)) : 0.f;
+  const int cexp = (int)(__float_as_uint(c32) >> 23 & 0xffu);
   const bool single = std::is_same<TX, float>::value && ne == 1 &&
-                      to_double(c32) == val_of(0, 0) && (!CPLX || val_of(0, CPLX) == 0.0);
+                      (!CPLX || val_of(0, CPLX) == 0.0) &&
+                      ((unsigned)(cexp - 28) < 200u || val_of(0, 0) == 0.0);
+  auto product = [&](float x) {
+    const float p = c32 * x;
+    return p + fmaf(cl, x, fmaf(c32, x, -p));
+  };
+  if (!CPLX && single && !sk.arange) {
+    // a warp's run stays the same from column to column
+    const int64_t ro = sk.xmap ? s_roff[0] : 0, co = sk.xmap ? s_coff[0] : 0;
+    for (int64_t a0 = ((int64_t)blockIdx.x * 4 + threadIdx.x / 32) * (32 * MIXU); a0 < A;
+         a0 += (int64_t)gridDim.x * (128 * MIXU)) {
+      const int left = (int)min(A - a0 - lane, (int64_t)(32 * MIXU));
+      const int64_t k = k0J + a0, kfirst = k / BK;
+      const int koff = (int)(k - kfirst * BK) + lane;
+      const int64_t q0 = ((a0 + ro) >> 7) * sk.onc;
+      const int64_t q1 = ((min(a0 + 32 * MIXU - 1, A - 1) + ro) >> 7) * sk.onc;
+      int64_t last = -1;
+      uint32_t seen = 0;  // k-blocks marked in the row tile `last`
+      for (int64_t n = n0; n < n1; n += MIXN) {
+        // the map's words, then the values, of MIXN columns in flight
+        bool hit[MIXN];
+#pragma unroll
+        for (int j = 0; j < MIXN; ++j) {
+          hit[j] = n + j < n1;
+          if (sk.xmap && hit[j]) {
+            const int64_t cb = (co + (n + j) * sk.xnM) >> 7, p0 = q0 + cb, p1 = q1 + cb;
+            hit[j] = ((sk.xmap[p0 >> 5] >> (p0 & 31)) | (sk.xmap[p1 >> 5] >> (p1 & 31))) & 1u;
+          }
+        }
+        float v[MIXN][MIXU];
+#pragma unroll
+        for (int j = 0; j < MIXN; ++j) {
+          const float* xp = (const float*)x + in_of(0) + (n + j) * xn + a0 + lane;
+#pragma unroll
+          for (int u = 0; u < MIXU; ++u) v[j][u] = hit[j] && 32 * u < left ? xp[32 * u] : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < MIXN; ++j) {
+          if (n + j >= n1) break;
+          const int64_t m = m0J + (n + j) * mn;
+          if (m / MASK_ROWS != last) {
+            last = m / MASK_ROWS;
+            seen = 0;
+          }
+          if (!hit[j]) {
+            for (int u = 0; u < MIXU && 32 * u < left; ++u) {
+              const int64_t kb = kfirst + (koff + 32 * u) / BK;
+              if ((sk.prev[last * kw + kb / 32] >> (kb % 32)) & 1u) put(m, k + lane + 32 * u, 0.0);
+            }
+            continue;
+          }
+          E* h0 = hi + m * Kp + k + lane;
+          uint32_t want = 0;
+#pragma unroll
+          for (int u = 0; u < MIXU; ++u) {
+            if (32 * u >= left) continue;
+            const float w = product(v[j][u]);
+            split_put_f(h0, h0 + plane, 32 * u, w);
+            if (__float_as_uint(w) << 1) want |= 1u << ((koff + 32 * u) / BK);
+          }
+          want = __reduce_or_sync(0xffffffffu, want) & ~seen;
+          if (want) {
+            seen |= want;
+            if ((want >> lane) & 1u) {
+              const int64_t kb = kfirst + lane;
+              atomicOr(&mask[last * kw + kb / 32], 1u << (kb % 32));
+            }
+          }
+        }
+      }
+    }
+    return;
+  }
   // k-blocks already marked in the row tile that the last column fell into, counted from the
   // first one of the warp's run
   int64_t tile = -1, tile_im = -1;
@@ -419,8 +498,8 @@ __global__ void __launch_bounds__(128)
         }
 #pragma unroll
         for (int u = 0; u < MIXU; ++u) {
-          re[u] *= c32;
-          if (CPLX) im[u] *= c32;
+          re[u] = product(re[u]);
+          if (CPLX) im[u] = product(im[u]);
         }
       } else {
         double dre[MIXU], dim[MIXU];

@@ -37,3 +37,49 @@ def test_environment_step(ctx, Dl, Dr, cx):
     ref = np.einsum("bwta,wstv->bsva", ref, W, optimize=True)
     ref = np.einsum("bsva,bsc->cva", ref, A.conj(), optimize=True)
     assert np.linalg.norm(got - ref) <= 3e-15 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("prec", ["bf16x3", "tf32x3"])
+@pytest.mark.parametrize("cx", [False, True])
+@pytest.mark.parametrize("Dl,Dr", [(5, 3), (37, 41), (131, 128), (300, 257)])
+def test_chain_mix_in_planes(ctx, Dl, Dr, cx, prec):
+    """The mix that writes split planes: rows of one input with a coefficient that FP32 does not
+    hold, rows of several, columns around the numbers in flight.  A plane pair keeps 16 (bf16) or
+    22 bits (tf32: at least the 16) of each of four roundings, and the product of the low planes
+    is dropped: 4 2^-17 + 2 2^-16 = 2^-14 of the result at most."""
+    rng = np.random.default_rng(Dl * Dr)
+    dt = np.complex128 if cx else np.float64
+    n = 4
+    W = np.zeros((n, 2, 2, n), dtype=dt)
+    sz, sp = np.diag([0.5, -0.5]), np.array([[0.0, 1.0], [0.0, 0.0]])
+    W[0, :, :, 0] = W[-1, :, :, -1] = np.eye(2)
+    for c, o in ((1, sz), (2, sp + sp.T)):  # exponentially decaying couplings
+        W[0, :, :, c] = rng.uniform(0.5, 1.0) * o
+        W[c, :, :, c] = rng.uniform(0.1, 0.9) * np.eye(2)
+        W[c, :, :, -1] = o
+    W[1, :, :, 2] = 0.3 * sz  # an output of two inputs
+    W[0, :, :, -1] = 0.7 * sp + 0.7 * sp.T
+
+    def env(D):
+        g = rng.standard_normal((D, n, D)) / np.sqrt(D)
+        return (g + 1j * rng.standard_normal((D, n, D)) / np.sqrt(D)).astype(dt) if cx else g
+
+    GL, GR = env(Dl), env(Dr)
+    GL[:, 0, :] = np.eye(Dl)
+    GR[:, -1, :] = np.eye(Dr)
+    x = rng.standard_normal((Dl, 2, Dr, 2)).astype(dt)
+    dev = lambda k, a: mpsgb.DeviceTensor.from_numpy(ctx, k, a)
+    w = dev("mpo", W)
+
+    def apply(p, times):
+        op = mpsgb.DerivativeOperator(ctx, mpsgb._lib.GB_HEFF_AC2, dev("gl", GL), w, w,
+                                      dev("gr", GR), mpsgb.GB300Backend(p))
+        xd = dev("ac2", x)
+        for _ in range(times):
+            y = op(xd)
+        return y.numpy()
+
+    ref = apply("fp64", 1)
+    got = apply(prec, 1)
+    assert np.linalg.norm(got - ref) <= 2.0 ** -14 * np.linalg.norm(ref)
+    assert np.array_equal(apply(prec, 3), got)  # over planes and maps of an earlier apply
