@@ -273,9 +273,12 @@ struct SmallPlan {
   bool ok = false;
 };
 SmallPlan gemm_small_plan(int sms, int64_t M, int64_t N, int64_t K, int64_t batch, bool cx);
-// digits of x as the left operand (R1 x K1) of one product and the right one (K2 x R2) of another
-bool slice_both(gb_ctx* ctx, int dtype, const void* x, int64_t R1, int64_t K1, int64_t R2,
-                int64_t K2, Packed& a, Packed& b);
+// y = x R + L x (+ y) of operators whose constants are cut into digits (R, Lp): x is M1 x K1 on the
+// left of R and K2 x N2 on the right of L.  False (nothing done) when the digits do not fit.
+bool gemm_sliced_pair(gb_ctx* ctx, int dtype, const void* x, int64_t M1, int64_t N1, int64_t K1,
+                      const Packed& R, const void* Rsrc, int64_t ldr, int64_t M2, int64_t N2,
+                      int64_t K2, const Packed& Lp, const void* Lsrc, int64_t ldl, bool accumulate,
+                      void* y);
 // y = x R + L x (+ y) of a small operator in one launch; false: run them one by one
 bool gemm_small_dual(gb_ctx* ctx, int dtype, int64_t Ml, int64_t d, int64_t Nr, int64_t K1,
                      const void* R, int64_t ldr, int64_t K2, const void* L, int64_t ldl,

@@ -281,7 +281,8 @@ __device__ __forceinline__ void slice_flags(const SliceArgs& p, int z, int64_t r
 // is one launch: complex 256 x 256, 16.5 us as
 // a launch for the maxima and one for the digits, 8.8 us here.
 template <int RB>
-__global__ void __launch_bounds__(256) slice_cluster_kernel(SliceArgs a, SliceArgs b, int cs) {
+__global__ void __launch_bounds__(256) slice_cluster_kernel(SliceArgs a, SliceArgs b, int cs,
+                                                            double* zero, int64_t nzero) {
   __shared__ SliceSmem<RB> s;
   const int rank = (int)blockIdx.x % cs;  // clusters are runs of cs CTAs
   int blk = (int)blockIdx.x / cs;
@@ -296,6 +297,8 @@ __global__ void __launch_bounds__(256) slice_cluster_kernel(SliceArgs a, SliceAr
   if (tid < RB) s.e[tid] = 0;
   chain_release();
   chain_wait();
+  for (int64_t i = blockIdx.x * (int64_t)256 + tid; i < nzero; i += (int64_t)gridDim.x * 256)
+    zero[i] = 0.0;
   const int mine = rank < kbs ? (kbs - rank + cs - 1) / cs : 0;
   int nz = 0;
   for (int i = 0; i < mine; ++i) {
@@ -398,6 +401,14 @@ struct SGArgs {
   const double *A, *B;
   int64_t lda, sA, ldb, sB, K;
   int opA, opB;      // 0 'N', 1 'T', 2 'C'
+  int add;           // C += by atomics: two products of one launch share an output
+};
+// one product, or two whose blocks along x follow one another
+template <int PRODUCTS>
+struct SGLaunch {
+  CUtensorMap a[PRODUCTS], b[PRODUCTS];
+  SGArgs g[PRODUCTS];
+  int first;         // blocks of the first
 };
 
 // products of one digit of A with n digits of B (adjacent rows, adjacent accumulators)
@@ -494,10 +505,13 @@ __device__ __noinline__ void plain_entry(const SGArgs& g, int z, int64_t m, int6
 // densely) are left out.  A tile grid under half the chip splits the k-blocks over the CTAs of
 // a cluster; each then adds the integer sums of all of them for its share of the columns
 // (through distributed shared memory: exact, so the result does not depend on the split).
-template <int BN>
+template <int BN, int PRODUCTS>
 __global__ void __launch_bounds__(SG_THREADS, 1)
-    gemm_sliced_kernel(const __grid_constant__ CUtensorMap mapA,
-                       const __grid_constant__ CUtensorMap mapB, SGArgs g) {
+    gemm_sliced_kernel(const __grid_constant__ SGLaunch<PRODUCTS> L) {
+  const int which = PRODUCTS > 1 && (int)blockIdx.x >= L.first ? 1 : 0;
+  const int block = (int)blockIdx.x - (which ? L.first : 0);
+  const SGArgs& g = L.g[which];
+  const CUtensorMap &mapA = L.a[which], &mapB = L.b[which];
   using S = SGShape<BN>;
   constexpr int HC = BN / 2;  // columns per epilogue thread
   extern __shared__ uint8_t smem_raw[];
@@ -516,7 +530,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1)
   int* sea = seb + BN;               // [128] row exponents
 
   const int warp = warp_index(), lane = threadIdx.x % 32;
-  const int mi = blockIdx.x % g.mt, rest = blockIdx.x / g.mt;
+  const int mi = block % g.mt, rest = block / g.mt;
   const int ni = rest % g.nt, z = rest / g.nt;
   const int split = blockIdx.y;
   const int64_t m0 = (int64_t)mi * 128, n0 = (int64_t)ni * BN;
@@ -764,6 +778,10 @@ __global__ void __launch_bounds__(SG_THREADS, 1)
       // executed and selected, and each costs as much as the conversion
       uint32_t slow = 0;  // entries that the conversion does not cover
       auto update = [&](auto form, double* p, double v) {
+        if constexpr (form.value == 3) {
+          atomicAdd(p, v);
+          return;
+        }
         if constexpr (form.value == 1) v += *p;
         if constexpr (form.value == 2) {
           v *= g.alpha;
@@ -807,7 +825,8 @@ __global__ void __launch_bounds__(SG_THREADS, 1)
           update(form, C + step * j, v);
         }
       };
-      if (g.alpha == 1.0 && g.beta == 0.0) store(std::integral_constant<int, 0>{});
+      if (g.add) store(std::integral_constant<int, 3>{});
+      else if (g.alpha == 1.0 && g.beta == 0.0) store(std::integral_constant<int, 0>{});
       else if (g.alpha == 1.0 && g.beta == 1.0) store(std::integral_constant<int, 1>{});
       else store(std::integral_constant<int, 2>{});
     }
@@ -1031,7 +1050,9 @@ static SliceArgs slice_args(gb_ctx* ctx, int dtype, int role, char op, int64_t R
   return a;
 }
 
-static void slice_launch(gb_ctx* ctx, SliceArgs a, SliceArgs b) {
+// also sets `zero` to zero, the output that products of the cut operands add up in
+static void slice_launch(gb_ctx* ctx, SliceArgs a, SliceArgs b, double* zero = nullptr,
+                         int64_t nzero = 0) {
   auto blocks = [](SliceArgs& s, int64_t per) {
     const int64_t n = s.src ? (int64_t)s.rblk * s.batch * per : 0;
     GB_REQUIRE(n < (int64_t)1 << 30, "gemm: operand too large to slice");
@@ -1056,10 +1077,12 @@ static void slice_launch(gb_ctx* ctx, SliceArgs a, SliceArgs b) {
     GB_REQUIRE((int64_t)(a.nblk + b.nblk) * cs < (int64_t)1 << 31,
                "gemm: operand too large to slice");
     launch_chained(small ? slice_cluster_kernel<8> : slice_cluster_kernel<32>,
-                   dim3((unsigned)(a.nblk + b.nblk) * cs), 256, 0, ctx->stream, cs, 1, a, b, cs);
+                   dim3((unsigned)(a.nblk + b.nblk) * cs), 256, 0, ctx->stream, cs, 1, a, b, cs,
+                   zero, nzero);
     count_launch(ctx);
     return;
   }
+  if (nzero) fill_zero(ctx, zero, (size_t)nzero * 8);
   blocks(a, a.nchunk);
   blocks(b, b.nchunk);
   launch_chained(slice_max_kernel, dim3(a.nblk + b.nblk), 256, 0, ctx->stream, 1, 1, a, b);
@@ -1079,8 +1102,8 @@ void slice_operand(gb_ctx* ctx, int dtype, int role, char op, int64_t R, int64_t
 
 // x as the left operand of one product (R1 x K1) and the right operand of another (K2 x R2), cut in
 // one launch; both stay in the context's scratch.  False when that does not fit.
-bool slice_both(gb_ctx* ctx, int dtype, const void* x, int64_t R1, int64_t K1, int64_t R2,
-                int64_t K2, Packed& a, Packed& b) {
+static bool slice_both(gb_ctx* ctx, int dtype, const void* x, int64_t R1, int64_t K1, int64_t R2,
+                int64_t K2, Packed& a, Packed& b, double* zero, int64_t nzero) {
   const bool cx = is_cplx(dtype);
   void *da = nullptr, *db = nullptr;
   try {
@@ -1093,7 +1116,7 @@ bool slice_both(gb_ctx* ctx, int dtype, const void* x, int64_t R1, int64_t K1, i
   }
   const SliceArgs aa = slice_args(ctx, dtype, PACK_AS_A, 'N', R1, K1, x, R1, 0, 1, da, a);
   const SliceArgs ab = slice_args(ctx, dtype, PACK_AS_B, 'N', R2, K2, x, K2, 0, 1, db, b);
-  slice_launch(ctx, aa, ab);
+  slice_launch(ctx, aa, ab, zero, nzero);
   return true;
 }
 
@@ -1107,20 +1130,28 @@ bool gemm_sliced_wanted(gb_ctx* ctx, int dtype, int64_t M, int64_t N, int64_t K,
 
 static int opcode(char op) { return op == 'N' ? 0 : op == 'T' ? 1 : 2; }
 
-template <int BN>
-static void launch_sliced(gb_ctx* ctx, const Packed& a, const Packed& b, SGArgs& g, int64_t batch) {
+// one product, or two that add up in one output
+template <int BN, int PRODUCTS>
+static void launch_sliced(gb_ctx* ctx, const Packed* const* a, const Packed* const* b,
+                          const SGArgs* g, int64_t batch) {
   using S = SGShape<BN>;
   static std::once_flag once;  // contexts may launch from several host threads
   std::call_once(once, [] {
-    GB_CHECK_CUDA(cudaFuncSetAttribute(gemm_sliced_kernel<BN>,
+    GB_CHECK_CUDA(cudaFuncSetAttribute(gemm_sliced_kernel<BN, PRODUCTS>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM));
   });
-  const CUtensorMap ma = make_slice_map(a.data, a.Kp, a.rows, a.batch * SL, 128, 1);
-  const CUtensorMap mb = make_slice_map(b.data, b.Kp, b.rows, b.batch * SL, BN, SL);
-  const int64_t tiles = (int64_t)g.mt * g.nt * batch;
-  GB_REQUIRE(tiles < (int64_t)1 << 31, "gemm: too many tiles");
-  launch_chained(gemm_sliced_kernel<BN>, dim3((unsigned)tiles, (unsigned)g.splits), SG_THREADS,
-                 S::SMEM, ctx->stream, 1, g.splits, ma, mb, g);
+  SGLaunch<PRODUCTS> L{};
+  int64_t tiles = 0;
+  for (int i = 0; i < PRODUCTS; ++i) {
+    L.a[i] = make_slice_map(a[i]->data, a[i]->Kp, a[i]->rows, a[i]->batch * SL, 128, 1);
+    L.b[i] = make_slice_map(b[i]->data, b[i]->Kp, b[i]->rows, b[i]->batch * SL, BN, SL);
+    L.g[i] = g[i];
+    tiles += (int64_t)g[i].mt * g[i].nt * batch;
+    GB_REQUIRE(tiles < (int64_t)1 << 31, "gemm: too many tiles");
+    if (i == 0) L.first = (int)tiles;
+  }
+  launch_chained(gemm_sliced_kernel<BN, PRODUCTS>, dim3((unsigned)tiles, (unsigned)g[0].splits),
+                 SG_THREADS, S::SMEM, ctx->stream, 1, g[0].splits, L);
   count_launch(ctx);
 }
 
@@ -1152,24 +1183,11 @@ struct DigitBuf {
   DigitBuf& operator=(const DigitBuf&) = delete;
 };
 
-bool gemm_fp64_sliced(gb_ctx* ctx, int dtype, char opA, char opB, int64_t M, int64_t N, int64_t K,
-                      double alpha, const void* A, int64_t lda, int64_t sA, const void* B,
-                      int64_t ldb, int64_t sB, double beta, void* C, int64_t ldc, int64_t sC,
-                      int64_t batch, const Packed* pA, const Packed* pB) {
+static SGArgs sliced_args(gb_ctx* ctx, int dtype, char opA, char opB, int64_t M, int64_t N,
+                          int64_t K, double alpha, const void* A, int64_t lda, int64_t sA,
+                          const void* B, int64_t ldb, int64_t sB, double beta, void* C,
+                          int64_t ldc, int64_t sC, const Packed& a, const Packed& b) {
   const bool cx = is_cplx(dtype);
-  const int64_t bA = sA ? batch : 1, bB = sB ? batch : 1;
-  Packed a, b;
-  DigitBuf da(ctx), db(ctx);
-  if (!pA && !da.get(SLOT_PACK_A, sliced_bytes(M, K, cx, PACK_AS_A, bA))) return false;
-  if (!pB && !db.get(SLOT_PACK_B, sliced_bytes(N, K, cx, PACK_AS_B, bB))) return false;
-  SliceArgs aa{}, ab{};
-  if (pA) a = *pA;
-  else aa = slice_args(ctx, dtype, PACK_AS_A, opA, M, K, A, lda, sA, bA, da.p, a);
-  if (pB) b = *pB;
-  else ab = slice_args(ctx, dtype, PACK_AS_B, opB, N, K, B, ldb, sB, bB, db.p, b);
-  if (!pA && !pB) slice_launch(ctx, aa, ab);
-  else if (!pA) slice_launch(ctx, aa, SliceArgs{});
-  else if (!pB) slice_launch(ctx, ab, SliceArgs{});
   SGArgs g{};
   g.M = M;
   g.N = N;
@@ -1202,32 +1220,114 @@ bool gemm_fp64_sliced(gb_ctx* ctx, int dtype, char opA, char opB, int64_t M, int
   g.opA = opcode(opA);
   g.opB = opcode(opB);
   g.mt = (int)((M + 127) / 128);
-  const int sms = std::max(1, ctx->num_sms);
-  // Tile width and split by a model of the measured clocks: a k-block takes 3600 (64 columns;
-  // 1300 more for the accumulators, which that width cannot double-buffer) or 3300 (32
-  // columns) -- the loads bound both, and 64 columns read A half as often -- a tile 7500 of
-  // start-up and pipeline ends, its output 110 per column of a thread, adding the partial
-  // sums of a split 1000.
-  double best = 1e300;
+  return g;
+}
+
+// Tile width and split by a model of the measured clocks.  A k-block moves its digits into and out
+// of shared memory at 128 bytes a clock (388 KB at 32 columns, 616 KB at 64, which read A half as
+// often); measured 3300 and 4900.  A tile has 7500 of start-up and pipeline ends, its output 110
+// per column of a thread, adding the partial sums of a split 1000.  With a second product (mt2 > 0)
+// for both in one launch.
+struct SGPlan {
+  double clocks = 1e300;
   bool wide = false;
+  int nt[2] = {0, 0}, splits = 1;
+};
+static SGPlan sliced_plan(int sms, int mt, int64_t rows, int nkb, int64_t batch, int mt2 = 0,
+                          int64_t rows2 = 0, int nkb2 = 0) {
+  SGPlan p;
   for (int w = 0; w < 2; ++w) {
-    const int64_t nt = (b.rows + (w ? 63 : 31)) / (w ? 64 : 32);
-    const int64_t tiles = (int64_t)g.mt * nt * batch;
-    for (int sp = 1; sp <= 8 && (sp == 1 || (tiles * sp <= sms && sp * 2 <= g.nkb)); sp *= 2) {
+    const int64_t nt = (rows + (w ? 63 : 31)) / (w ? 64 : 32);
+    const int64_t nt2 = (rows2 + (w ? 63 : 31)) / (w ? 64 : 32);
+    const int64_t tiles = (int64_t)mt * nt * batch + (int64_t)mt2 * nt2;
+    const int least = mt2 ? std::min(nkb, nkb2) : nkb, most = std::max(nkb, nkb2);
+    for (int sp = 1; sp <= 8 && (sp == 1 || (tiles * sp <= sms && sp * 2 <= least)); sp *= 2) {
       const double waves = (double)((tiles * sp + sms - 1) / sms);
-      const double kb = (double)((g.nkb + sp - 1) / sp);
+      const double kb = (double)((most + sp - 1) / sp);
       const double t = waves * (kb * (w ? 4900.0 : 3300.0) + 7500.0 + (w ? 3520.0 : 1760.0) / sp) +
                        (sp > 1 ? 1000.0 : 0.0);
-      if (t < best) {
-        best = t;
-        wide = w;
-        g.nt = (int)nt;
-        g.splits = sp;
+      if (t < p.clocks) {
+        p.clocks = t;
+        p.wide = w;
+        p.nt[0] = (int)nt;
+        p.nt[1] = (int)nt2;
+        p.splits = sp;
       }
     }
   }
-  if (wide) launch_sliced<64>(ctx, a, b, g, batch);
-  else launch_sliced<32>(ctx, a, b, g, batch);
+  return p;
+}
+
+bool gemm_fp64_sliced(gb_ctx* ctx, int dtype, char opA, char opB, int64_t M, int64_t N, int64_t K,
+                      double alpha, const void* A, int64_t lda, int64_t sA, const void* B,
+                      int64_t ldb, int64_t sB, double beta, void* C, int64_t ldc, int64_t sC,
+                      int64_t batch, const Packed* pA, const Packed* pB) {
+  const bool cx = is_cplx(dtype);
+  const int64_t bA = sA ? batch : 1, bB = sB ? batch : 1;
+  Packed a, b;
+  DigitBuf da(ctx), db(ctx);
+  if (!pA && !da.get(SLOT_PACK_A, sliced_bytes(M, K, cx, PACK_AS_A, bA))) return false;
+  if (!pB && !db.get(SLOT_PACK_B, sliced_bytes(N, K, cx, PACK_AS_B, bB))) return false;
+  SliceArgs aa{}, ab{};
+  if (pA) a = *pA;
+  else aa = slice_args(ctx, dtype, PACK_AS_A, opA, M, K, A, lda, sA, bA, da.p, a);
+  if (pB) b = *pB;
+  else ab = slice_args(ctx, dtype, PACK_AS_B, opB, N, K, B, ldb, sB, bB, db.p, b);
+  if (!pA && !pB) slice_launch(ctx, aa, ab);
+  else if (!pA) slice_launch(ctx, aa, SliceArgs{});
+  else if (!pB) slice_launch(ctx, ab, SliceArgs{});
+  SGArgs g = sliced_args(ctx, dtype, opA, opB, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc,
+                         sC, a, b);
+  const int sms = std::max(1, ctx->num_sms);
+  const SGPlan p = sliced_plan(sms, g.mt, b.rows, g.nkb, batch);
+  g.nt = p.nt[0];
+  g.splits = p.splits;
+  const Packed *pa = &a, *pb = &b;
+  if (p.wide) launch_sliced<64, 1>(ctx, &pa, &pb, &g, batch);
+  else launch_sliced<32, 1>(ctx, &pa, &pb, &g, batch);
+  return true;
+}
+
+// y = x R + L x (+ y), x and the constants cut into digits: both products in one launch when
+// together they leave fewer SMs idle than one after the other; their outputs meet by atomic adds of
+// two values, whose sum does not depend on the order.  An apply of two complex products of 128 x
+// 256 x 256: 31.0 us one by one, 20.9 us; of 256 x 512 x 512: 58 and 49 us.
+bool gemm_sliced_pair(gb_ctx* ctx, int dtype, const void* x, int64_t M1, int64_t N1, int64_t K1,
+                      const Packed& R, const void* Rsrc, int64_t ldr, int64_t M2, int64_t N2,
+                      int64_t K2, const Packed& Lp, const void* Lsrc, int64_t ldl, bool accumulate,
+                      void* y) {
+  const bool cx = is_cplx(dtype);
+  const int sms = std::max(1, ctx->num_sms);
+  const int mt[2] = {(int)((M1 + 127) / 128), (int)((M2 + 127) / 128)};
+  const int64_t rows[2] = {R.rows, cx ? 2 * rup(N2, 32) : N2};
+  const int nkb[2] = {(int)(R.Kp / 64), (int)(Lp.Kp / 64)};
+  const SGPlan p = sliced_plan(sms, mt[0], rows[0], nkb[0], 1, mt[1], rows[1], nkb[1]);
+  const SGPlan p0 = sliced_plan(sms, mt[0], rows[0], nkb[0], 1);
+  const SGPlan p1 = sliced_plan(sms, mt[1], rows[1], nkb[1], 1);
+  Packed xa, xb;
+  const bool together = p.clocks < p0.clocks + p1.clocks;
+  const int64_t n = M1 * N1 * (cx ? 2 : 1);
+  if (!slice_both(ctx, dtype, x, M1, K1, N2, K2, xa, xb, (double*)y,
+                  together && !accumulate ? n : 0))
+    return false;
+  if (!together)
+    return gemm_fp64_sliced(ctx, dtype, 'N', 'N', M1, N1, K1, 1.0, x, M1, 0, Rsrc, ldr, 0,
+                            accumulate ? 1.0 : 0.0, y, M1, 0, 1, &xa, &R) &&
+           gemm_fp64_sliced(ctx, dtype, 'N', 'N', M2, N2, K2, 1.0, Lsrc, ldl, 0, x, K2, 0, 1.0, y,
+                            M2, 0, 1, &Lp, &xb);
+  SGArgs g[2] = {sliced_args(ctx, dtype, 'N', 'N', M1, N1, K1, 1.0, x, M1, 0, Rsrc, ldr, 0, 1.0, y,
+                             M1, 0, xa, R),
+                 sliced_args(ctx, dtype, 'N', 'N', M2, N2, K2, 1.0, Lsrc, ldl, 0, x, K2, 0, 1.0, y,
+                             M2, 0, Lp, xb)};
+  for (int i = 0; i < 2; ++i) {
+    g[i].nt = p.nt[i];
+    g[i].splits = p.splits;
+    g[i].add = 1;
+  }
+  const Packed* pa[2] = {&xa, &Lp};
+  const Packed* pb[2] = {&R, &xb};
+  if (p.wide) launch_sliced<64, 2>(ctx, pa, pb, g, 1);
+  else launch_sliced<32, 2>(ctx, pa, pb, g, 1);
   return true;
 }
 

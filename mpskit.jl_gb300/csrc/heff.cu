@@ -1992,17 +1992,9 @@ void heff_apply_raw(gb_heff* h, const void* x, void* y) {
         ++i;
         continue;
       }
-      // both products with cut constants: the two cuts of x in one launch (an apply of complex
-      // 256 x 512 x 512 and 512 x 256 x 512 65 -> 58 us)
-      Packed xa, xb;
       if (!ctx->lane && s.hasPB && s.pB.slices && q.hasPA && q.pA.slices &&
-          slice_both(ctx, h->dtype, x, s.M, s.K, q.N, q.K, xa, xb)) {
-        const bool ok =
-            gemm_fp64_sliced(ctx, h->dtype, 'N', 'N', s.M, s.N, s.K, 1.0, x, s.lda, 0, s.cB, s.ldb,
-                             0, s.accumulate ? 1.0 : 0.0, y, s.ldc, 0, 1, &xa, &s.pB) &&
-            gemm_fp64_sliced(ctx, h->dtype, 'N', 'N', q.M, q.N, q.K, 1.0, q.cA, q.lda, 0, x, q.ldb,
-                             0, 1.0, y, q.ldc, 0, 1, &q.pA, &xb);
-        GB_REQUIRE(ok, "heff: product of cut operands");
+          gemm_sliced_pair(ctx, h->dtype, x, s.M, s.N, s.K, s.pB, s.cB, s.ldb, q.M, q.N, q.K, q.pA,
+                           q.cA, q.lda, s.accumulate, y)) {
         ++i;
         continue;
       }
