@@ -368,7 +368,11 @@ void packed_layout(Packed& out, void* data, int64_t R, int64_t K, bool cplx, int
                    int64_t batch, int prec = GB_PREC_BF16X3);
 void pack_operand(gb_ctx* ctx, int dtype, int role, char op, int64_t M_or_N, int64_t K,
                   const void* src, int64_t ld, int64_t stride, int64_t batch, Packed& out,
-                  void* dst, int prec = GB_PREC_BF16X3);
+                  void* dst, int prec = GB_PREC_BF16X3, double* zero = nullptr,
+                  int64_t nzero = 0);
+bool gemm_split_pair(gb_ctx* ctx, int dtype, int prec, const void* x, int64_t M1, int64_t N1,
+                     int64_t K1, const Packed& R, int64_t M2, int64_t N2, int64_t K2,
+                     const Packed& Lp, bool accumulate, void* y);
 // Skipping structurally zero work in mixpack_run: x is the output of a GEMM with an output
 // map (xmap, onc columns of 128 per row tile of 128); input i of the mix at (a, n) sits at
 // row a + roff[i], column coff[i] + n*xnM of that matrix.  prev: scratch of the packed

@@ -231,8 +231,9 @@ __global__ void nonzero_products_kernel(const uint32_t* __restrict__ ca, const u
   if ((threadIdx.x & 31) == 0 && acc != 0.0) atomicAdd(&work[1], 2.0 * acc);
 }
 
-// prev = map (if asked for), map = 0
-__global__ void map_reset_kernel(uint32_t* map, uint32_t* prev, int64_t n) {
+// prev = map (if asked for), map = 0; also = 0
+__global__ void map_reset_kernel(uint32_t* map, uint32_t* prev, int64_t n, double* also,
+                                 int64_t n2) {
   chain_release();
   chain_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
@@ -240,13 +241,17 @@ __global__ void map_reset_kernel(uint32_t* map, uint32_t* prev, int64_t n) {
     if (prev) prev[i] = map[i];
     map[i] = 0;
   }
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n2;
+       i += (int64_t)gridDim.x * blockDim.x)
+    also[i] = 0.0;
 }
 
-static void map_reset(gb_ctx* ctx, uint32_t* map, uint32_t* prev, size_t bytes) {
-  const int64_t n = (int64_t)(bytes / 4);
-  if (!n) return;
-  launch_chained(map_reset_kernel, dim3((unsigned)std::min<int64_t>((n + 255) / 256, 128)), 256, 0,
-                 ctx->stream, 1, 1, map, prev, n);
+static void map_reset(gb_ctx* ctx, uint32_t* map, uint32_t* prev, size_t bytes,
+                      double* also = nullptr, int64_t n2 = 0) {
+  const int64_t n = (int64_t)(bytes / 4), most = std::max(n, n2);
+  if (!most) return;
+  launch_chained(map_reset_kernel, dim3((unsigned)std::min<int64_t>((most + 255) / 256, 608)), 256,
+                 0, ctx->stream, 1, 1, map, prev, n, also, n2);
   count_launch(ctx);
 }
 
@@ -254,7 +259,7 @@ static size_t mask_bytes(const Packed& p) { return (size_t)p.batch * p.mrows * p
 
 void pack_operand(gb_ctx* ctx, int dtype, int role, char op, int64_t R, int64_t K,
                   const void* src, int64_t ld, int64_t stride, int64_t batch, Packed& out,
-                  void* dst, int prec) {
+                  void* dst, int prec, double* zero, int64_t nzero) {
   bool cx = is_cplx(dtype);
   PackArgs p;
   p.role = role;
@@ -270,7 +275,7 @@ void pack_operand(gb_ctx* ctx, int dtype, int role, char op, int64_t R, int64_t 
   packed_layout(out, dst, R, K, cx, role, batch, prec);
   // the planes need no memset: the kernel writes every (row, k < Kh) entry, zeros
   // included for k >= K; only the nonzero map starts cleared
-  map_reset(ctx, out.mask, nullptr, mask_bytes(out));
+  map_reset(ctx, out.mask, nullptr, mask_bytes(out), zero, nzero);
   GB_REQUIRE(batch <= 65535 && (R + 31) / 32 <= 65535, "pack: grid too large");
   dim3 grid((unsigned)((p.Kh + 31) / 32), (unsigned)((R + 31) / 32), (unsigned)batch);
   auto run = [&](auto kernel, auto* planes) {
@@ -802,6 +807,13 @@ struct PArgs {
   int skip_zero_out;
   int c_f32;  // C is stored in FP32 (exact when alpha = 1 and beta = 0: C is the accumulator)
 };
+// one product, or two with a tile per CTA, those of the second after those of the first, that add
+// up in one output
+template <int PRODUCTS>
+struct PLaunch {
+  CUtensorMap a[PRODUCTS], b[PRODUCTS];
+  PArgs p[PRODUCTS];
+};
 
 constexpr int PS_RING = 4;
 constexpr int PS_THREADS = 224;  // A loads and schedule, MMA, four epilogue warps, B loads
@@ -830,10 +842,12 @@ __device__ __forceinline__ TileMasks<BN> tile_masks(const PArgs& p, int mi, int 
   return t;
 }
 
-template <int BN, int STAGES, bool TF32>
+template <int BN, int STAGES, bool TF32, int PRODUCTS>
 __global__ void __launch_bounds__(PS_THREADS, 1)
-    gemm_bf16x3_persistent(const __grid_constant__ CUtensorMap mapA,
-                           const __grid_constant__ CUtensorMap mapB, PArgs args) {
+    gemm_bf16x3_persistent(const __grid_constant__ PLaunch<PRODUCTS> L) {
+  const int which = PRODUCTS > 1 && (int)blockIdx.x >= L.p[0].ntiles ? 1 : 0;
+  const PArgs args = L.p[which];  // (a reference into the parameters is read through memory)
+  const CUtensorMap &mapA = L.a[which], &mapB = L.b[which];
   constexpr int BKE = TF32 ? 32 : 64;  // k elements per stage (one 128-byte swizzle row)
   constexpr int A_BYTES = TC_BM * 128;
   constexpr int B_BYTES = BN * 128;
@@ -927,11 +941,18 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
   if (warp == 0 && elect_one()) {
     // ---------------- scheduler + producer of A
     uint32_t g = 0;
+    int tiles_taken = 0;
     bool ok = true;
     for (int j = 0; ok; ++j) {
       int t = -1, nk = 0, mi = 0, ni = 0, z = 0;
       for (;;) {
-        int c = (int)atomicAdd(args.counter, 1u);
+        int c;
+        if (PRODUCTS > 1) {  // this CTA's tile, then none
+          if (tiles_taken++) break;
+          c = (int)blockIdx.x - (which ? L.p[0].ntiles : 0);
+        } else {
+          c = (int)atomicAdd(args.counter, 1u);
+        }
         if (c >= args.ntiles) break;
         z = c / mn;
         int r = c - z * mn;
@@ -1126,7 +1147,13 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
         // addition of an accumulating term: the FP64 pipe issues a warp instruction in 16
         // clocks, and a conversion and an unused multiply or add per element were most of a
         // tile's time
-        if (plain && args.c_f32) {
+        if (PRODUCTS > 1) {
+#pragma unroll
+          for (int jj = 0; jj < 32; ++jj) {
+            const int64_t n = n0 + c0 + jj;
+            if (n < args.N) atomicAdd(args.C + off(n), to_double(__uint_as_float(v[jj])));
+          }
+        } else if (plain && args.c_f32) {
 #pragma unroll
           for (int jj = 0; jj < 32; ++jj) {
             const int64_t n = n0 + c0 + jj;
@@ -1168,7 +1195,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
   }
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0) tiles_done(args.counter);
+  if (PRODUCTS == 1 && threadIdx.x == 0) tiles_done(args.counter);
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
@@ -1258,6 +1285,72 @@ bool tc_available(gb_ctx* ctx) {
   return major == 10 && minor == 3;
 }
 
+static PArgs persistent_args(gb_ctx* ctx, const Packed& A, const Packed& B, int64_t M, int64_t N,
+                             double alpha, double beta, void* C, int64_t ldc, int64_t sC,
+                             int bn) {
+  const int64_t batch = std::max(A.batch, B.batch), Npk = B.rows;
+  PArgs p{};
+  p.M = M;
+  p.N = Npk;
+  p.Nlog = N;
+  p.cplx = A.cplx;
+  p.kblocks = (int)(A.Kp / A.bk);
+  p.mt = (int)((M + TC_BM - 1) / TC_BM);
+  p.nt = (int)((Npk + bn - 1) / bn);
+  const int64_t ntiles = (int64_t)p.mt * p.nt * batch;
+  GB_REQUIRE(ntiles < (int64_t)INT32_MAX / 2, "gemm_split: too many tiles");
+  p.ntiles = (int)ntiles;
+  p.batchA = (int)A.batch;
+  p.batchB = (int)B.batch;
+  p.alpha = alpha;
+  p.beta = beta;
+  p.C = (double*)C;
+  p.ldc = ldc;
+  p.sC = sC;
+  const bool masked = ctx->gemm_schedule != GB_SCHED_PERSISTENT_DENSE && A.mask && B.mask;
+  GB_REQUIRE(!masked || A.kw == B.kw, "gemm_split: nonzero maps differ in width");
+  p.maskA = masked ? A.mask : nullptr;
+  p.maskB = masked ? B.mask : nullptr;
+  p.kw = A.kw;
+  p.mskA_b = A.mrows * A.kw;
+  p.mskB_b = B.mrows * B.kw;
+  p.mrowsB = B.mrows;
+  p.counter = ctx->d_tile_counter;
+  p.status = ctx->d_status;
+  p.wait_ns = ctx->wait_ns;
+  p.work = (ctx->profiling || ctx->counting) ? ctx->d_work : nullptr;
+  return p;
+}
+
+template <int BN, int ST, bool TF, int PRODUCTS>
+static void persistent_launch(gb_ctx* ctx, unsigned grid, const PLaunch<PRODUCTS>& l) {
+  constexpr int SM = persistent_smem<BN, ST>();
+  static std::once_flag once;  // contexts may launch from several host threads
+  std::call_once(once, [] {
+    GB_CHECK_CUDA(cudaFuncSetAttribute(gemm_bf16x3_persistent<BN, ST, TF, PRODUCTS>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, SM));
+  });
+  launch_chained(gemm_bf16x3_persistent<BN, ST, TF, PRODUCTS>, dim3(grid), PS_THREADS, SM,
+                 ctx->stream, 1, 1, l);
+}
+template <int PRODUCTS>
+static void persistent_launch(gb_ctx* ctx, int bn, bool tf32, unsigned grid,
+                              const PLaunch<PRODUCTS>& l) {
+  if (bn == 32) {
+    if (tf32) persistent_launch<32, 9, true>(ctx, grid, l);
+    else persistent_launch<32, 9, false>(ctx, grid, l);
+  } else if (bn == 64) {
+    if (tf32) persistent_launch<64, 8, true>(ctx, grid, l);
+    else persistent_launch<64, 8, false>(ctx, grid, l);
+  } else if (bn == 128) {
+    if (tf32) persistent_launch<128, 6, true>(ctx, grid, l);
+    else persistent_launch<128, 6, false>(ctx, grid, l);
+  } else {
+    if (tf32) persistent_launch<256, 4, true>(ctx, grid, l);
+    else persistent_launch<256, 4, false>(ctx, grid, l);
+  }
+}
+
 void gemm_split(gb_ctx* ctx, int dtype, const Packed& A, const Packed& B, int64_t M,
                 int64_t N, double alpha, double beta, void* C, int64_t ldc, int64_t sC,
                 uint32_t* outmap, bool c_f32) {
@@ -1340,36 +1433,8 @@ void gemm_split(gb_ctx* ctx, int dtype, const Packed& A, const Packed& B, int64_
       }
     }
     if (bn != TC_BN) mb = make_map(B, bn);
-    PArgs p;
-    p.M = M;
-    p.N = Npk;
-    p.Nlog = N;
-    p.cplx = A.cplx;
-    p.kblocks = (int)(A.Kp / A.bk);
-    p.mt = (int)((M + TC_BM - 1) / TC_BM);
-    p.nt = (int)((Npk + bn - 1) / bn);
-    const int64_t ntiles = (int64_t)p.mt * p.nt * batch;
-    GB_REQUIRE(ntiles < (int64_t)INT32_MAX / 2, "gemm_split: too many tiles");
-    p.ntiles = (int)ntiles;
-    p.batchA = (int)A.batch;
-    p.batchB = (int)B.batch;
-    p.alpha = alpha;
-    p.beta = beta;
-    p.C = (double*)C;
-    p.ldc = ldc;
-    p.sC = sC;
-    const bool masked = ctx->gemm_schedule != GB_SCHED_PERSISTENT_DENSE && A.mask && B.mask;
-    GB_REQUIRE(!masked || A.kw == B.kw, "gemm_split: nonzero maps differ in width");
-    p.maskA = masked ? A.mask : nullptr;
-    p.maskB = masked ? B.mask : nullptr;
-    p.kw = A.kw;
-    p.mskA_b = A.mrows * A.kw;
-    p.mskB_b = B.mrows * B.kw;
-    p.mrowsB = B.mrows;
-    p.counter = ctx->d_tile_counter;
-    p.status = ctx->d_status;
-    p.wait_ns = ctx->wait_ns;
-    p.work = (ctx->profiling || ctx->counting) ? ctx->d_work : nullptr;
+    PArgs p = persistent_args(ctx, A, B, M, N, alpha, beta, C, ldc, sC, bn);
+    const int64_t ntiles = p.ntiles;
     p.outmap = outmap;
     p.prevmap = nullptr;
     p.onc = (N + 127) / 128;
@@ -1384,31 +1449,11 @@ void gemm_split(gb_ctx* ctx, int dtype, const Packed& A, const Packed& B, int64_
       map_reset(ctx, outmap, p.skip_zero_out ? outmap + mb / 4 : nullptr, mb);
     }
     const unsigned grid = (unsigned)std::min<int64_t>(ntiles, std::max(1, ctx->num_sms));
-#define GB_PERSISTENT(BN_, ST_, TF_)                                                          \
-  do {                                                                                        \
-    constexpr int SM = persistent_smem<BN_, ST_>();                                           \
-    static std::once_flag once;                                                               \
-    std::call_once(once, [] {                                                                 \
-      GB_CHECK_CUDA(cudaFuncSetAttribute(gemm_bf16x3_persistent<BN_, ST_, TF_>,               \
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, SM));   \
-    });                                                                                       \
-    launch_chained(gemm_bf16x3_persistent<BN_, ST_, TF_>, dim3(grid), PS_THREADS, SM,         \
-                   ctx->stream, 1, 1, ma, mb, p);                                             \
-  } while (0)
-    if (bn == 32) {
-      if (tf32) GB_PERSISTENT(32, 9, true);
-      else GB_PERSISTENT(32, 9, false);
-    } else if (bn == 64) {
-      if (tf32) GB_PERSISTENT(64, 8, true);
-      else GB_PERSISTENT(64, 8, false);
-    } else if (bn == 128) {
-      if (tf32) GB_PERSISTENT(128, 6, true);
-      else GB_PERSISTENT(128, 6, false);
-    } else {
-      if (tf32) GB_PERSISTENT(256, 4, true);
-      else GB_PERSISTENT(256, 4, false);
-    }
-#undef GB_PERSISTENT
+    PLaunch<1> l{};
+    l.a[0] = ma;
+    l.b[0] = mb;
+    l.p[0] = p;
+    persistent_launch(ctx, bn, tf32, grid, l);
   }
   GB_CHECK_CUDA(cudaGetLastError());
   if (ev1) GB_CHECK_CUDA(cudaEventRecord(ev1, ctx->stream));
@@ -1419,6 +1464,61 @@ void gemm_split(gb_ctx* ctx, int dtype, const Packed& A, const Packed& B, int64_
     GB_CHECK_CUDA(cudaGetLastError());
     count_launch(ctx);
   }
+}
+
+// y = x R + L x (+ y) with packed constants: both products in one launch, a tile per CTA, when that
+// is done earlier than one after the other; their outputs meet by atomic adds of two values, whose
+// sum does not depend on the order.  False (nothing done) otherwise.  (tf32x3, complex 256 x 512 x
+// 512 and 512 x 256 x 512, an apply: 64.8 us one by one, 38.8 us.)
+bool gemm_split_pair(gb_ctx* ctx, int dtype, int prec, const void* x, int64_t M1, int64_t N1,
+                     int64_t K1, const Packed& R, int64_t M2, int64_t N2, int64_t K2,
+                     const Packed& Lp, bool accumulate, void* y) {
+  if (ctx->profiling || ctx->counting || ctx->gemm_bn || ctx->gemm_schedule == GB_SCHED_TILE ||
+      !tc_available(ctx))
+    return false;
+  const bool cx = is_cplx(dtype);
+  const int64_t sms = std::max(1, ctx->num_sms);
+  const int64_t mt[2] = {(M1 + TC_BM - 1) / TC_BM, (M2 + TC_BM - 1) / TC_BM};
+  const int64_t rows[2] = {R.rows, cx ? 2 * N2 : N2};
+  const int64_t kb[2] = {R.Kp / R.bk, Lp.Kp / Lp.bk};
+  // clocks: three passes over the k-blocks of a wave of tiles, 3000 for a launch of a chain, the
+  // atomic output 10000 and 1.2 per entry of a tile (bf16x3 509 x 2036 x 2036 and 2036 x 509 x
+  // 2036: 41 us one by one, 45 together)
+  auto tiles = [&](int i, int w) { return mt[i] * ((rows[i] + w - 1) / w); };
+  double each = 0;
+  for (int i = 0; i < 2; ++i) {
+    double best = 1e300;
+    for (int w = 256; w >= 32; w /= 2)
+      best = std::min(best, 3.0 * kb[i] * ((tiles(i, w) + sms - 1) / sms) * (256 + 2 * w));
+    each += best + 3000.0;
+  }
+  int bn = 0;
+  double both = each;
+  for (int w = 256; w >= 32; w /= 2) {
+    const double t = 3.0 * std::max(kb[0], kb[1]) * (256 + 2 * w) + 13000.0 + 1.2 * TC_BM * w;
+    if (tiles(0, w) + tiles(1, w) <= sms && t < both) {
+      both = t;
+      bn = w;
+    }
+  }
+  if (!bn) return false;
+  Packed xa, xb;
+  void* da = scratch(ctx, SLOT_PACK_A, packed_bytes(M1, K1, cx, PACK_AS_A, 1, prec));
+  void* db = scratch(ctx, SLOT_PACK_B, packed_bytes(N2, K2, cx, PACK_AS_B, 1, prec));
+  pack_operand(ctx, dtype, PACK_AS_A, 'N', M1, K1, x, M1, 0, 1, xa, da, prec, (double*)y,
+               accumulate ? 0 : M1 * N1 * (cx ? 2 : 1));
+  pack_operand(ctx, dtype, PACK_AS_B, 'N', N2, K2, x, K2, 0, 1, xb, db, prec);
+  load_encode();
+  PLaunch<2> l{};
+  l.a[0] = make_map(xa, TC_BM);
+  l.b[0] = make_map(R, bn);
+  l.p[0] = persistent_args(ctx, xa, R, M1, N1, 1.0, 1.0, y, M1, 0, bn);
+  l.a[1] = make_map(Lp, TC_BM);
+  l.b[1] = make_map(xb, bn);
+  l.p[1] = persistent_args(ctx, Lp, xb, M2, N2, 1.0, 1.0, y, M2, 0, bn);
+  persistent_launch(ctx, bn, xa.esz == 4, (unsigned)(l.p[0].ntiles + l.p[1].ntiles), l);
+  count_launch(ctx);
+  return true;
 }
 
 size_t outmap_bytes(int64_t M, int64_t N) {

@@ -1975,7 +1975,7 @@ void heff_apply_raw(gb_heff* h, const void* x, void* y) {
     h->t2 = dalloc(h, (size_t)h->t2_elems * elem_size(h->dtype));
   // a product with x on the left and the next one with x on the right, both into y
   auto pair_of = [&](size_t i) {
-    if (h->prec != GB_PREC_FP64 || i + 1 >= h->steps.size()) return false;
+    if (i + 1 >= h->steps.size()) return false;
     const Step &p = h->steps[i], &q = h->steps[i + 1];
     return p.is_gemm && q.is_gemm && p.srcA == S_X && p.srcB == S_CONST && p.dst == S_Y &&
            q.srcA == S_CONST && q.srcB == S_X && q.dst == S_Y && q.accumulate && p.opA == 'N' &&
@@ -1987,14 +1987,18 @@ void heff_apply_raw(gb_heff* h, const void* x, void* y) {
     const Step& s = h->steps[i];
     if (pair_of(i)) {
       const Step& q = h->steps[i + 1];
-      if (gemm_small_dual(ctx, h->dtype, s.M, q.M / s.M, q.N, s.K, s.cB, s.ldb, q.K, q.cA, q.lda, x,
-                          s.accumulate, y)) {
-        ++i;
-        continue;
-      }
-      if (!ctx->lane && s.hasPB && s.pB.slices && q.hasPA && q.pA.slices &&
-          gemm_sliced_pair(ctx, h->dtype, x, s.M, s.N, s.K, s.pB, s.cB, s.ldb, q.M, q.N, q.K, q.pA,
-                           q.cA, q.lda, s.accumulate, y)) {
+      if (h->prec != GB_PREC_FP64) {
+        if (s.hasPB && q.hasPA &&
+            gemm_split_pair(ctx, h->dtype, h->prec, x, s.M, s.N, s.K, s.pB, q.M, q.N, q.K, q.pA,
+                            s.accumulate, y)) {
+          ++i;
+          continue;
+        }
+      } else if (gemm_small_dual(ctx, h->dtype, s.M, q.M / s.M, q.N, s.K, s.cB, s.ldb, q.K, q.cA,
+                                 q.lda, x, s.accumulate, y) ||
+                 (!ctx->lane && s.hasPB && s.pB.slices && q.hasPA && q.pA.slices &&
+                  gemm_sliced_pair(ctx, h->dtype, x, s.M, s.N, s.K, s.pB, s.cB, s.ldb, q.M, q.N,
+                                   q.K, q.pA, q.cA, q.lda, s.accumulate, y))) {
         ++i;
         continue;
       }

@@ -83,3 +83,36 @@ def test_chain_mix_in_planes(ctx, Dl, Dr, cx, prec):
     got = apply(prec, 1)
     assert np.linalg.norm(got - ref) <= 2.0 ** -14 * np.linalg.norm(ref)
     assert np.array_equal(apply(prec, 3), got)  # over planes and maps of an earlier apply
+
+
+@pytest.mark.parametrize("prec", ["bf16x3", "tf32x3"])
+@pytest.mark.parametrize("cx", [False, True])
+@pytest.mark.parametrize("Dl,Dr", [(3, 2), (40, 41), (128, 130), (200, 256)])
+def test_both_products_in_one_launch(ctx, Dl, Dr, cx, prec):
+    """A one-site operator in split precision whose products with the two environments share a
+    launch: within the planes' 2^-14 of FP64, and the same bits from apply to apply (sums of two
+    values do not depend on their order)."""
+    rng = np.random.default_rng(Dl + 7 * Dr)
+    dt = np.complex128 if cx else np.float64
+    H = mpsgb.heisenberg_XXX(6, dtype=dt)
+    n = np.asarray(H.W[2]).shape[0]
+
+    def env(D, unit):
+        g = rng.standard_normal((D, n, D)) + (1j * rng.standard_normal((D, n, D)) if cx else 0)
+        g[:, unit, :] = np.eye(D)
+        return g.astype(dt)
+
+    GL, GR = env(Dl, 0), env(Dr, -1)
+    dev = lambda k, a: mpsgb.DeviceTensor.from_numpy(ctx, k, a)
+    x = dev("mps", rng.standard_normal((Dl, 2, Dr)).astype(dt))
+
+    def op(p):
+        return mpsgb.DerivativeOperator(ctx, mpsgb._lib.GB_HEFF_AC, dev("gl", GL),
+                                        H.device(ctx, dt)[2], None, dev("gr", GR),
+                                        mpsgb.GB300Backend(p))
+
+    ref = op("fp64")(x).numpy()
+    o = op(prec)
+    got = [o(x).numpy() for _ in range(3)]
+    assert np.linalg.norm(got[0] - ref) <= 2.0 ** -14 * np.linalg.norm(ref)
+    assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
