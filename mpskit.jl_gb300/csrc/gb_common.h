@@ -251,10 +251,12 @@ void gemm_fp64(gb_ctx* ctx, int dtype, char opA, char opB, int64_t M, int64_t N,
 
 // FP64 products on the tensor cores in exact integer arithmetic (gemm_f64.cu)
 constexpr int F64_SLICES = 7;
-// Real multiply-adds from which the digits win: the small-tile kernel takes 6.5 us + 1.75 us
-// per million (128 x 128 x 128 complex, 8.4 M: 23 us; 256 x 128 x 128: 35 us), the digit path
-// 25-28 us for anything up to 70 M and 8 us less with one operand already cut.
-constexpr double F64_SLICED_MIN_MAC = 1.2e7;
+// Real multiply-adds from which the digits win, in us for the small tiles and for the digits, both
+// operands cut: complex 80^3 (2.0 M) 14.4 and 16.9, 96^3 (3.5 M) 19.9 and 16.9, 128^3 (8.4 M) 29.7
+// and 17.3; real 128 x 160 x 160 (3.3 M) 16.9 both, 1000 x 30 x 300 (9 M) 18.8 and 13.2.  With a
+// constant operand the other side is two small products in one launch.
+constexpr double F64_SLICED_MIN_MAC = 3.5e6;
+constexpr double F64_SMALL_MAX_MAC = 1.2e7;  // small tiles, where the digits are not to be had
 constexpr double F64_SLICED_MIN_MAC_CUT = 8e6;  // one operand constant
 bool gemm_sliced_wanted(gb_ctx* ctx, int dtype, int64_t M, int64_t N, int64_t K, int64_t batch,
                         double min_mac = F64_SLICED_MIN_MAC);

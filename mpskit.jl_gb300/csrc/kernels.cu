@@ -499,7 +499,7 @@ void gemm_fp64(gb_ctx* ctx, int dtype, char opA, char opB, int64_t M, int64_t N,
                        ldc, sC, batch, pA, pB))
     return;
   const double mac = (double)M * (double)N * (double)K * (double)batch * (is_cplx(dtype) ? 4 : 1);
-  if (mac < F64_SLICED_MIN_MAC) {
+  if (mac < F64_SMALL_MAX_MAC) {
     const SmallPlan p = gemm_small_plan(std::max(1, ctx->num_sms), M, N, K, batch,
                                         is_cplx(dtype));
     if (p.ok) {
