@@ -17,9 +17,9 @@
 // remaining rows once these are long, and two grid barriers per block.
 //
 // Measured (QR and LQ of a 256 x 2 x 256 complex tensor): 11.9 ms with the library's Householder
-// routines, 1.31 ms here; one complex 512 x 256 factorisation 5.9 ms before, 0.59 ms here (0.1 ms
-// of it the products).  Blocks of 16 took 0.84 ms: the chain through a diagonal block grows with
-// its square, the grid barriers saved are 3 k clocks each.
+// routines, 1.1 ms here; one complex 512 x 256 factorisation 5.9 ms before, 0.50 ms here (0.13 ms
+// of it the products).  Blocks of 16 took 0.84 ms (the chain through a diagonal block grows with its
+// square, the grid barriers saved are 3 k clocks each), updates of one column at a time 0.59.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -82,7 +82,7 @@ __device__ __forceinline__ double inverse(double d) {
   const int hi = __double2hiint(d);
   const int s = ((hi >> 20) & 0x7ff) - 1023;
   const double m = __hiloint2double(hi - (s << 20), __double2loint(d));
-  const double y = to_double(__frcp_rn(to_float(m)));
+  const double y = to_double(__fdividef(1.0f, to_float(m)));
   const double e = fma(-m, y, 1.0);
   const double r = fma(y, fma(e, e, e), y);
   return __hiloint2double(__double2hiint(r) - (s << 20), __double2loint(r));
@@ -171,31 +171,38 @@ __device__ void diag_block(const CholArgs& g, int k0, int nb, T (*row)[2 * NB + 
   __syncthreads();
 }
 
-// A(r, c) -= sum_k conj(P(k, r)) P(k, c) over the block row k0..k0+nb-1, for the 32 rows from r0
+// A(r, c) -= sum_k conj(P(k, r)) P(k, c) over the block row k0..k0+nb-1, for the 32 rows from r0 and
+// columns q0..q1-1 of the list cl..n-1 (left part, only the upper triangle), n.. (right part).  Two
+// columns at a time, all their loads ahead of the arithmetic.
 template <typename T>
 __device__ __forceinline__ void update_columns(const CholArgs& g, int k0, int nb, int r0, int rend,
-                                               int c0, int c1, int lane) {
+                                               int cl, int q0, int q1, int lane) {
   T* A = (T*)g.A;
   const int64_t ld = g.n;
-  const int r = r0 + lane;
+  const int r = r0 + lane, nl = g.n - cl;
   T p[NB];
 #pragma unroll
   for (int k = 0; k < NB; ++k) p[k] = (r < rend && k < nb) ? A[k0 + k + ld * r] : T{};
-  for (int c = c0; c < c1; ++c) {
-    // left part: only the upper triangle
-    if (c < g.n && c < r0) continue;
-    T* q = A + ld * c;
-    const bool live = r < rend && (c >= g.n || r <= c);
-    T v = live ? q[r] : T{};
-    if (nb == NB) {
+  for (int qq = q0; qq < q1; qq += 2) {
+    T v[2], w[2][NB];
+    T* at[2];
+    bool live[2];
 #pragma unroll
-      for (int k = 0; k < NB; ++k) sub_cmul(v, p[k], q[k0 + k]);
-    } else {
+    for (int u = 0; u < 2; ++u) {
+      const int q = min(qq + u, q1 - 1), c = q < nl ? cl + q : g.n + (q - nl);
+      at[u] = A + ld * c;
+      live[u] = qq + u < q1 && r < rend && (c >= g.n || r <= c);
+      v[u] = live[u] ? at[u][r] : T{};
 #pragma unroll
-      for (int k = 0; k < NB; ++k)
-        if (k < nb) sub_cmul(v, p[k], q[k0 + k]);
+      for (int k = 0; k < NB; ++k) w[u][k] = at[u][k0 + min(k, nb - 1)];
     }
-    if (live) q[r] = v;
+    // p is zero from nb on
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+#pragma unroll
+      for (int k = 0; k < NB; ++k) sub_cmul(v[u], p[k], w[u][k]);
+      if (live[u]) at[u][r] = v[u];
+    }
   }
 }
 
@@ -270,23 +277,20 @@ __global__ void __launch_bounds__(QT, 1) gram_chol_kernel(CholArgs g) {
     } else if (gridDim.x > 1) {
       const int w = (int)(blockIdx.x - 1) + warp * (int)(gridDim.x - 1);
       const int ws = (int)(gridDim.x - 1) * QW;
-      // items: a group of rows and a run of four of its columns; the first group is the next
-      // block row (its own diagonal block apart), the others 32 rows each
+      // items: a group of rows and a run of four of its columns, of two while that leaves warps
+      // idle; the first group is the next block row (its own diagonal block apart), the others 32
+      // rows each
       const int groups = 1 + (n - k1 - nb2 + 31) / 32;
+      const int run = groups * ((n + 3) / 4) > ws ? 4 : 2;
       int done = 0;
       for (int gr = 0; gr < groups; ++gr) {
         const int r0 = gr ? k1 + nb2 + 32 * (gr - 1) : k1;
         const int rend = gr ? min(n, r0 + 32) : k1 + nb2;
         const int cl = gr ? r0 : k1 + nb2;         // first left column
         const int cols = (n - cl) + k1;            // left columns, then right columns 0..k1-1
-        const int items = (cols + 3) / 4;
-        for (int it = ((w - done) % ws + ws) % ws; it < items; it += ws) {
-          const int q0 = 4 * it, q1 = min(cols, q0 + 4), nl = n - cl;
-          const int a0 = min(q0, nl), a1 = min(q1, nl);
-          if (a0 < a1) update_columns<T>(g, k0, nb, r0, rend, cl + a0, cl + a1, lane);
-          const int b0 = max(q0, nl) - nl, b1 = q1 - nl;
-          if (b0 < b1) update_columns<T>(g, k0, nb, r0, rend, n + b0, n + b1, lane);
-        }
+        const int items = (cols + run - 1) / run;
+        for (int it = ((w - done) % ws + ws) % ws; it < items; it += ws)
+          update_columns<T>(g, k0, nb, r0, rend, cl, run * it, min(cols, run * it + run), lane);
         done = (done + items) % ws;
       }
     }
