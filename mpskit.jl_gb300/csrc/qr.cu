@@ -6,9 +6,11 @@
 // step that makes Q1 orthonormal to rounding (CholeskyQR2: Yamamoto, Nakatsukasa, Yanagisawa &
 // Fukaya, ETNA 44 (2015) 306-326).  With |E| small the Cholesky factor of 1 + E is 1 + u to
 // first order, u the upper triangle of E with half its diagonal, and its inverse 1 - u: the
-// second step is two products and no factorisation; while |E| is not yet below 1e-9 it is
-// repeated (the error goes as E^2).  A matrix whose Gram matrix has no Cholesky factor, or
-// whose E exceeds 0.1, is left to the caller's Householder routine.
+// second step is a product and no factorisation; it is repeated while E^2 is not yet rounding.
+// R is then the upper triangle of Q' A.  (The product of the passes' factors (1 + u) R1 is not:
+// (1 - u)(1 + u) = 1 - u^2, and the u^2 of the first pass, up to 1e-2, stays in Q R for good --
+// a residual of 2e-10 |A| at a condition number of 1e8, 2e-16 here.)  A matrix whose Gram matrix
+// has no Cholesky factor, or whose E exceeds 0.1, is left to the caller's Householder routine.
 //
 // The products run as the plain-precision GEMMs (gemm_f64.cu).  gram_chol_kernel does the rest
 // in one cooperative launch: the Cholesky factor of G and its inverse, by eliminating [G | 1]
@@ -90,9 +92,9 @@ __device__ __forceinline__ double inverse(double d) {
 
 struct CholArgs {
   int n;
-  void* A;      // n x 2n column-major: [G | 1] on entry (G: upper triangle), [R | R^-H] on exit
+  void* A;      // n x 2n column-major: [G | 1] on entry (G: upper triangle), R^-H in the right
+                // half on exit
   void* Z;      // NB x NB: inverse of the current diagonal block's (lower) factor
-  void* R;      // n x n: the factor with zeros below the diagonal
   int* fail;    // set when a pivot is not positive
   unsigned int* bar;
   int* status;
@@ -295,17 +297,6 @@ __global__ void __launch_bounds__(QT, 1) gram_chol_kernel(CholArgs g) {
       }
     }
   }
-  // R with zeros below its diagonal
-  target += gridDim.x;
-  if (ok) ok = chol_barrier(g, target);
-  if (ok) {
-    T* R = (T*)g.R;
-    for (int64_t e = blockIdx.x * (int64_t)QT + threadIdx.x; e < (int64_t)n * n;
-         e += (int64_t)gridDim.x * QT) {
-      const int r = (int)(e % n), c = (int)(e / n);
-      R[e] = r <= c ? A[r + ld * c] : T{};
-    }
-  }
   // the last block to leave makes the counters ready for the next launch
   __syncthreads();
   if (threadIdx.x == 0 && atomicAdd(&g.bar[1], 1u) == gridDim.x - 1) {
@@ -324,26 +315,39 @@ __global__ void unit_kernel(int n, typename Sc<CX>::T* X) {
     X[e] = e % n == e / n ? from_real(T{}, 1.0) : T{};
 }
 
-// E = G - 1 (G Hermitian): um = 1 - u, up = 1 + u with u the upper triangle of E and half its
-// diagonal; *worst = bits of max |E|
+// R = upper triangle of P, the diagonal real
+template <bool CX>
+__global__ void upper_kernel(int n, const typename Sc<CX>::T* P, typename Sc<CX>::T* R) {
+  using T = typename Sc<CX>::T;
+  chain_release();
+  chain_wait();
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)n * n;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    const int r = (int)(e % n), c = (int)(e / n);
+    T v = T{};
+    if (r <= c) v = P[e];
+    R[e] = r == c ? from_real(T{}, real_of(v)) : v;
+  }
+}
+
+// E = G - 1 (G Hermitian): um = 1 - u with u the upper triangle of E and half its diagonal;
+// *worst = bits of max |E|
 template <bool CX>
 __global__ void correction_kernel(int n, const typename Sc<CX>::T* __restrict__ G,
                                   typename Sc<CX>::T* __restrict__ um,
-                                  typename Sc<CX>::T* __restrict__ up,
                                   unsigned long long* worst) {
   using T = typename Sc<CX>::T;
   unsigned long long m = 0;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)n * n;
        e += (int64_t)gridDim.x * blockDim.x) {
     const int r = (int)(e % n), c = (int)(e / n);
-    T a = T{}, b = T{};
+    T a = T{};
     if (r == c) {
       const double d = real_of(G[e]) - 1.0;
       m = max(m, (unsigned long long)__double_as_longlong(d) & ~(1ull << 63));
       a = from_real(T{}, fma(-0.5, d, 1.0));
-      b = from_real(T{}, fma(0.5, d, 1.0));
     } else if (r < c) {
-      b = G[e];
+      const T b = G[e];
       if constexpr (CX) {
         m = max(m, (unsigned long long)__double_as_longlong(b.x) & ~(1ull << 63));
         m = max(m, (unsigned long long)__double_as_longlong(b.y) & ~(1ull << 63));
@@ -354,7 +358,6 @@ __global__ void correction_kernel(int n, const typename Sc<CX>::T* __restrict__ 
       }
     }
     um[e] = a;
-    up[e] = b;
   }
   for (int o = 16; o > 0; o >>= 1)
     m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -388,15 +391,13 @@ bool qr_gram(gb_ctx* ctx, int dtype, int64_t m, int64_t n, const void* M, void* 
   const bool cx = is_cplx(dtype);
   const size_t es = elem_size(dtype);
   const size_t nn = up256((size_t)n * n * es), mn = up256((size_t)m * n * es);
-  WorkBuf w(ctx, 256 + up256(NB * NB * es) + up256(2 * (size_t)n * n * es) + 3 * nn + 2 * mn);
+  WorkBuf w(ctx, 256 + up256(NB * NB * es) + up256(2 * (size_t)n * n * es) + nn + 2 * mn);
   if (!w.p) return false;
   unsigned long long* res = (unsigned long long*)w.p;  // [0] max |E|, [1] failed pivots (int)
   char* Z = w.p + 256;
   char* A = Z + up256(NB * NB * es);
   char* um = A + up256(2 * (size_t)n * n * es);
-  char* up = um + nn;
-  char* R1 = up + nn;
-  char* Q1 = R1 + nn;
+  char* Q1 = um + nn;
   char* Q2 = Q1 + mn;
   const cplx one{1, 0}, none{0, 0};
   const int sms = std::max(1, ctx->num_sms);
@@ -411,7 +412,6 @@ bool qr_gram(gb_ctx* ctx, int dtype, int64_t m, int64_t n, const void* M, void* 
   a.n = (int)n;
   a.A = A;
   a.Z = Z;
-  a.R = R1;
   a.fail = (int*)(res + 1);
   a.bar = (unsigned int*)((char*)ctx->d_status + 96);
   a.status = ctx->d_status;
@@ -427,21 +427,29 @@ bool qr_gram(gb_ctx* ctx, int dtype, int64_t m, int64_t n, const void* M, void* 
   // Q1 = A R1^-1 (the right half holds R1^-H)
   gemm_fp64(ctx, dtype, 'N', 'C', m, n, n, one, M, m, 0, X, n, 0, none, Q1, m, 0, 1);
   count_launch_n(ctx, 2);
-  // orthonormal to first order, until the second order is rounding
-  char *q = Q1, *qn = Q2, *r = R1;
+  // orthonormal to first order, until the second order is rounding: |E^2| <= (n max |E|)^2, which
+  // is to stay below n eps / 4
+  const double done = std::sqrt(0x1p-54 / (double)n);
+  char *q = Q1, *qn = Q2;
   for (int pass = 0; pass < 5; ++pass) {
     gemm_fp64(ctx, dtype, 'C', 'N', n, n, m, one, q, m, 0, q, m, 0, none, A, n, 0, 1);
     if (cx)
       correction_kernel<true><<<eb, 256, 0, ctx->stream>>>((int)n, (const double2*)A, (double2*)um,
-                                                           (double2*)up, res);
+                                                           res);
     else
       correction_kernel<false><<<eb, 256, 0, ctx->stream>>>((int)n, (const double*)A, (double*)um,
-                                                            (double*)up, res);
+                                                            res);
     GB_CHECK_CUDA(cudaGetLastError());
-    count_launch(ctx);
     // the outputs directly, in the hope that this pass is the last
     gemm_fp64(ctx, dtype, 'N', 'N', m, n, n, one, q, m, 0, um, n, 0, none, Q, m, 0, 1);
-    gemm_fp64(ctx, dtype, 'N', 'N', n, n, n, one, up, n, 0, r, n, 0, none, R, n, 0, 1);
+    gemm_fp64(ctx, dtype, 'C', 'N', n, n, m, one, Q, m, 0, M, m, 0, none, A, n, 0, 1);
+    if (cx)
+      launch_chained(upper_kernel<true>, dim3(eb), 256, 0, ctx->stream, 1, 1, (int)n,
+                     (const double2*)A, (double2*)R);
+    else
+      launch_chained(upper_kernel<false>, dim3(eb), 256, 0, ctx->stream, 1, 1, (int)n,
+                     (const double*)A, (double*)R);
+    count_launch_n(ctx, 2);
     double* host = host_results(ctx, 512);
     GB_CHECK_CUDA(cudaMemcpyAsync(host, res, 16, cudaMemcpyDeviceToHost, ctx->stream));
     GB_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -449,9 +457,8 @@ bool qr_gram(gb_ctx* ctx, int dtype, int64_t m, int64_t n, const void* M, void* 
     std::memcpy(&failed, host + 1, sizeof(int));
     const double worst = host[0];
     if (failed || !(worst < 0.1)) return false;
-    if (worst < 1e-9) return true;
+    if (worst <= done) return true;
     GB_CHECK_CUDA(cudaMemcpyAsync(qn, Q, (size_t)m * n * es, cudaMemcpyDeviceToDevice, ctx->stream));
-    GB_CHECK_CUDA(cudaMemcpyAsync(R1, R, (size_t)n * n * es, cudaMemcpyDeviceToDevice, ctx->stream));
     GB_CHECK_CUDA(cudaMemsetAsync(res, 0, 8, ctx->stream));
     std::swap(q, qn);
   }

@@ -106,3 +106,34 @@ def test_rank_deficient_scaled_and_non_finite(ctx):
                               - np.eye(30)) <= 8 * 30 * EPS
         assert np.all(np.abs(b - q.reshape(80, 30, order="F") @ r) <= 240 * EPS * np.abs(b).max())
     assert ctx.device_status() == 0
+
+
+def _factors(ctx, a):
+    """Positive QR of `a` (rows a multiple of two) and, from the LQ of its adjoint, again."""
+    m, n = a.shape
+    q, r = mpsgb.left_orth(mpsgb.DeviceTensor.from_numpy(
+        ctx, "mps", a.reshape(m // 2, 2, n, order="F")))
+    yield q.numpy().reshape(m, n, order="F"), r.numpy()
+    c, q = mpsgb.right_orth(mpsgb.DeviceTensor.from_numpy(
+        ctx, "mps", a.conj().T.reshape(n, 2, m // 2, order="F")))
+    yield q.numpy().reshape(-1, m, order="F").conj().T, c.numpy().conj().T
+
+
+@pytest.mark.parametrize("triangular", [False, True])
+@pytest.mark.parametrize("shape", [(200, 90), (512, 256)])  # FMA products, digit products
+@pytest.mark.parametrize("cx", [False, True])
+def test_condition_numbers_of_several_passes(ctx, cx, shape, triangular):
+    """Condition numbers of 1e6 to 1e9, where the factor of the Gram matrix needs from one to
+    several corrections or is given up: Q R = A throughout.  Also as a gauge step meets them, an
+    isometry times a triangular bond matrix."""
+    m, n = shape
+    rng = np.random.default_rng(m)
+    for cond in 1e6 * 2.0 ** np.arange(11):
+        a, _ = _matrix(rng, m, n, cx, cond)
+        if triangular:
+            a = _matrix(rng, m, n, cx, None)[0]
+            v = np.linalg.qr(_matrix(rng, n, n, cx, None)[0])[0]
+            a = np.linalg.qr(a)[0] @ np.linalg.qr(np.logspace(0, -np.log10(cond), n)[:, None] * v)[1]
+        for q, r in _factors(ctx, a):
+            _check(a, q, r, None)
+    assert ctx.device_status() == 0
