@@ -12,6 +12,11 @@
 // a residual of 2e-10 |A| at a condition number of 1e8, 2e-16 here.)  A matrix whose Gram matrix
 // has no Cholesky factor, or whose E exceeds 0.1, is left to the caller's Householder routine.
 //
+// The columns are first brought to one scale, by powers of two and therefore exactly.  Site
+// tensors have columns graded by Schmidt values, and the digits of the products hold a row of A
+// to 2^-55 of its largest entry: unscaled, a column 1e-8 of the largest is kept to 1e-9 of its
+// own norm (Householder and scaled columns: 1e-15), and E sees the grading as a condition.
+//
 // The products run as the plain-precision GEMMs (gemm_f64.cu).  gram_chol_kernel does the rest
 // in one cooperative launch: the Cholesky factor of G and its inverse, by eliminating [G | 1]
 // in block rows of 8.  Its chain is the 8 x 8 diagonal blocks (a scheduler issues an FP64 warp
@@ -315,9 +320,38 @@ __global__ void unit_kernel(int n, typename Sc<CX>::T* X) {
     X[e] = e % n == e / n ? from_real(T{}, 1.0) : T{};
 }
 
-// R = upper triangle of P, the diagonal real
+// As = A with column j scaled by 2^(1023 - ex[j]), ex[j] the largest biased exponent of its parts
+// (columns of zeros or with Inf or NaN: 2^0).  A block per column.  Bound by its latency (2 MB of
+// a 512 x 256 complex matrix).
 template <bool CX>
-__global__ void upper_kernel(int n, const typename Sc<CX>::T* P, typename Sc<CX>::T* R) {
+__global__ void __launch_bounds__(QT)
+    equilibrate_kernel(int64_t m, int64_t n, const double* A, double* As, int* ex) {
+  chain_release();
+  chain_wait();
+  __shared__ int most;
+  const int64_t len = CX ? 2 * m : m;  // reals of a column
+  for (int64_t j = blockIdx.x; j < n; j += gridDim.x) {
+    const double* a = A + j * len;
+    if (threadIdx.x == 0) most = 0;
+    __syncthreads();
+    int e = 0;
+    for (int64_t i = threadIdx.x; i < len; i += QT)
+      e = max(e, (__double2hiint(a[i]) >> 20) & 0x7ff);
+    e = __reduce_max_sync(0xffffffffu, e);
+    if (threadIdx.x % 32 == 0) atomicMax(&most, e);
+    __syncthreads();
+    e = most == 0 || most == 0x7ff ? 1023 : min(most, 2045);
+    const double s = __hiloint2double((2046 - e) << 20, 0);
+    for (int64_t i = threadIdx.x; i < len; i += QT) As[j * len + i] = a[i] * s;
+    if (threadIdx.x == 0) ex[j] = e;
+    __syncthreads();
+  }
+}
+
+// R = upper triangle of P, the columns scaled back, the diagonal real
+template <bool CX>
+__global__ void upper_kernel(int n, const typename Sc<CX>::T* P, const int* ex,
+                             typename Sc<CX>::T* R) {
   using T = typename Sc<CX>::T;
   chain_release();
   chain_wait();
@@ -325,7 +359,7 @@ __global__ void upper_kernel(int n, const typename Sc<CX>::T* P, typename Sc<CX>
        e += (int64_t)gridDim.x * blockDim.x) {
     const int r = (int)(e % n), c = (int)(e / n);
     T v = T{};
-    if (r <= c) v = P[e];
+    if (r <= c) v = times(P[e], __hiloint2double(ex[c] << 20, 0));
     R[e] = r == c ? from_real(T{}, real_of(v)) : v;
   }
 }
@@ -391,19 +425,25 @@ bool qr_gram(gb_ctx* ctx, int dtype, int64_t m, int64_t n, const void* M, void* 
   const bool cx = is_cplx(dtype);
   const size_t es = elem_size(dtype);
   const size_t nn = up256((size_t)n * n * es), mn = up256((size_t)m * n * es);
-  WorkBuf w(ctx, 256 + up256(NB * NB * es) + up256(2 * (size_t)n * n * es) + nn + 2 * mn);
+  WorkBuf w(ctx, 256 + up256(n * sizeof(int)) + up256(NB * NB * es) +
+                     up256(2 * (size_t)n * n * es) + nn + 3 * mn);
   if (!w.p) return false;
   unsigned long long* res = (unsigned long long*)w.p;  // [0] max |E|, [1] failed pivots (int)
-  char* Z = w.p + 256;
+  int* ex = (int*)(w.p + 256);
+  char* Z = w.p + 256 + up256(n * sizeof(int));
   char* A = Z + up256(NB * NB * es);
   char* um = A + up256(2 * (size_t)n * n * es);
-  char* Q1 = um + nn;
+  char* As = um + nn;
+  char* Q1 = As + mn;
   char* Q2 = Q1 + mn;
   const cplx one{1, 0}, none{0, 0};
   const int sms = std::max(1, ctx->num_sms);
   GB_CHECK_CUDA(cudaMemsetAsync(res, 0, 256, ctx->stream));
   const unsigned eb = (unsigned)std::min<int64_t>((n * n + 255) / 256, 4 * sms);
-  gemm_fp64(ctx, dtype, 'C', 'N', n, n, m, one, M, m, 0, M, m, 0, none, A, n, 0, 1);
+  launch_chained(cx ? equilibrate_kernel<true> : equilibrate_kernel<false>,
+                 dim3((unsigned)std::min<int64_t>(n, 8 * sms)), QT, 0, ctx->stream, 1, 1, m, n,
+                 (const double*)M, (double*)As, ex);
+  gemm_fp64(ctx, dtype, 'C', 'N', n, n, m, one, As, m, 0, As, m, 0, none, A, n, 0, 1);
   char* X = A + (size_t)n * n * es;
   if (cx) unit_kernel<true><<<eb, 256, 0, ctx->stream>>>((int)n, (double2*)X);
   else unit_kernel<false><<<eb, 256, 0, ctx->stream>>>((int)n, (double*)X);
@@ -425,8 +465,8 @@ bool qr_gram(gb_ctx* ctx, int dtype, int64_t m, int64_t n, const void* M, void* 
       cx ? (const void*)gram_chol_kernel<true> : (const void*)gram_chol_kernel<false>, dim3(blocks),
       dim3(QT), args, 0, ctx->stream));
   // Q1 = A R1^-1 (the right half holds R1^-H)
-  gemm_fp64(ctx, dtype, 'N', 'C', m, n, n, one, M, m, 0, X, n, 0, none, Q1, m, 0, 1);
-  count_launch_n(ctx, 2);
+  gemm_fp64(ctx, dtype, 'N', 'C', m, n, n, one, As, m, 0, X, n, 0, none, Q1, m, 0, 1);
+  count_launch_n(ctx, 3);
   // orthonormal to first order, until the second order is rounding: |E^2| <= (n max |E|)^2, which
   // is to stay below n eps / 4
   const double done = std::sqrt(0x1p-54 / (double)n);
@@ -442,13 +482,13 @@ bool qr_gram(gb_ctx* ctx, int dtype, int64_t m, int64_t n, const void* M, void* 
     GB_CHECK_CUDA(cudaGetLastError());
     // the outputs directly, in the hope that this pass is the last
     gemm_fp64(ctx, dtype, 'N', 'N', m, n, n, one, q, m, 0, um, n, 0, none, Q, m, 0, 1);
-    gemm_fp64(ctx, dtype, 'C', 'N', n, n, m, one, Q, m, 0, M, m, 0, none, A, n, 0, 1);
+    gemm_fp64(ctx, dtype, 'C', 'N', n, n, m, one, Q, m, 0, As, m, 0, none, A, n, 0, 1);
     if (cx)
       launch_chained(upper_kernel<true>, dim3(eb), 256, 0, ctx->stream, 1, 1, (int)n,
-                     (const double2*)A, (double2*)R);
+                     (const double2*)A, (const int*)ex, (double2*)R);
     else
       launch_chained(upper_kernel<false>, dim3(eb), 256, 0, ctx->stream, 1, 1, (int)n,
-                     (const double*)A, (double*)R);
+                     (const double*)A, (const int*)ex, (double*)R);
     count_launch_n(ctx, 2);
     double* host = host_results(ctx, 512);
     GB_CHECK_CUDA(cudaMemcpyAsync(host, res, 16, cudaMemcpyDeviceToHost, ctx->stream));

@@ -113,7 +113,7 @@ def _factors(ctx, a):
     m, n = a.shape
     q, r = mpsgb.left_orth(mpsgb.DeviceTensor.from_numpy(
         ctx, "mps", a.reshape(m // 2, 2, n, order="F")))
-    yield q.numpy().reshape(m, n, order="F"), r.numpy()
+    yield q.numpy().reshape(m, -1, order="F"), r.numpy()
     c, q = mpsgb.right_orth(mpsgb.DeviceTensor.from_numpy(
         ctx, "mps", a.conj().T.reshape(n, 2, m // 2, order="F")))
     yield q.numpy().reshape(-1, m, order="F").conj().T, c.numpy().conj().T
@@ -136,4 +136,33 @@ def test_condition_numbers_of_several_passes(ctx, cx, shape, triangular):
             a = np.linalg.qr(a)[0] @ np.linalg.qr(np.logspace(0, -np.log10(cond), n)[:, None] * v)[1]
         for q, r in _factors(ctx, a):
             _check(a, q, r, None)
+    assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("decades", [4, 8, 12])
+@pytest.mark.parametrize("shape", [(200, 90), (512, 256), (128, 300)])
+@pytest.mark.parametrize("cx", [False, True])
+def test_graded_columns(ctx, cx, shape, decades):
+    """Columns of very different norm, as a site tensor times its Schmidt values has them.  Each is
+    held to its own norm (a backward error of Householder's size per column), and Q is that of the
+    matrix without the grading.  Alone (rows), the grading of the rows changes nothing either."""
+    m, n = shape
+    rng = np.random.default_rng(m + decades)
+    a, cond = _matrix(rng, m, n, cx, None)
+    k = min(m, n)
+    if m < n:
+        s = np.linalg.svd(a[:, :m], compute_uv=False)
+        cond = s[0] / s[-1]
+    q0, _ = _ref(a)
+    d = np.logspace(0, -decades, n)[rng.permutation(n)]
+    b = a * d
+    q, r = next(_factors(ctx, b))
+    assert np.linalg.norm(q.conj().T @ q - np.eye(k)) <= 8 * n * EPS
+    assert np.all(np.linalg.norm(b - q @ r, axis=0) <= 8 * n * EPS * np.linalg.norm(b, axis=0))
+    assert np.linalg.norm(q - q0[:, :k]) <= 8 * n * EPS * cond
+    if m >= n:
+        c = np.logspace(0, -decades, m)[rng.permutation(m)][:, None] * a
+        for q, r in _factors(ctx, c):
+            assert np.linalg.norm(q.conj().T @ q - np.eye(k)) <= 8 * n * EPS
+            assert np.all(np.linalg.norm(c - q @ r, axis=0) <= 8 * n * EPS * np.linalg.norm(c, axis=0))
     assert ctx.device_status() == 0
