@@ -275,12 +275,11 @@ struct SmallPlan {
   bool ok = false;
 };
 SmallPlan gemm_small_plan(int sms, int64_t M, int64_t N, int64_t K, int64_t batch, bool cx);
-// y = x R + L x (+ y) of operators whose constants are cut into digits (R, Lp): x is M1 x K1 on the
+// y = x R + L x of operators whose constants are cut into digits (R, Lp): x is M1 x K1 on the
 // left of R and K2 x N2 on the right of L.  False (nothing done) when the digits do not fit.
 bool gemm_sliced_pair(gb_ctx* ctx, int dtype, const void* x, int64_t M1, int64_t N1, int64_t K1,
                       const Packed& R, const void* Rsrc, int64_t ldr, int64_t M2, int64_t N2,
-                      int64_t K2, const Packed& Lp, const void* Lsrc, int64_t ldl, bool accumulate,
-                      void* y);
+                      int64_t K2, const Packed& Lp, const void* Lsrc, int64_t ldl, void* y);
 // y = x R + L x (+ y) of a small operator in one launch; false: run them one by one
 bool gemm_small_dual(gb_ctx* ctx, int dtype, int64_t Ml, int64_t d, int64_t Nr, int64_t K1,
                      const void* R, int64_t ldr, int64_t K2, const void* L, int64_t ldl,
@@ -374,7 +373,7 @@ void pack_operand(gb_ctx* ctx, int dtype, int role, char op, int64_t M_or_N, int
                   int64_t nzero = 0);
 bool gemm_split_pair(gb_ctx* ctx, int dtype, int prec, const void* x, int64_t M1, int64_t N1,
                      int64_t K1, const Packed& R, int64_t M2, int64_t N2, int64_t K2,
-                     const Packed& Lp, bool accumulate, void* y);
+                     const Packed& Lp, void* y);
 // Skipping structurally zero work in mixpack_run: x is the output of a GEMM with an output
 // map (xmap, onc columns of 128 per row tile of 128); input i of the mix at (a, n) sits at
 // row a + roff[i], column coff[i] + n*xnM of that matrix.  prev: scratch of the packed

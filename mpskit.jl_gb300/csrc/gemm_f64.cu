@@ -1288,14 +1288,13 @@ bool gemm_fp64_sliced(gb_ctx* ctx, int dtype, char opA, char opB, int64_t M, int
   return true;
 }
 
-// y = x R + L x (+ y), x and the constants cut into digits: both products in one launch when
+// y = x R + L x, x and the constants cut into digits: both products in one launch when
 // together they leave fewer SMs idle than one after the other; their outputs meet by atomic adds of
-// two values, whose sum does not depend on the order.  An apply of two complex products of 128 x
+// two values on a cleared y, whose sum does not depend on the order (that of three would).  An apply of two complex products of 128 x
 // 256 x 256: 31.0 us one by one, 20.9 us; of 256 x 512 x 512: 58 and 49 us.
 bool gemm_sliced_pair(gb_ctx* ctx, int dtype, const void* x, int64_t M1, int64_t N1, int64_t K1,
                       const Packed& R, const void* Rsrc, int64_t ldr, int64_t M2, int64_t N2,
-                      int64_t K2, const Packed& Lp, const void* Lsrc, int64_t ldl, bool accumulate,
-                      void* y) {
+                      int64_t K2, const Packed& Lp, const void* Lsrc, int64_t ldl, void* y) {
   const bool cx = is_cplx(dtype);
   const int sms = std::max(1, ctx->num_sms);
   const int mt[2] = {(int)((M1 + 127) / 128), (int)((M2 + 127) / 128)};
@@ -1308,11 +1307,11 @@ bool gemm_sliced_pair(gb_ctx* ctx, int dtype, const void* x, int64_t M1, int64_t
   const bool together = p.clocks < p0.clocks + p1.clocks;
   const int64_t n = M1 * N1 * (cx ? 2 : 1);
   if (!slice_both(ctx, dtype, x, M1, K1, N2, K2, xa, xb, (double*)y,
-                  together && !accumulate ? n : 0))
+                  together ? n : 0))
     return false;
   if (!together)
     return gemm_fp64_sliced(ctx, dtype, 'N', 'N', M1, N1, K1, 1.0, x, M1, 0, Rsrc, ldr, 0,
-                            accumulate ? 1.0 : 0.0, y, M1, 0, 1, &xa, &R) &&
+                            0.0, y, M1, 0, 1, &xa, &R) &&
            gemm_fp64_sliced(ctx, dtype, 'N', 'N', M2, N2, K2, 1.0, Lsrc, ldl, 0, x, K2, 0, 1.0, y,
                             M2, 0, 1, &Lp, &xb);
   SGArgs g[2] = {sliced_args(ctx, dtype, 'N', 'N', M1, N1, K1, 1.0, x, M1, 0, Rsrc, ldr, 0, 1.0, y,

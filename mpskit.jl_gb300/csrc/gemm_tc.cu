@@ -1466,13 +1466,13 @@ void gemm_split(gb_ctx* ctx, int dtype, const Packed& A, const Packed& B, int64_
   }
 }
 
-// y = x R + L x (+ y) with packed constants: both products in one launch, a tile per CTA, when that
-// is done earlier than one after the other; their outputs meet by atomic adds of two values, whose
-// sum does not depend on the order.  False (nothing done) otherwise.  (tf32x3, complex 256 x 512 x
+// y = x R + L x with packed constants: both products in one launch, a tile per CTA, when that
+// is done earlier than one after the other; their outputs meet by atomic adds of two values on a
+// cleared y, whose sum does not depend on the order (that of three would).  False (nothing done) otherwise.  (tf32x3, complex 256 x 512 x
 // 512 and 512 x 256 x 512, an apply: 64.8 us one by one, 38.8 us.)
 bool gemm_split_pair(gb_ctx* ctx, int dtype, int prec, const void* x, int64_t M1, int64_t N1,
                      int64_t K1, const Packed& R, int64_t M2, int64_t N2, int64_t K2,
-                     const Packed& Lp, bool accumulate, void* y) {
+                     const Packed& Lp, void* y) {
   if (ctx->profiling || ctx->counting || ctx->gemm_bn || ctx->gemm_schedule == GB_SCHED_TILE ||
       !tc_available(ctx))
     return false;
@@ -1506,7 +1506,7 @@ bool gemm_split_pair(gb_ctx* ctx, int dtype, int prec, const void* x, int64_t M1
   void* da = scratch(ctx, SLOT_PACK_A, packed_bytes(M1, K1, cx, PACK_AS_A, 1, prec));
   void* db = scratch(ctx, SLOT_PACK_B, packed_bytes(N2, K2, cx, PACK_AS_B, 1, prec));
   pack_operand(ctx, dtype, PACK_AS_A, 'N', M1, K1, x, M1, 0, 1, xa, da, prec, (double*)y,
-               accumulate ? 0 : M1 * N1 * (cx ? 2 : 1));
+               M1 * N1 * (cx ? 2 : 1));
   pack_operand(ctx, dtype, PACK_AS_B, 'N', N2, K2, x, K2, 0, 1, xb, db, prec);
   load_encode();
   PLaunch<2> l{};

@@ -1983,29 +1983,42 @@ void heff_apply_raw(gb_heff* h, const void* x, void* y) {
            q.ldb == q.K && q.ldc == q.M && q.M % p.M == 0 && p.N == q.N * (q.M / p.M) &&
            p.M * p.K == q.K * q.N;
   };
+  // Such a pair in one launch adds up by atomics.  Two values give the same sum in either order,
+  // three do not, so y must hold nothing before: where a chain (AA, A) comes first in the list, the
+  // pair is launched ahead of it and the chain accumulates.
+  auto pair_launched = [&](const Step& s, const Step& q) {
+    if (h->prec != GB_PREC_FP64)
+      return s.hasPB && q.hasPA &&
+             gemm_split_pair(ctx, h->dtype, h->prec, x, s.M, s.N, s.K, s.pB, q.M, q.N, q.K, q.pA, y);
+    return !ctx->lane && s.hasPB && s.pB.slices && q.hasPA && q.pA.slices &&
+           gemm_sliced_pair(ctx, h->dtype, x, s.M, s.N, s.K, s.pB, s.cB, s.ldb, q.M, q.N, q.K, q.pA,
+                            q.cA, q.lda, y);
+  };
+  size_t pair = h->steps.size();  // first step of the pair that has run
+  for (size_t i = 0; i < h->steps.size() && !h->y_zero_first; ++i) {
+    if (!h->steps[i].is_gemm && h->steps[i].dst == S_Y) break;
+    if (!pair_of(i)) continue;
+    if (pair_launched(h->steps[i], h->steps[i + 1])) pair = i;
+    break;
+  }
+  const bool begun = pair < h->steps.size();
   for (size_t i = 0; i < h->steps.size(); ++i) {
     const Step& s = h->steps[i];
-    if (pair_of(i)) {
+    if (i == pair) {
+      ++i;
+      continue;
+    }
+    if (h->prec == GB_PREC_FP64 && pair_of(i)) {
       const Step& q = h->steps[i + 1];
-      if (h->prec != GB_PREC_FP64) {
-        if (s.hasPB && q.hasPA &&
-            gemm_split_pair(ctx, h->dtype, h->prec, x, s.M, s.N, s.K, s.pB, q.M, q.N, q.K, q.pA,
-                            s.accumulate, y)) {
-          ++i;
-          continue;
-        }
-      } else if (gemm_small_dual(ctx, h->dtype, s.M, q.M / s.M, q.N, s.K, s.cB, s.ldb, q.K, q.cA,
-                                 q.lda, x, s.accumulate, y) ||
-                 (!ctx->lane && s.hasPB && s.pB.slices && q.hasPA && q.pA.slices &&
-                  gemm_sliced_pair(ctx, h->dtype, x, s.M, s.N, s.K, s.pB, s.cB, s.ldb, q.M, q.N,
-                                   q.K, q.pA, q.cA, q.lda, s.accumulate, y))) {
+      if (gemm_small_dual(ctx, h->dtype, s.M, q.M / s.M, q.N, s.K, s.cB, s.ldb, q.K, q.cA, q.lda, x,
+                          s.accumulate, y)) {
         ++i;
         continue;
       }
     }
     if (s.is_gemm) {
       void* C = (void*)ptr(s.dst, nullptr);
-      double beta = s.accumulate ? 1.0 : 0.0;
+      double beta = s.accumulate || (begun && s.dst == S_Y) ? 1.0 : 0.0;
       const Packed* pB = s.hasPB ? &s.pB : nullptr;
       if (fused_t2 && s.t2_consumer) pB = &h->t2p;
       uint32_t* omap = (fused_t2 && s.dst == S_T1 && h->t1map) ? h->t1map : nullptr;

@@ -116,3 +116,55 @@ def test_both_products_in_one_launch(ctx, Dl, Dr, cx, prec):
     got = [o(x).numpy() for _ in range(3)]
     assert np.linalg.norm(got[0] - ref) <= 2.0 ** -14 * np.linalg.norm(ref)
     assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
+
+
+@pytest.mark.parametrize("kind", ["AC", "AC2"])
+@pytest.mark.parametrize("cx", [False, True])
+@pytest.mark.parametrize("prec", ["fp64", "bf16x3", "tf32x3"])
+def test_long_range_operator_repeats_bit_for_bit(ctx, kind, cx, prec):
+    """Decaying couplings: a chain over the continuing channels writes y beside the two products
+    that may share a launch.  The same bits from apply to apply, at sizes on both sides of the rule
+    that puts the two together, and the operator itself against einsum."""
+    dt = np.complex128 if cx else np.float64
+    sp, sz, eye = np.array([[0, 1], [0, 0]]), np.diag([0.5, -0.5]), np.eye(2)
+    W = np.zeros((5, 2, 2, 5))
+    W[0, :, :, 0] = W[4, :, :, 4] = eye
+    for c, (a, b) in enumerate(((sp, sp.T), (sp.T, sp), (sz, sz))):
+        W[0, :, :, 1 + c], W[1 + c, :, :, 1 + c], W[1 + c, :, :, 4] = a, 0.6 * eye, b
+    W = W.astype(dt)
+    dev = lambda k, a: mpsgb.DeviceTensor.from_numpy(ctx, k, a)
+    for D in ((130, 200, 256) if kind == "AC" else (72, 100, 150)):
+        rng = np.random.default_rng(D)
+        rand = lambda *s: (rng.standard_normal(s) + (1j * rng.standard_normal(s) if cx else 0))
+        GL, GR = rand(D, 5, D).astype(dt), rand(D, 5, D).astype(dt)
+        GL[:, 0, :] = GR[:, -1, :] = np.eye(D)
+        Wd = dev("mpo", W)
+        if kind == "AC":
+            x = rand(D, 2, D)
+            op = mpsgb.DerivativeOperator(ctx, mpsgb._lib.GB_HEFF_AC, dev("gl", GL), Wd, None,
+                                          dev("gr", GR), mpsgb.GB300Backend(prec))
+            ref = np.einsum("bwk,kta->bwta", GL, x, optimize=True)
+            ref = np.einsum("bwta,wstv->bsva", ref, W, optimize=True)
+            ref = np.einsum("bsva,avc->bsc", ref, GR, optimize=True)
+            xd = dev("mps", x)
+        else:
+            x = rand(D, 2, D, 2)
+            op = mpsgb.DerivativeOperator(ctx, mpsgb._lib.GB_HEFF_AC2, dev("gl", GL), Wd, Wd,
+                                          dev("gr", GR), mpsgb.GB300Backend(prec))
+            ref = np.einsum("bwk,ktau->bwtau", GL, x, optimize=True)
+            ref = np.einsum("bwtau,wstv->bsvau", ref, W, optimize=True)
+            ref = np.einsum("bsvau,vzuq->bsqza", ref, W, optimize=True)
+            ref = np.einsum("bsqza,aqc->bscz", ref, GR, optimize=True)
+            xd = dev("ac2", x)
+        got = [op(xd).numpy() for _ in range(25)]
+        if prec == "fp64":
+            assert np.linalg.norm(got[0] - ref) <= 1e-14 * np.linalg.norm(ref)
+        else:  # the products one by one (a fixed tile width): the same addends, summed in FP64
+            ctx.set_gemm_schedule("grouped", 128)
+            try:
+                apart = op(xd).numpy()
+            finally:
+                ctx.set_gemm_schedule("grouped", 0)
+            assert np.linalg.norm(got[0] - apart) <= 1e-15 * np.linalg.norm(ref)
+        for g in got[1:]:
+            assert np.array_equal(got[0], g)
