@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "../../include/mpsgb.h"
+#include "device_once.h"
 
 namespace gb {
 

@@ -1135,8 +1135,8 @@ template <int BN, int PRODUCTS>
 static void launch_sliced(gb_ctx* ctx, const Packed* const* a, const Packed* const* b,
                           const SGArgs* g, int64_t batch) {
   using S = SGShape<BN>;
-  static std::once_flag once;  // contexts may launch from several host threads
-  std::call_once(once, [] {
+  static DeviceOnce once;
+  once(ctx->device, [] {
     GB_CHECK_CUDA(cudaFuncSetAttribute(gemm_sliced_kernel<BN, PRODUCTS>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM));
   });

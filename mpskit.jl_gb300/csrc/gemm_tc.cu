@@ -1325,8 +1325,8 @@ static PArgs persistent_args(gb_ctx* ctx, const Packed& A, const Packed& B, int6
 template <int BN, int ST, bool TF, int PRODUCTS>
 static void persistent_launch(gb_ctx* ctx, unsigned grid, const PLaunch<PRODUCTS>& l) {
   constexpr int SM = persistent_smem<BN, ST>();
-  static std::once_flag once;  // contexts may launch from several host threads
-  std::call_once(once, [] {
+  static DeviceOnce once;
+  once(ctx->device, [] {
     GB_CHECK_CUDA(cudaFuncSetAttribute(gemm_bf16x3_persistent<BN, ST, TF, PRODUCTS>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, SM));
   });
@@ -1360,8 +1360,8 @@ void gemm_split(gb_ctx* ctx, int dtype, const Packed& A, const Packed& B, int64_
   GB_REQUIRE(A.Kp % A.bk == 0, "gemm_split: Kp alignment");
   const bool tf32 = A.esz == 4;
   load_encode();
-  static std::once_flag attr_once;  // contexts may launch from several host threads
-  std::call_once(attr_once, [] {
+  static DeviceOnce attr_once;
+  attr_once(ctx->device, [] {
     GB_CHECK_CUDA(cudaFuncSetAttribute(gemm_bf16x3_kernel,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        TC_SMEM_BYTES));

@@ -643,8 +643,8 @@ void gmix_staged_run(gb_ctx* ctx, const MixDev& m, const GMixStaged& g, const GM
   GB_REQUIRE(g.NL <= 65535 && m.N <= 0x7fffffff, "grouped mix: grid too large");
   dim3 grid((unsigned)m.N, (unsigned)g.NL);
   const int64_t plane = out.rows * out.kmax;
-  static std::once_flag attr_once;
-  std::call_once(attr_once, [] {
+  static DeviceOnce attr_once;
+  attr_once(ctx->device, [] {
     cudaFuncSetAttribute(gmix_staged_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          96 * 1024);
     cudaFuncSetAttribute(gmix_staged_kernel<__nv_bfloat16>,
@@ -1149,8 +1149,8 @@ void gemm_grouped(gb_ctx* ctx, const GPlan& p, const GOperand& A, const GOperand
 #define GB_GROUPED(ST_, TF_)                                                                  \
   do {                                                                                        \
     constexpr int SM = grouped_smem<ST_>();                                                   \
-    static std::once_flag once;                                                               \
-    std::call_once(once, [] {                                                                 \
+    static DeviceOnce once;                                                                   \
+    once(ctx->device, [] {                                                                    \
       GB_CHECK_CUDA(cudaFuncSetAttribute(gemm_grouped_kernel<ST_, TF_>,                       \
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, SM));   \
     });                                                                                       \

@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <map>
 #include <mutex>
 
 #include "gb_common.h"
@@ -476,11 +477,12 @@ __global__ void __launch_bounds__(OT) krylov_combine_kernel(CombineArgs a) {
 }
 
 // clusters of more than eight blocks need a device that grants them
-bool orth_cluster_fits() {
-  static std::once_flag once;
-  static bool fits = false;
-  std::call_once(once, [] {
-    fits = true;
+bool orth_cluster_fits(int device) {
+  static DeviceOnce once;
+  static std::mutex mu;
+  static std::map<int, bool> granted;
+  once(device, [device] {
+    bool fits = true;
     auto allow = [&](const void* kernel) {
       if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
           cudaSuccess) {
@@ -504,8 +506,11 @@ bool orth_cluster_fits() {
     allow((const void*)krylov_orth_kernel<false>);
     allow((const void*)krylov_combine_kernel<true>);
     allow((const void*)krylov_combine_kernel<false>);
+    std::lock_guard<std::mutex> lk(mu);
+    granted[device] = fits;
   });
-  return fits;
+  std::lock_guard<std::mutex> lk(mu);
+  return granted[device];
 }
 
 // blocks of a launch: one per SM at most, pieces of 64 entries at least.  Up to 128 complex (256
@@ -517,7 +522,7 @@ constexpr int OCLUSTER = 16;
 int orth_blocks(gb_ctx* ctx, int dtype, int64_t n, bool* cluster) {
   const int64_t most = std::max(1, ctx->num_sms);
   const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(most, (n + 63) / 64));
-  *cluster = blocks > 1 && n <= OCLUSTER * (is_cplx(dtype) ? 128 : 256) && orth_cluster_fits();
+  *cluster = blocks > 1 && n <= OCLUSTER * (is_cplx(dtype) ? 128 : 256) && orth_cluster_fits(ctx->device);
   return (int)(*cluster ? std::min<int64_t>(blocks, OCLUSTER) : blocks);
 }
 
@@ -587,8 +592,8 @@ void krylov_orth_start(gb_ctx* ctx, int dtype, int64_t n, int k, bool predict, c
   g.out = host_results(ctx, OSLOT * ORTH_SLOTS) + OSLOT * slot;
   if (!ctx->orth_done[slot])
     GB_CHECK_CUDA(cudaEventCreateWithFlags(&ctx->orth_done[slot], cudaEventDisableTiming));
-  static std::once_flag once;  // contexts may launch from several host threads
-  std::call_once(once, [] {
+  static DeviceOnce once;
+  once(ctx->device, [] {
     GB_CHECK_CUDA(cudaFuncSetAttribute(krylov_orth_kernel<true>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OPIECE));
     GB_CHECK_CUDA(cudaFuncSetAttribute(krylov_orth_kernel<false>,
