@@ -54,6 +54,7 @@ struct OrthArgs {
                    // write those of the next pass while another still adds this one's
   double* coef;    // [OKMAX + 1] complex sums
   double* out;     // pinned host: k projections (complex), then the norm
+  double* gave_up; // pinned host: set by a block whose wait ran out (null: nobody reads it)
   unsigned int* bar;  // [0] arrivals, [1] blocks that have left
   int* status;
   unsigned long long wait_ns;
@@ -416,6 +417,14 @@ __global__ void __launch_bounds__(OT, 1) krylov_orth_kernel(OrthArgs g) {
     __syncthreads();
     if (last) break;
   }
+  if (!ok) {
+    // any block may give up, and the others may not notice: the host is told beside the numbers
+    if (tid == 0) {
+      *g.gave_up = 1.0;
+      sleft = __longlong_as_double(0x7ff8000000000000ll);
+    }
+    __syncthreads();
+  }
   if (blockIdx.x == 0) {
     for (int j = tid; j < g.k; j += OT) ((double2*)g.out)[j] = sh[j];
     if (tid == 0) {
@@ -460,18 +469,17 @@ __global__ void __launch_bounds__(OT) krylov_combine_kernel(CombineArgs a) {
     __shared__ double2 sred[DOT_SUMS];
     block_dots<CPLX>(g, (const T*)nullptr, src, c0, len, 0, sred);
     __shared__ double sinv;
-    if (all_sums<CPLX>(g, 1, sc, target)) {
-      if (threadIdx.x == 0) {
-        const double nrm = sqrt(sc[0].x);
-        sinv = 1.0 / nrm;
-        if (blockIdx.x == 0 && g.out) {
-          g.out[0] = nrm;
-        }
-      }
-      __syncthreads();
-      const double inv = sinv;
-      for (int i = threadIdx.x; i < len; i += OT) dst[i] = scaled(src[i], inv);
+    const bool ok = all_sums<CPLX>(g, 1, sc, target);
+    if (threadIdx.x == 0) {
+      // NaN where the wait ran out: a piece without its norm must not pass for a result
+      const double nrm = ok ? sqrt(sc[0].x) : __longlong_as_double(0x7ff8000000000000ll);
+      sinv = 1.0 / nrm;
+      if (blockIdx.x == 0 && g.out) g.out[0] = nrm;
+      if (!ok && g.gave_up) *g.gave_up = 1.0;
     }
+    __syncthreads();
+    const double inv = sinv;
+    for (int i = threadIdx.x; i < len; i += OT) dst[i] = scaled(src[i], inv);
     grid_leave(g);
   }
 }
@@ -570,7 +578,8 @@ double* host_results(gb_ctx* ctx, size_t elems) {
 
 bool krylov_orth_fits(int k) { return k <= OKMAX; }
 
-constexpr size_t OSLOT = 2 * (OKMAX + 1) + 2;  // doubles of one step's results
+// doubles of one step's results; the last one: a block gave up
+constexpr size_t OSLOT = 2 * (OKMAX + 1) + 2;
 
 void krylov_orth_start(gb_ctx* ctx, int dtype, int64_t n, int k, bool predict, const void* V,
                        void* w, void* vnext, int slot) {
@@ -590,6 +599,8 @@ void krylov_orth_start(gb_ctx* ctx, int dtype, int64_t n, int k, bool predict, c
   const size_t bytes = (size_t)per * elem_size(dtype);
   g.in_smem = bytes <= OPIECE;
   g.out = host_results(ctx, OSLOT * ORTH_SLOTS) + OSLOT * slot;
+  g.gave_up = g.out + OSLOT - 1;
+  *g.gave_up = 0.0;
   if (!ctx->orth_done[slot])
     GB_CHECK_CUDA(cudaEventCreateWithFlags(&ctx->orth_done[slot], cudaEventDisableTiming));
   static DeviceOnce once;
@@ -607,6 +618,7 @@ void krylov_orth_start(gb_ctx* ctx, int dtype, int64_t n, int k, bool predict, c
 void krylov_orth_wait(gb_ctx* ctx, int k, int slot, cplx* h, double* norm) {
   GB_CHECK_CUDA(cudaEventSynchronize(ctx->orth_done[slot]));
   const double* out = ctx->h_pinned + OSLOT * slot;
+  if (out[OSLOT - 1] != 0.0) throw Error(GB_ERR_TIMEOUT, "Krylov step: a device wait ran out");
   for (int j = 0; j < k; ++j) h[j] = cplx{out[2 * j], out[2 * j + 1]};
   *norm = out[2 * k];
 }
@@ -633,6 +645,10 @@ void krylov_combine(gb_ctx* ctx, int dtype, int64_t n, int k, const void* V, con
   a.g.w = (double*)src;
   a.g.vnext = (double*)dst;
   a.g.out = norm ? host_results(ctx, OSLOT * ORTH_SLOTS) : nullptr;
+  if (norm) {
+    a.g.gave_up = a.g.out + OSLOT - 1;
+    *a.g.gave_up = 0.0;
+  }
   a.normalize = normalize;
   for (int j = 0; j < k; ++j) {
     a.c[2 * j] = coef[j].re;
@@ -642,6 +658,7 @@ void krylov_combine(gb_ctx* ctx, int dtype, int64_t n, int k, const void* V, con
               blocks, cluster, 0, a);
   if (norm) {
     GB_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (*a.g.gave_up != 0.0) throw Error(GB_ERR_TIMEOUT, "Krylov vector: a device wait ran out");
     *norm = a.g.out[0];
   }
 }

@@ -100,7 +100,7 @@ struct CholArgs {
   void* A;      // n x 2n column-major: [G | 1] on entry (G: upper triangle), R^-H in the right
                 // half on exit
   void* Z;      // NB x NB: inverse of the current diagonal block's (lower) factor
-  int* fail;    // set when a pivot is not positive
+  int* fail;    // set when a pivot is not positive, or when a wait ran out
   unsigned int* bar;
   int* status;
   unsigned long long wait_ns;
@@ -302,6 +302,7 @@ __global__ void __launch_bounds__(QT, 1) gram_chol_kernel(CholArgs g) {
       }
     }
   }
+  if (!ok && threadIdx.x == 0) atomicExch(g.fail, 1);
   // the last block to leave makes the counters ready for the next launch
   __syncthreads();
   if (threadIdx.x == 0 && atomicAdd(&g.bar[1], 1u) == gridDim.x - 1) {

@@ -125,3 +125,81 @@ def test_forced_non_convergence_is_not_an_error():
     assert np.isfinite(val)
     # the returned vector is the normalised best Ritz vector
     assert abs(vec.norm() - 1.0) < 1e-12
+
+
+def _until_timeout(ctx, call):
+    """Run `call` with the bound at zero until the status word says that a wait ran out (a grid
+    barrier may be passed before the clock ticks)."""
+    ctx.synchronize()
+    ctx.set_wait_bound(0.0)
+    try:
+        for _ in range(50):
+            out = call()
+            ctx.synchronize()
+            if ctx.device_status() == L.GB_ERR_TIMEOUT:
+                return out
+    finally:
+        ctx.set_wait_bound(2.0)
+    pytest.fail("no wait ran out")
+
+
+@pytest.mark.parametrize("h,K,N", [(160, 320, 200),   # splits share a tile through a cluster
+                                   (3000, 130, 900)])  # a tile per CTA, wide tiles
+def test_wait_timeout_in_the_digit_products(h, K, N):
+    """The plain-precision products on the tensor cores: reported, and right again afterwards."""
+    ctx = mpsgb.Context(0)
+    rng = np.random.default_rng(K)
+    A, B = rng.standard_normal((h, 2, K)), rng.standard_normal((K, N))
+    a = mpsgb.DeviceTensor.from_numpy(ctx, "mps", A)
+    b = mpsgb.DeviceTensor.from_numpy(ctx, "bond", B)
+    _until_timeout(ctx, lambda: mpsgb.states.mul_tail(a, b))
+    out = mpsgb.states.mul_tail(a, b).numpy()
+    ref = np.tensordot(A, B, axes=(2, 0))
+    assert np.linalg.norm(out - ref) <= 1e-14 * np.linalg.norm(ref)
+    assert ctx.device_status() == 0
+
+
+def test_wait_timeout_in_a_krylov_step():
+    """The grid barrier of the orthogonalisation: an error at once (no norm is made up), and the
+    same context orthogonalises correctly afterwards."""
+    import ctypes
+    ctx = mpsgb.Context(0)
+    n, k = 400001, 5  # every block, two barriers a pass
+    rng = np.random.default_rng(1)
+    V, w = np.linalg.qr(rng.standard_normal((n, k)))[0], rng.standard_normal(n)
+    basis = mpsgb.DeviceTensor.from_numpy(ctx, "generic", V)
+
+    def call():
+        x = mpsgb.DeviceTensor.from_numpy(ctx, "generic", w)
+        h = np.zeros(2 * k)
+        rc = L.lib().gb_basis_orthogonalize(ctx.handle, basis.handle, k, x.handle,
+                                            h.ctypes.data_as(ctypes.POINTER(ctypes.c_double)))
+        return rc, x, h
+
+    rc, _, _ = _until_timeout(ctx, call)
+    assert rc == L.GB_ERR_TIMEOUT
+    rc, x, h = call()
+    assert rc == 0 and ctx.device_status() == 0
+    ref = w - V @ (V.T @ w)
+    assert np.linalg.norm(x.numpy() - ref) <= 1e-13 * np.linalg.norm(ref)
+    assert np.linalg.norm(h[0::2] - V.T @ w) <= 1e-13 * np.linalg.norm(w)
+
+
+def test_wait_timeout_in_the_positive_qr():
+    """The grid barrier of the Cholesky factorisation: the factors come from the Householder
+    routine, and the status word tells."""
+    ctx = mpsgb.Context(0)
+    rng = np.random.default_rng(2)
+    a = rng.standard_normal((64, 33))
+    t = mpsgb.DeviceTensor.from_numpy(ctx, "mps", a.reshape(32, 2, 33, order="F"))
+
+    def check(out):
+        q, r = (v.numpy() for v in out)
+        q = q.reshape(64, 33, order="F")
+        assert np.linalg.norm(q.T @ q - np.eye(33)) <= 1e-13
+        assert np.linalg.norm(a - q @ r) <= 1e-13 * np.linalg.norm(a)
+        assert np.all(np.diagonal(r) > 0)
+
+    check(_until_timeout(ctx, lambda: mpsgb.left_orth(t)))
+    check(mpsgb.left_orth(t))
+    assert ctx.device_status() == 0
