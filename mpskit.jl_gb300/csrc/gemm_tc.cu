@@ -855,8 +855,12 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = (uint64_t*)(smem + STAGES * STAGE_BYTES);
-  uint64_t* full = bars;                        // [STAGES]  TMA -> MMA
-  uint64_t* empty = full + STAGES;              // [STAGES]  MMA -> TMA
+  // [STAGES] each, TMA -> MMA: the two producers' barriers are apart, so that one that gives up
+  // waits for its own copies alone (on a common one it would wait for the other's arrivals too,
+  // which may never come: 2 s of the drain's bound a stage, 26 s in all, for a wait that ran out)
+  uint64_t* fullA = bars;
+  uint64_t* fullB = fullA + STAGES;
+  uint64_t* empty = fullB + STAGES;             // [STAGES]  MMA -> TMA
   uint64_t* tfull = empty + STAGES;             // [2]       MMA -> epilogue
   uint64_t* tempty = tfull + 2;                 // [2]       epilogue -> MMA
   uint64_t* sfull = tempty + 2;                 // [RING]    producer -> consumers
@@ -871,7 +875,8 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
-      mbar_init(smem_u32(&full[s]), 2);  // both producers
+      mbar_init(smem_u32(&fullA[s]), 1);
+      mbar_init(smem_u32(&fullB[s]), 1);
       mbar_init(smem_u32(&empty[s]), 1);
     }
     for (int b = 0; b < 2; ++b) {
@@ -932,7 +937,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
     return true;
   };
   // drain copies still in flight before this CTA may exit
-  auto drain = [&](uint32_t issued) {
+  auto drain = [&](uint64_t* full, uint32_t issued) {
     for (uint32_t it = issued > (uint32_t)STAGES ? issued - STAGES : 0; it < issued; ++it)
       mbar_wait_bounded(smem_u32(&full[it % STAGES]), (it / STAGES) & 1, args.status,
                         DRAIN_WAIT_NS);
@@ -1011,12 +1016,12 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
       const int64_t m0 = (int64_t)mi * TC_BM;
       const int za0 = (args.batchA > 1 ? z : 0) * 2;
       ok = produce(mi, ni, z, g, [&](int s, int kb, int planeA, int) {
-        const uint32_t fb = smem_u32(&full[s]);
+        const uint32_t fb = smem_u32(&fullA[s]);
         mbar_expect_tx(fb, A_BYTES);
         tma_load_3d(smem_u32(smem + s * STAGE_BYTES), &mapA, fb, kb * BKE, (int)m0, za0 + planeA);
       });
     }
-    if (!ok) drain(g);
+    if (!ok) drain(fullA, g);
   } else if (warp == 6 && elect_one()) {
     // ---------------- producer of B
     uint32_t g = 0;
@@ -1033,13 +1038,13 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
       const int ni = r / args.mt, mi = r - ni * args.mt;
       const int n0 = ni * BN, zb0 = (args.batchB > 1 ? z : 0) * 2;
       ok = produce(mi, ni, z, g, [&](int s, int kb, int, int planeB) {
-        const uint32_t fb = smem_u32(&full[s]);
+        const uint32_t fb = smem_u32(&fullB[s]);
         mbar_expect_tx(fb, B_BYTES);
         tma_load_3d(smem_u32(smem + s * STAGE_BYTES) + A_BYTES, &mapB, fb, kb * BKE, n0,
                     zb0 + planeB);
       });
     }
-    if (!ok) drain(g);
+    if (!ok) drain(fullB, g);
   } else if (warp == 1 && elect_one()) {
     // ---------------- MMA issuer
     const uint32_t idesc = TF32 ? idesc_tf32(TC_BM, BN) : idesc_bf16(TC_BM, BN);
@@ -1061,7 +1066,8 @@ __global__ void __launch_bounds__(PS_THREADS, 1)
       const int total = 3 * nk;
       for (int it = 0; it < total; ++it) {
         const int s = g % STAGES;
-        ok = mbar_wait_bounded(smem_u32(&full[s]), (g / STAGES) & 1, args.status, args.wait_ns);
+        ok = mbar_wait_bounded(smem_u32(&fullA[s]), (g / STAGES) & 1, args.status, args.wait_ns) &&
+             mbar_wait_bounded(smem_u32(&fullB[s]), (g / STAGES) & 1, args.status, args.wait_ns);
         if (!ok) break;
         tc_fence_after();
         const uint32_t sa = smem_u32(smem + s * STAGE_BYTES);

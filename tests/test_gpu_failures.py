@@ -203,3 +203,25 @@ def test_wait_timeout_in_the_positive_qr():
     check(_until_timeout(ctx, lambda: mpsgb.left_orth(t)))
     check(mpsgb.left_orth(t))
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("prec", ["bf16x3", "tf32x3"])
+def test_wait_timeout_leaves_at_once(prec):
+    """A kernel whose wait runs out waits only for copies and MMAs of its own that are in flight,
+    microseconds: well below the two seconds that bound such a wait."""
+    import time
+    ctx = mpsgb.Context(0)
+    op, x, keep = _operator(ctx, prec)
+    xd = mpsgb.DeviceTensor.from_numpy(ctx, "ac2", x)
+    ref = op(xd).numpy()
+    ctx.set_wait_bound(0.0)
+    try:
+        t0 = time.perf_counter()
+        op(xd)
+        ctx.synchronize()
+        spent = time.perf_counter() - t0
+        assert ctx.device_status() == L.GB_ERR_TIMEOUT
+    finally:
+        ctx.set_wait_bound(2.0)
+    assert spent < 1.0
+    assert np.array_equal(op(xd).numpy(), ref)
