@@ -23,6 +23,7 @@
 #include <map>
 #include <sstream>
 
+#include "digit_budget.h"
 #include "gb_common.h"
 #include "tc_ptx.cuh"
 #include "grouped.h"
@@ -276,30 +277,88 @@ static void prepare_t2p(gb_heff* h) {
   h->t2p_ready = true;
 }
 
+// Digits of the operator's own constants, cut once for all applications (an environment that a
+// term reads in place may be written to between applications): bytes of either operand of a step,
+// zero where it keeps none.
+struct DigitBytes {
+  size_t a = 0, b = 0;
+};
+static DigitBytes digit_bytes(gb_heff* h, const Step& s) {
+  DigitBytes n;
+  if (!s.is_gemm || s.hasPA || s.hasPB ||
+      !gemm_sliced_wanted(h->ctx, h->dtype, s.M, s.N, s.K, 1, F64_SLICED_MIN_MAC_CUT))
+    return n;
+  auto own = [h](const void* p) {
+    return std::find(h->owned.begin(), h->owned.end(), (void*)p) != h->owned.end();
+  };
+  const bool cx = is_cplx(h->dtype);
+  if (s.srcA == S_CONST && own(s.cA)) n.a = sliced_bytes(s.M, s.K, cx, PACK_AS_A, 1);
+  if (s.srcB == S_CONST && own(s.cB)) n.b = sliced_bytes(s.N, s.K, cx, PACK_AS_B, 1);
+  return n;
+}
+
+// whether the digits of all its constants leave the operator's solves their memory
+static bool keep_digits(gb_heff* h) {
+  gb_ctx* ctx = h->ctx;
+  uint64_t bytes = 0;
+  for (const auto& s : h->steps) {
+    const DigitBytes n = digit_bytes(h, s);
+    bytes += n.a + n.b;
+  }
+  if (bytes <= DIGITS_SMALL) return true;
+  const size_t es = elem_size(h->dtype);
+  uint64_t need = DIGITS_VECTORS * (uint64_t)h->xnumel * es;
+  uint64_t held = 0;
+  for (int slot : {SLOT_KRYLOV, SLOT_KRYLOV_W, SLOT_TMP, SLOT_PACK_A, SLOT_PACK_B})
+    held += ctx->scratch[slot].bytes;
+  need = need > held ? need - held : 0;
+  if (!h->t2) need += (uint64_t)h->t2_elems * es;
+  size_t free_bytes = 0, total = 0;
+  GB_CHECK_CUDA(cudaMemGetInfo(&free_bytes, &total));
+  uint64_t reserved = 0, used = 0;
+  cudaMemPool_t pool;
+  if (cudaDeviceGetDefaultMemPool(&pool, ctx->device) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess) {
+    reserved = reserved > used ? reserved - used : 0;
+  } else {
+    cudaGetLastError();
+    reserved = 0;
+  }
+  return digits_affordable(bytes, need, free_bytes, reserved);
+}
+
+// the digits back to the pool (a change of precision: another set would be cut on the way back)
+static void drop_digits(gb_heff* h) {
+  auto drop = [h](Packed& p) {
+    if (!p.slices) return;
+    auto it = std::find(h->owned.begin(), h->owned.end(), p.data);
+    if (it != h->owned.end()) {
+      cudaFreeAsync(p.data, h->ctx->stream);
+      h->owned.erase(it);
+    }
+    p = Packed();
+  };
+  for (auto& s : h->steps) {
+    if (s.hasPA) drop(s.pA);
+    if (s.hasPB) drop(s.pB);
+  }
+}
+
 static void prepack(gb_heff* h, Step& s) {
   gb_ctx* ctx = h->ctx;
   if (h->prec == GB_PREC_FP64) {
-    // digits of the operator's own constants, cut once for all applications (an environment
-    // that a term reads in place may be written to between applications)
-    auto own = [h](const void* p) {
-      return std::find(h->owned.begin(), h->owned.end(), (void*)p) != h->owned.end();
-    };
-    if (s.hasPA || s.hasPB ||
-        !gemm_sliced_wanted(ctx, h->dtype, s.M, s.N, s.K, 1, F64_SLICED_MIN_MAC_CUT))
-      return;
-    const bool cx = is_cplx(h->dtype);
-    if (s.srcA == S_CONST && own(s.cA)) {
-      if (void* d = try_dalloc(h, sliced_bytes(s.M, s.K, cx, PACK_AS_A, 1))) {
+    const DigitBytes want = digit_bytes(h, s);
+    if (want.a)
+      if (void* d = try_dalloc(h, want.a)) {
         slice_operand(ctx, h->dtype, PACK_AS_A, s.opA, s.M, s.K, s.cA, s.lda, 0, 1, s.pA, d);
         s.hasPA = true;
       }
-    }
-    if (s.srcB == S_CONST && own(s.cB)) {
-      if (void* d = try_dalloc(h, sliced_bytes(s.N, s.K, cx, PACK_AS_B, 1))) {
+    if (want.b)
+      if (void* d = try_dalloc(h, want.b)) {
         slice_operand(ctx, h->dtype, PACK_AS_B, s.opB, s.N, s.K, s.cB, s.ldb, 0, 1, s.pB, d);
         s.hasPB = true;
       }
-    }
     return;
   }
   prepare_t2p(h);
@@ -1930,8 +1989,9 @@ static void heff_apply_grouped(gb_heff* h, const void* x, void* y) {
 
 static void ensure_prepacked(gb_heff* h) {
   if (h->prepacked) return;
-  for (auto& st : h->steps)
-    if (st.is_gemm) prepack(h, st);
+  if (h->prec != GB_PREC_FP64 || keep_digits(h))
+    for (auto& st : h->steps)
+      if (st.is_gemm) prepack(h, st);
   h->prepacked = true;
 }
 
@@ -1940,7 +2000,8 @@ void heff_set_precision(gb_heff* h, int prec) {
              "heff: precision");
   if (prec != h->prec) {
     // packed constants and the packed T2 follow the plane type; repack on change (the old
-    // buffers stay owned by the operator until it is freed)
+    // planes stay owned by the operator until it is freed, digits go back)
+    drop_digits(h);
     for (auto& s : h->steps) s.hasPA = s.hasPB = false;
     h->t2p_ready = false;
     h->prepacked = false;
