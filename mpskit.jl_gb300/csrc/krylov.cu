@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "gb_common.h"
+#include "tridiag_eig.h"
 
 namespace gb {
 
@@ -86,102 +87,6 @@ void sym_eig(int n, const std::vector<double>& Ain, std::vector<double>& D,
     D[j] = A[idx[j] * n + idx[j]];
     for (int i = 0; i < n; ++i) U[i * n + j] = Ut[idx[j] * n + i];
   }
-}
-
-// The same by Householder tridiagonalisation and the implicit QL iteration (Golub & Van Loan,
-// Matrix Computations, sections 8.3-8.4), for callers that need no particular sign of the
-// eigenvectors: D ascending and, for the rows i0..n-1 of the eigenvector matrix only,
-// Z[(i - i0) * n + j].  With the last row alone a convergence test costs 4/3 n^3 instead of the
-// ~50 n^3 of the Jacobi sweeps.  False if an eigenvalue does not converge.
-static bool sym_eig_rows(int n, const std::vector<double>& Ain, int i0, std::vector<double>& D,
-                         std::vector<double>& Z) {
-  std::vector<double> A(Ain), d(n), e(n, 0.0), v(n), p(n);
-  const int nr = n - i0;
-  Z.assign((size_t)nr * n, 0.0);
-  for (int i = 0; i < nr; ++i) Z[i * n + i0 + i] = 1.0;
-  for (int k = 0; k + 2 < n; ++k) {  // reflect column k below the subdiagonal away
-    double sigma = 0.0;
-    for (int i = k + 2; i < n; ++i) sigma += A[i * n + k] * A[i * n + k];
-    if (sigma == 0.0) continue;
-    const double x0 = A[(k + 1) * n + k], mu = std::sqrt(x0 * x0 + sigma);
-    const double v0 = x0 <= 0 ? x0 - mu : -sigma / (x0 + mu);
-    const double beta = 2.0 * v0 * v0 / (sigma + v0 * v0);
-    v[k + 1] = 1.0;
-    for (int i = k + 2; i < n; ++i) v[i] = A[i * n + k] / v0;
-    double pv = 0.0;
-    for (int i = k + 1; i < n; ++i) {
-      double acc = 0.0;
-      for (int j = k + 1; j < n; ++j) acc += A[i * n + j] * v[j];
-      p[i] = beta * acc;
-      pv += p[i] * v[i];
-    }
-    const double h = 0.5 * beta * pv;
-    for (int i = k + 1; i < n; ++i) p[i] -= h * v[i];
-    for (int i = k + 1; i < n; ++i)
-      for (int j = k + 1; j < n; ++j) A[i * n + j] -= v[i] * p[j] + p[i] * v[j];
-    A[(k + 1) * n + k] = mu;
-    for (int r = 0; r < nr; ++r) {  // Z <- Z (1 - beta v v')
-      double acc = 0.0;
-      for (int i = k + 1; i < n; ++i) acc += Z[r * n + i] * v[i];
-      acc *= beta;
-      for (int i = k + 1; i < n; ++i) Z[r * n + i] -= acc * v[i];
-    }
-  }
-  for (int i = 0; i < n; ++i) d[i] = A[i * n + i];
-  for (int i = 0; i + 1 < n; ++i) e[i] = A[(i + 1) * n + i];
-  for (int l = 0; l < n; ++l) {
-    for (int it = 0;; ++it) {
-      int m = l;  // the block l..m does not decouple before m
-      for (; m + 1 < n; ++m)
-        if (std::fabs(e[m]) <= 1.1e-16 * (std::fabs(d[m]) + std::fabs(d[m + 1])) + 1e-300) break;
-      if (m == l) break;
-      if (it == 60) return false;
-      // shift: the eigenvalue of the leading 2 x 2 block closer to d[l]
-      double g = (d[l + 1] - d[l]) / (2.0 * e[l]);
-      double r = std::hypot(g, 1.0);
-      g = d[m] - d[l] + e[l] / (g + (g >= 0 ? r : -r));
-      double s = 1.0, c = 1.0, q = 0.0;
-      int i = m - 1;
-      for (; i >= l; --i) {  // chase the bulge up with rotations of columns i, i + 1
-        double f = s * e[i];
-        const double b = c * e[i];
-        r = std::hypot(f, g);
-        e[i + 1] = r;
-        if (r == 0.0) {
-          d[i + 1] -= q;
-          e[m] = 0.0;
-          break;
-        }
-        s = f / r;
-        c = g / r;
-        g = d[i + 1] - q;
-        r = (d[i] - g) * s + 2.0 * c * b;
-        q = s * r;
-        d[i + 1] = g + q;
-        g = c * r - b;
-        for (int k = 0; k < nr; ++k) {
-          f = Z[k * n + i + 1];
-          Z[k * n + i + 1] = s * Z[k * n + i] + c * f;
-          Z[k * n + i] = c * Z[k * n + i] - s * f;
-        }
-      }
-      if (i >= l) continue;
-      d[l] -= q;
-      e[l] = g;
-      e[m] = 0.0;
-    }
-  }
-  std::vector<int> idx(n);
-  for (int i = 0; i < n; ++i) idx[i] = i;
-  std::sort(idx.begin(), idx.end(), [&](int a, int b) { return d[a] < d[b]; });
-  D.resize(n);
-  std::vector<double> Zs((size_t)nr * n);
-  for (int j = 0; j < n; ++j) {
-    D[j] = d[idx[j]];
-    for (int r = 0; r < nr; ++r) Zs[r * n + j] = Z[r * n + idx[j]];
-  }
-  Z.swap(Zs);
-  return true;
 }
 
 // The vector space of a solve: the dense vectors of the operator, or -- for a U(1)
