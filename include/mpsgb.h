@@ -61,7 +61,9 @@ enum { GB_HEFF_C = 0, GB_HEFF_AC = 1, GB_HEFF_AC2 = 2, GB_HEFF_AC_MPO = 3, GB_HE
 
 /* arithmetic of the bulk contractions */
 enum {
-  GB_PREC_FP64 = 0,    /* plain FP64 (CUDA-core FMA)                                 */
+  GB_PREC_FP64 = 0,    /* plain FP64: FMAs, and from 3.5e6 multiply-adds exact products of
+                          digits on the tensor cores, whose error is bounded by rows and
+                          columns rather than by entries (GB_OPT_FP64_FMA)            */
   GB_PREC_BF16X3 = 1,  /* split precision: hi/lo BF16 operands, 3 products
                           (hi*hi + hi*lo + lo*hi), FP32 accumulate in TMEM
                           (tcgen05), FP64 output                                      */
@@ -378,13 +380,22 @@ int gb_ctx_set_svd_method(gb_ctx* ctx, int method);
  * (1..32, default 8) over which the per-sector factorisations of a U(1) tensor are spread. */
 enum { GB_EIG_SYEVD = 0, GB_EIG_SYEVJ = 1, GB_EIG_SYEVD_DEVICE = 2 };
 int gb_ctx_set_gauge(gb_ctx* ctx, int eig_method, int lanes);
-/* Implementation switches that leave every result unchanged (for comparisons):
- *   GB_OPT_STAGED_MIX: the U(1) chain mix of the grouped schedule either stages the inputs
- *   of each charge's rows through shared memory or runs one warp per output row and column
- *   reading the intermediate directly; both sum in the same order.  0: direct, 2: staged,
- *   1 (default): staged when the mix has at least 4 entries per row (a long-range MPO's
- *   chain mix is close to a permutation, ~1 entry per row, where the direct form wins). */
-enum { GB_OPT_STAGED_MIX = 0 };
+/* Implementation switches.
+ *   GB_OPT_STAGED_MIX (every result unchanged, for comparisons): the U(1) chain mix of the
+ *   grouped schedule either stages the inputs of each charge's rows through shared memory or
+ *   runs one warp per output row and column reading the intermediate directly; both sum in the
+ *   same order.  0: direct, 2: staged, 1 (default): staged when the mix has at least 4 entries
+ *   per row (a long-range MPO's chain mix is close to a permutation, ~1 entry per row, where
+ *   the direct form wins).
+ *   GB_OPT_FP64_FMA: how plain FP64 products of 3.5e6 multiply-adds and more run.  0 (default):
+ *   on digits.  Entry (m, n) of a product over K terms then errs by at most
+ *   2 K 2^-54 max_k |a_mk| max_k |b_kn| (four times that for complex data): less than FMAs do on
+ *   average, but a term far below the largest entries of its row and column keeps fewer bits,
+ *   and below 2^-55 of them none.  1: by FMAs whatever the size, K 2^-53 sum_k |a_mk| |b_kn|:
+ *   for operands graded over many decades whose small results matter entry by entry; 15 to 25
+ *   times the time.  Read at every product; positive QR factors are column-wise accurate with
+ *   either. */
+enum { GB_OPT_STAGED_MIX = 0, GB_OPT_FP64_FMA = 1 };
 int gb_ctx_set_option(gb_ctx* ctx, int option, int64_t value);
 /* Truncated SVD of a two-site tensor, gauge2! (src/states/orthoview.jl:401-420) with
  * truncrank(maxdim) & trunctol(atol): AL[l s1; k], S (GB_KIND_BOND k x k: diagonal, or

@@ -824,6 +824,7 @@ void run_on_lanes_at(gb_ctx* ctx, int64_t n, const char* file, int line,
     l->svd_method = ctx->svd_method;
     l->eig_method = ctx->eig_method;
     l->aux_prec = ctx->aux_prec;
+    l->fp64_fma = ctx->fp64_fma;
     l->gemm_schedule = ctx->gemm_schedule;
     l->gemm_bn = ctx->gemm_bn;
     l->wait_ns = ctx->wait_ns;
@@ -980,6 +981,10 @@ int gb_ctx_set_option(gb_ctx* ctx, int option, int64_t value) {
     case GB_OPT_STAGED_MIX:
       GB_REQUIRE(value >= 0 && value <= 2, "staged_mix: 0, 1 or 2");
       ctx->staged_mix = (int)value;
+      break;
+    case GB_OPT_FP64_FMA:
+      GB_REQUIRE(value == 0 || value == 1, "fp64_fma: 0 or 1");
+      ctx->fp64_fma = value != 0;
       break;
     default: throw Error(GB_ERR_ARG, "unknown option");
   }

@@ -106,6 +106,7 @@ struct gb_ctx {
   int num_sms = 0;
   bool lane = false;             // an auxiliary lane context (its GPU is shared with the others)
   int aux_prec = GB_PREC_FP64;   // precision of auxiliary state contractions
+  bool fp64_fma = false;         // plain FP64 products by FMAs whatever their size
   int svd_method = 0;            // GB_SVD_* of gb_svd_trunc
   int eig_method = 0;            // GB_EIG_* of the Gram eigenproblems
   int lane_max = 8;              // host-thread lanes for per-sector work
@@ -245,6 +246,11 @@ struct Packed;
 // FP64 / complex GEMM, column-major, batched with strides.
 // op: 'N', 'T' or 'C'.  C = alpha*op(A)*op(B) + beta*C (beta = 0 does not read C).
 // pA / pB: the same operands already cut into digits (slice_operand).
+// Products of F64_SLICED_MIN_MAC and more run on digits: entry (m, n) errs by up to
+// 2 K 2^-54 max_k |a_mk| max_k |b_kn| (four times that when complex), 5.7e-17 of the result on
+// average, but relative to the row's and the column's largest entries, not to the terms of the entry
+// itself.  A caller that needs small entries of graded operands scales rows and columns first
+// (qr.cu) or has ctx->fp64_fma set: K 2^-53 sum_k |a_mk| |b_kn|, at FMA pace.
 void gemm_fp64(gb_ctx* ctx, int dtype, char opA, char opB, int64_t M, int64_t N, int64_t K,
                cplx alpha, const void* A, int64_t lda, int64_t sA, const void* B, int64_t ldb,
                int64_t sB, cplx beta, void* C, int64_t ldc, int64_t sC, int64_t batch,

@@ -20,7 +20,12 @@
 //    Measured (one product, operands cut included; SIMT tiles / here): complex 256 x 256 x 256
 //    531 / 21 us, complex 512 x 512 x 256 530 / 39 us, real 2048^3 8.6 / 0.58 ms = 30 TFLOP/s.
 //    Its error against extended precision at K = 128..256 is 5.7e-17 of the result (the FMAs':
-//    3.8e-16).
+//    3.8e-16).  That is norm by norm.  The bound of an entry is one of its row and column,
+//    2 K 2^-54 max |a| max |b| (four times that when complex), where the FMAs' is
+//    K 2^-53 sum |a_k| |b_k|: terms far below the largest entries of the row and the column keep
+//    fewer bits, and those below 2^-55 of them vanish ((1, 1e-10) times (1e-10, 1)' is off by 1e-7
+//    of itself).  Krylov vectors, environments and Gram matrices are used by norms; the positive QR
+//    scales its columns first; other callers have GB_OPT_FP64_FMA.
 //
 //  * gemm_small_kernel -- plain FP64 FMAs in tiles small enough that a product of a few
 //    million FMAs is spread over all SMs (complex 22 x 69 x 23: 240 / 3.6 us).
@@ -1124,7 +1129,7 @@ bool gemm_sliced_wanted(gb_ctx* ctx, int dtype, int64_t M, int64_t N, int64_t K,
                         double min_mac) {
   const double mac = (double)M * (double)N * (double)K * (double)batch * (is_cplx(dtype) ? 4 : 1);
   const int64_t nkb = rup(K, 64) * (is_cplx(dtype) ? 2 : 1) / 64;
-  return mac >= min_mac && nkb <= SG_MAX_KB && M < (int64_t)1 << 30 &&
+  return !ctx->fp64_fma && mac >= min_mac && nkb <= SG_MAX_KB && M < (int64_t)1 << 30 &&
          N < (int64_t)1 << 29 && tc_available(ctx);
 }
 

@@ -2051,7 +2051,7 @@ void heff_apply_raw(gb_heff* h, const void* x, void* y) {
     if (h->prec != GB_PREC_FP64)
       return s.hasPB && q.hasPA &&
              gemm_split_pair(ctx, h->dtype, h->prec, x, s.M, s.N, s.K, s.pB, q.M, q.N, q.K, q.pA, y);
-    return !ctx->lane && s.hasPB && s.pB.slices && q.hasPA && q.pA.slices &&
+    return !ctx->lane && !ctx->fp64_fma && s.hasPB && s.pB.slices && q.hasPA && q.pA.slices &&
            gemm_sliced_pair(ctx, h->dtype, x, s.M, s.N, s.K, s.pB, s.cB, s.ldb, q.M, q.N, q.K, q.pA,
                             q.cA, q.lda, y);
   };

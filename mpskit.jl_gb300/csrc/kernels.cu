@@ -493,7 +493,7 @@ void gemm_fp64(gb_ctx* ctx, int dtype, char opA, char opB, int64_t M, int64_t N,
     }
     return;
   }
-  if (alpha.im == 0.0 && beta.im == 0.0 &&
+  if (!ctx->fp64_fma && alpha.im == 0.0 && beta.im == 0.0 &&
       (pA || pB || gemm_sliced_wanted(ctx, dtype, M, N, K, batch)) &&
       gemm_fp64_sliced(ctx, dtype, opA, opB, M, N, K, alpha.re, A, lda, sA, B, ldb, sB, beta.re, C,
                        ldc, sC, batch, pA, pB))

@@ -79,9 +79,11 @@ class Context:
                                          int(lanes)))
 
     def set_option(self, name, value):
-        """Implementation switches that leave results unchanged (gb_ctx_set_option):
-        'staged_mix' (0 direct, 1 by density, 2 staged)."""
-        L.check(L.lib().gb_ctx_set_option(self.handle, {"staged_mix": 0}[name], int(value)))
+        """Implementation switches (gb_ctx_set_option): 'staged_mix' (0 direct, 1 by density, 2
+        staged; results unchanged) and 'fp64_fma' (0: large plain FP64 products on digits, errors
+        bounded by rows and columns; 1: by FMAs, bounded entry by entry, and slower)."""
+        L.check(L.lib().gb_ctx_set_option(self.handle, {"staged_mix": 0, "fp64_fma": 1}[name],
+                                          int(value)))
 
     def profile_begin(self):
         L.check(L.lib().gb_ctx_profile_begin(self.handle))

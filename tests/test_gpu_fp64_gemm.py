@@ -200,3 +200,70 @@ def test_left_and_right_products_together(ctx, Dl, Dr, cx):
     scale = np.linalg.norm(np.einsum("bsva,avc->bsc", np.abs(ref), np.abs(GR), optimize=True))
     ref = np.einsum("bsva,avc->bsc", ref, GR, optimize=True)
     assert np.linalg.norm(op(dev("mps", x)).numpy() - ref) <= 4e-15 * scale
+
+
+def _entry_bounds(A, B):
+    """The bounds of an entry: by its row and column (digits), by its terms (FMAs)."""
+    K = A.shape[1]
+    four = 4.0 if np.iscomplexobj(A) else 1.0
+    row = four * 2 * K * 2.0 ** -54 * np.outer(_part(A, 1), _part(B, 0))
+    terms = four * K * 2.0 ** -53 * (np.abs(A) @ np.abs(B))
+    return row, terms
+
+
+# real multiply-adds just below and above 3.5 million, where digits take over, and far above
+@pytest.mark.parametrize("shape,digits", [((64, 170, 160), False), ((64, 172, 160), True),
+                                          ((160, 128, 129), True), ((256, 512, 256), True)])
+@pytest.mark.parametrize("cx", [False, True])
+def test_entry_bounds_at_the_threshold(ctx, shape, digits, cx):
+    """Both sides of the rule meet the bound of their own kernel, on operands graded within rows and
+    columns."""
+    h, K, N = shape
+    if cx:
+        K //= 4
+    rng = np.random.default_rng(K)
+    A, B = _rand(rng, (2 * h, K), cx, 8), _rand(rng, (K, N), cx, 8)
+    out = mpsgb.states.mul_tail(
+        mpsgb.DeviceTensor.from_numpy(ctx, "mps", A.reshape(h, 2, K, order="F")),
+        mpsgb.DeviceTensor.from_numpy(ctx, "bond", B)).numpy().reshape(2 * h, N, order="F")
+    ref = _wide(A) @ _wide(B)
+    err = np.abs(_wide(out) - ref).astype(np.float64)
+    row, terms = _entry_bounds(A, B)
+    assert np.all(err <= (row if digits else terms) + 2.0 ** -52 * np.abs(ref).astype(np.float64))
+
+
+@pytest.mark.parametrize("cx", [False, True])
+def test_entries_of_graded_operands_by_fmas(cx):
+    """With 'fp64_fma' every entry keeps the bound of its own terms: columns of A graded down and rows
+    of B graded up, so that results are made of entries far below the largest ones; also an operator
+    built before the switch, whose constants are in digits.  Back at 0: the same bits as before."""
+    ctx = mpsgb.Context(0)
+    rng = np.random.default_rng(3)
+    h, K, N = 160, 320, 200
+    s = 10.0 ** -np.linspace(0, 20, K)
+    A = _rand(rng, (2 * h, K), cx, 0) * s
+    B = _rand(rng, (K, N), cx, 0) / s[:, None]
+    B[: K // 2] = 0
+    A[:, 0] = 1.0
+    a = mpsgb.DeviceTensor.from_numpy(ctx, "mps", A.reshape(h, 2, K, order="F"))
+    b = mpsgb.DeviceTensor.from_numpy(ctx, "bond", B)
+    D = 160
+    H = mpsgb.heisenberg_XXX(6, dtype=A.dtype)
+    n = np.asarray(H.W[2]).shape[0]
+    G = _rand(rng, (D, n, D), cx, 0)
+    G[:, 0, :] = G[:, -1, :] = np.eye(D)
+    dev = lambda k, v: mpsgb.DeviceTensor.from_numpy(ctx, k, v)
+    op = mpsgb.DerivativeOperator(ctx, L.GB_HEFF_AC, dev("gl", G), H.device(ctx, A.dtype)[2], None,
+                                  dev("gr", G), mpsgb.GB300Backend("fp64"))
+    x = dev("mps", _rand(rng, (D, 2, D), cx, 0))
+    y0, c0 = op(x).numpy(), mpsgb.states.mul_tail(a, b).numpy()
+    ctx.set_option("fp64_fma", 1)
+    out = mpsgb.states.mul_tail(a, b).numpy().reshape(2 * h, N, order="F")
+    y1 = op(x).numpy()
+    ctx.set_option("fp64_fma", 0)
+    ref = _wide(A) @ _wide(B)
+    err = np.abs(_wide(out) - ref).astype(np.float64)
+    assert np.all(err <= _entry_bounds(A, B)[1])
+    assert np.linalg.norm(y1 - y0) <= 1e-14 * np.linalg.norm(y0) and not np.array_equal(y1, y0)
+    assert np.array_equal(op(x).numpy(), y0)
+    assert np.array_equal(mpsgb.states.mul_tail(a, b).numpy(), c0)
