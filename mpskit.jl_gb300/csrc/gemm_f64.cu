@@ -389,7 +389,6 @@ struct SGArgs {
   int64_t M, N;      // logical
   int cplx;
   int64_t imrow;     // packed row of B where the imaginary parts begin
-  int64_t rowsB;     // packed rows of B
   int nkb;           // Kp / 64
   int batchA, batchB;
   const uint32_t *nzA, *nzB;
@@ -1198,7 +1197,6 @@ static SGArgs sliced_args(gb_ctx* ctx, int dtype, char opA, char opB, int64_t M,
   g.N = N;
   g.cplx = cx;
   g.imrow = cx ? rup(N, 32) : 0;
-  g.rowsB = b.rows;
   g.nkb = (int)(a.Kp / 64);
   g.batchA = (int)a.batch;
   g.batchB = (int)b.batch;
