@@ -305,8 +305,10 @@ int gb_project_complement_right(gb_ctx* ctx, gb_tensor* Y, const gb_tensor* X);
  * GB_KIND_GENERIC tensor (n, kmax) whose column j holds a vector of n elements.
  *   gb_basis_set:           column j <- v
  *   gb_basis_orthogonalize: w <- w - sum_j <v_j, w> v_j over columns 0..k-1, classical
- *                           Gram-Schmidt in two passes; h[2j], h[2j+1] = the projection
- *                           (re, im) summed over both passes
+ *                           Gram-Schmidt, repeated (up to three passes) while a pass removes
+ *                           more than half of |w|^2; h[2j], h[2j+1] = the projection (re, im)
+ *                           summed over the passes.  GB_ERR_TIMEOUT when a wait between
+ *                           the blocks ran out
  *   gb_basis_combine:       out <- sum_j coef[j] v_j (coef as re, im pairs) */
 int gb_basis_set(gb_ctx* ctx, gb_tensor* basis, int64_t j, const gb_tensor* v);
 int gb_basis_orthogonalize(gb_ctx* ctx, const gb_tensor* basis, int64_t k, gb_tensor* w,

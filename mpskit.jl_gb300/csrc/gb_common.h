@@ -326,8 +326,8 @@ void krylov_combine(gb_ctx* ctx, int dtype, int64_t n, int k, const void* V, con
 double* host_results(gb_ctx* ctx, size_t elems);
 // Positive QR of M (m x n, m >= n) from Gram matrices (qr.cu): Q (m x n), R (n x n).  False, with
 // Q and R undefined, when M is too ill conditioned for it.  Synchronises the stream.
-// Against the library's Householder routines (complex, left_orth): 0.50 and 5.9 ms at 512 x 256,
-// 6.0 and 63 ms at 2048 x 1024, 36 and 330 ms at 4096 x 2048, 208 and 887 ms at 4096 x 4096, the
+// Against the library's Householder routines (complex, left_orth): 0.52 and 5.9 ms at 512 x 256,
+// 6.5 and 63 ms at 2048 x 1024, 39 and 330 ms at 4096 x 2048, 252 and 887 ms at 4096 x 4096, the
 // largest size measured.
 constexpr int64_t QR_GRAM_MAX = 4096;
 bool qr_gram(gb_ctx* ctx, int dtype, int64_t m, int64_t n, const void* M, void* Q, void* R);

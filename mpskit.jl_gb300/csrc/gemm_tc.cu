@@ -1475,7 +1475,7 @@ void gemm_split(gb_ctx* ctx, int dtype, const Packed& A, const Packed& B, int64_
 // y = x R + L x with packed constants: both products in one launch, a tile per CTA, when that
 // is done earlier than one after the other; their outputs meet by atomic adds of two values on a
 // cleared y, whose sum does not depend on the order (that of three would).  False (nothing done) otherwise.  (tf32x3, complex 256 x 512 x
-// 512 and 512 x 256 x 512, an apply: 64.8 us one by one, 38.8 us.)
+// 512 and 512 x 256 x 512, an apply: 66 us one by one, 33 us.)
 bool gemm_split_pair(gb_ctx* ctx, int dtype, int prec, const void* x, int64_t M1, int64_t N1,
                      int64_t K1, const Packed& R, int64_t M2, int64_t N2, int64_t K2,
                      const Packed& Lp, void* y) {

@@ -340,7 +340,7 @@ int heff_exponentiate_raw(gb_ctx* ctx, gb_heff* h, int64_t n_dense, int dtype, v
 // src/environments/infinite_envs.jl:236, 252, 307, 322): T(v) = transfer(v, W, A, A) (left
 // or right), followed, when lvec is given, by the regularisation v_c -= tr(lvec v_c) rvec on
 // every channel c (the identity levels).  Restarted GMRES with Givens rotations on the host;
-// the Krylov vectors stay on the device and are orthogonalised in two batched CGS passes.
+// the Krylov vectors stay on the device and are orthogonalised in one launch each (orth.cu).
 // With a split-precision transfer a restart that reduces the true residual by less than 10%
 // ends the solve (the operator is accurate to ~1e-6; see heff_eigsolve_raw).
 int env_linsolve_raw(gb_ctx* ctx, int side, const gb_tensor* W, const gb_tensor* A, int prec,

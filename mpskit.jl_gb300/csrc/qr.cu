@@ -24,8 +24,8 @@
 // remaining rows once these are long, and two grid barriers per block.
 //
 // Measured (QR and LQ of a 256 x 2 x 256 complex tensor): 11.9 ms with the library's Householder
-// routines, 1.1 ms here; one complex 512 x 256 factorisation 5.9 ms before, 0.50 ms here (0.13 ms
-// of it the products).  Blocks of 16 took 0.84 ms (the chain through a diagonal block grows with its
+// routines, 1.14 ms here; one complex 512 x 256 factorisation 5.9 ms before, 0.52 ms here (0.31 ms
+// of it the factor; R from Q' A and the scaled copy of A are 10 us each).  Blocks of 16 took 0.84 ms (the chain through a diagonal block grows with its
 // square, the grid barriers saved are 3 k clocks each), updates of one column at a time 0.59.
 #include <cuda_runtime.h>
 

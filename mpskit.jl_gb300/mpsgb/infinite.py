@@ -108,8 +108,7 @@ def _transfer_bond(side, A, B, X):
 def _arnoldi_dominant(op, x0, tol, krylovdim=30, maxiter=200):
     """Eigenvector of the largest-magnitude eigenvalue of `op` (KrylovKit Arnoldi, :LM, eager;
     explicit restarts from the Ritz vector).  The basis lives in one device tensor and every
-    new vector is orthogonalised against it by two batched Gram-Schmidt passes
-    (gb_basis_orthogonalize); the Hessenberg matrix and its eigenproblem stay on the host."""
+    new vector is orthogonalised against it in one launch (gb_basis_orthogonalize); the Hessenberg matrix and its eigenproblem stay on the host."""
     real = x0.dtype.kind != "c"
     ctx = x0.ctx
     n = int(np.prod(x0.dims))
