@@ -780,15 +780,12 @@ void multi_dot(gb_ctx* ctx, int dtype, int64_t n, int k, const void* V, int64_t 
   finish_reduce_kernel<<<k, 256, 0, ctx->stream>>>(nblk, part, out);
   LAUNCH_CHECK();
   count_launch(ctx);
-  if (ctx->h_pinned_elems < (size_t)2 * k) {
-    if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
-    ctx->h_pinned_elems = std::max<size_t>(2 * k, 256);
-    GB_CHECK_CUDA(cudaMallocHost(&ctx->h_pinned, sizeof(double) * ctx->h_pinned_elems));
-  }
-  GB_CHECK_CUDA(cudaMemcpyAsync(ctx->h_pinned, out, sizeof(double) * 2 * k,
-                                cudaMemcpyDeviceToHost, ctx->stream));
+  // (grows, if it must, only after the Krylov steps in flight have written to it)
+  double* host = host_results(ctx, 2 * (size_t)k);
+  GB_CHECK_CUDA(cudaMemcpyAsync(host, out, sizeof(double) * 2 * k, cudaMemcpyDeviceToHost,
+                                ctx->stream));
   GB_CHECK_CUDA(cudaStreamSynchronize(ctx->stream));
-  for (int j = 0; j < k; ++j) host_out[j] = cplx{ctx->h_pinned[2 * j], ctx->h_pinned[2 * j + 1]};
+  for (int j = 0; j < k; ++j) host_out[j] = cplx{host[2 * j], host[2 * j + 1]};
 }
 
 cplx dot(gb_ctx* ctx, int dtype, int64_t n, const void* x, const void* y) {

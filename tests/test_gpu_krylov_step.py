@@ -123,3 +123,25 @@ def test_solve_over_pieces_short_and_long(ctx, Dl, Dr, dtype):
     y = op(vec).numpy()
     assert abs(np.vdot(v, y) - val) <= 1e-12 * np.linalg.norm(y)
     assert ctx.device_status() == 0
+
+
+def test_long_lists_after_a_solve_that_ended_early(ctx):
+    """A solve that stops with a step still queued, then more dot products than the pinned results
+    have room for: the room grows once the queued step has written its numbers."""
+    own = mpsgb.Context(0)
+    H = mpsgb.heisenberg_XXX(10, dtype=np.float64)
+    As = mpsgb.states.random_tensors(10, 2, 32, seed=4, dtype=np.float64)
+    psi = mpsgb.FiniteMPS.from_tensors(As, own, center=5)
+    envs = mpsgb.FiniteEnvironments(psi, H)
+    op = mpsgb.AC_hamiltonian(5, psi, H, envs)
+    rng = np.random.default_rng(5)
+    n, k = 2000, 700  # 1400 doubles; the steps' own slots are 1040
+    V = np.linalg.qr(rng.standard_normal((n, k)))[0]
+    w = rng.standard_normal(n)
+    for _ in range(3):
+        lam, _, info = mpsgb.fixedpoint(op, psi.ac(5), "SR", mpsgb.Lanczos(30, 1, 1e-3, True))
+        assert info.numops < 30 and np.isfinite(lam)
+        out, h = _orthogonalize(own, V, w)
+        assert np.linalg.norm(w - V @ h - out) <= 16 * k * EPS * np.linalg.norm(w)
+        assert np.linalg.norm(V.T @ out) <= 16 * k * EPS * np.linalg.norm(out)
+    assert own.device_status() == 0
