@@ -166,3 +166,18 @@ def test_graded_columns(ctx, cx, shape, decades):
             assert np.linalg.norm(q.conj().T @ q - np.eye(k)) <= 8 * n * EPS
             assert np.all(np.linalg.norm(c - q @ r, axis=0) <= 8 * n * EPS * np.linalg.norm(c, axis=0))
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("cx", [False, True])
+def test_where_the_products_would_be_slow(ctx, cx):
+    """More rows than the digits' contraction takes and too many for the small tiles: the library's
+    panels, as their four launches tell; the Gram route on either side of it."""
+    rng = np.random.default_rng(4)
+    for m, n, gram in ((200000, 4, not cx), (270000, 8, False), (131072 if cx else 262144, 8, True)):
+        a = rng.standard_normal((m, n)) + (1j * rng.standard_normal((m, n)) if cx else 0)
+        t = mpsgb.DeviceTensor.from_numpy(ctx, "mps", a.reshape(m // 2, 2, n, order="F"))
+        before = ctx.kernel_launches()
+        q, r = mpsgb.left_orth(t)
+        assert (ctx.kernel_launches() - before > 6) == gram, (m, n)
+        _check(a, q.numpy().reshape(m, n, order="F"), r.numpy(), None)
+    assert ctx.device_status() == 0
