@@ -79,10 +79,15 @@ struct CholArgs {
                 // half on exit
   void* Z;      // NB x NB: inverse of the current diagonal block's (lower) factor
   int* fail;    // set when a pivot is not positive, or when a wait ran out
+  const int* skip;  // nonzero: a column is zero or not finite, there is nothing to factor
   unsigned int* bar;
   int* status;
   unsigned long long wait_ns;
 };
+
+// added to the arrivals by the first block when a pivot is not positive: every block stops at its
+// next barrier
+constexpr unsigned int CHOL_STOP = 1u << 30;
 
 __device__ bool chol_barrier(const CholArgs& g, unsigned int target) {
   __shared__ int ok;
@@ -92,13 +97,15 @@ __device__ bool chol_barrier(const CholArgs& g, unsigned int target) {
     atomicAdd(&g.bar[0], 1u);
     ok = 1;
     const unsigned long long t0 = globaltimer();
-    while (*(volatile unsigned int*)&g.bar[0] < target) {
+    unsigned int arrived;
+    while ((arrived = *(volatile unsigned int*)&g.bar[0]) < target) {
       if (globaltimer() - t0 > g.wait_ns) {
         atomicExch(g.status, GB_ERR_TIMEOUT);
         ok = 0;
         break;
       }
     }
+    if (arrived >= CHOL_STOP) ok = 0;
     __threadfence();
   }
   __syncthreads();
@@ -151,7 +158,10 @@ __device__ void diag_block(const CholArgs& g, int k0, int nb, T (*row)[2 * NB + 
     if (!left) Z[i + NB * jj] = a;
     if (i < nb && jj < nb && (!left || i <= jj))
       A[k0 + i + ld * ((left ? k0 : g.n + k0) + jj)] = a;
-    if (bad) atomicExch(g.fail, 1);
+    if (bad && threadIdx.x == 0) {
+      atomicExch(g.fail, 1);
+      atomicAdd(&g.bar[0], CHOL_STOP);
+    }
   }
   __syncthreads();
 }
@@ -202,8 +212,8 @@ __global__ void __launch_bounds__(QT, 1) gram_chol_kernel(CholArgs g) {
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int gw = blockIdx.x + warp * gridDim.x, nw = gridDim.x * QW;  // one warp per SM first
   unsigned int target = 0;
-  bool ok = true;
-  if (blockIdx.x == 0) diag_block<T>(g, 0, min(NB, n), row);
+  bool ok = *(volatile const int*)g.skip == 0;
+  if (ok && blockIdx.x == 0) diag_block<T>(g, 0, min(NB, n), row);
   for (int j = 0; j < steps && ok; ++j) {
     const int k0 = j * NB, nb = min(NB, n - k0), k1 = k0 + nb;
     target += gridDim.x;
@@ -300,11 +310,11 @@ __global__ void unit_kernel(int n, typename Sc<CX>::T* X) {
 }
 
 // As = A with column j scaled by 2^(1023 - ex[j]), ex[j] the largest biased exponent of its parts
-// (columns of zeros or with Inf or NaN: 2^0).  A block per column.  Bound by its latency (2 MB of
+// (columns of zeros or with Inf or NaN: 2^0, and *skip is set).  A block per column.  Bound by its latency (2 MB of
 // a 512 x 256 complex matrix).
 template <bool CX>
 __global__ void __launch_bounds__(QT)
-    equilibrate_kernel(int64_t m, int64_t n, const double* A, double* As, int* ex) {
+    equilibrate_kernel(int64_t m, int64_t n, const double* A, double* As, int* ex, int* skip) {
   chain_release();
   chain_wait();
   __shared__ int most;
@@ -322,7 +332,10 @@ __global__ void __launch_bounds__(QT)
     e = most == 0 || most == 0x7ff ? 1023 : min(most, 2045);
     const double s = __hiloint2double((2046 - e) << 20, 0);
     for (int64_t i = threadIdx.x; i < len; i += QT) As[j * len + i] = a[i] * s;
-    if (threadIdx.x == 0) ex[j] = e;
+    if (threadIdx.x == 0) {
+      ex[j] = e;
+      if (most == 0 || most == 0x7ff) atomicExch(skip, 1);
+    }
     __syncthreads();
   }
 }
@@ -412,7 +425,8 @@ bool qr_gram(gb_ctx* ctx, int dtype, int64_t m, int64_t n, const void* M, void* 
   WorkBuf w(ctx, 256 + up256(n * sizeof(int)) + up256(NB * NB * es) +
                      up256(2 * (size_t)n * n * es) + nn + 3 * mn);
   if (!w.p) return false;
-  unsigned long long* res = (unsigned long long*)w.p;  // [0] max |E|, [1] failed pivots (int)
+  // [0] max |E|, [1] failed pivots (int), [2] columns without a scale (int)
+  unsigned long long* res = (unsigned long long*)w.p;
   int* ex = (int*)(w.p + 256);
   char* Z = w.p + 256 + up256(n * sizeof(int));
   char* A = Z + up256(NB * NB * es);
@@ -426,7 +440,7 @@ bool qr_gram(gb_ctx* ctx, int dtype, int64_t m, int64_t n, const void* M, void* 
   const unsigned eb = (unsigned)std::min<int64_t>((n * n + 255) / 256, 4 * sms);
   launch_chained(cx ? equilibrate_kernel<true> : equilibrate_kernel<false>,
                  dim3((unsigned)std::min<int64_t>(n, 8 * sms)), QT, 0, ctx->stream, 1, 1, m, n,
-                 (const double*)M, (double*)As, ex);
+                 (const double*)M, (double*)As, ex, (int*)(res + 2));
   gemm_fp64(ctx, dtype, 'C', 'N', n, n, m, one, As, m, 0, As, m, 0, none, A, n, 0, 1);
   char* X = A + (size_t)n * n * es;
   if (cx) unit_kernel<true><<<eb, 256, 0, ctx->stream>>>((int)n, (double2*)X);
@@ -437,6 +451,7 @@ bool qr_gram(gb_ctx* ctx, int dtype, int64_t m, int64_t n, const void* M, void* 
   a.A = A;
   a.Z = Z;
   a.fail = (int*)(res + 1);
+  a.skip = (int*)(res + 2);
   a.bar = (unsigned int*)((char*)ctx->d_status + 96);
   a.status = ctx->d_status;
   a.wait_ns = ctx->wait_ns;

@@ -181,3 +181,28 @@ def test_where_the_products_would_be_slow(ctx, cx):
         assert (ctx.kernel_launches() - before > 6) == gram, (m, n)
         _check(a, q.numpy().reshape(m, n, order="F"), r.numpy(), None)
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("shape", [(64, 33), (512, 256)])
+@pytest.mark.parametrize("cx", [False, True])
+def test_factorisations_that_stop_early(ctx, cx, shape):
+    """Low rank (a pivot runs out on the way), zero and non-finite columns anywhere: the panels'
+    factors, and the counters ready for the next factorisation."""
+    m, n = shape
+    rng = np.random.default_rng(6)
+    good, cond = _matrix(rng, m, n, cx, None)
+    low = _matrix(rng, m, n // 3, cx, None)[0] @ _matrix(rng, n // 3, n, cx, None)[0]
+    first, last = good.copy(), good.copy()
+    first[:, 0] = 0
+    last[:, -1] = 0
+    nan = good.copy()
+    nan[5, 7] = np.nan
+    for a in (low, first, last, nan):
+        q, r = next(_factors(ctx, a))
+        if a is nan:
+            assert not np.isfinite(r).all()
+        else:
+            _check(a, q, r, None)
+        q, r = next(_factors(ctx, good))
+        _check(good, q, r, cond)
+    assert ctx.device_status() == 0
